@@ -157,21 +157,58 @@ cudaError_t relax_level(dsg_ctx *ctx, int n, int jj, double ls) {
   return e;
 }
 
+// Levels 1..tail64_top in one cluster launch: the full multigrid up to that
+// level (fmg), or one V-cycle from a zero correction.
+int coarse64(dsg_ctx *ctx, bool fmg) {
+  dsg::mgc::Args<double> &G = ctx->cl64;
+  for (int l = 1; l <= G.top; l++) {
+    double **L = ctx->lv[l];
+    dsg::mgc::Level<double> &x = G.lv[l];
+    x.u = L[1];
+    x.rhs = L[3];
+    x.a = L[4];
+    x.b = L[5];
+    x.c = L[6];
+    x.ei = L[7];
+    const double h1 = ctx->s.lengthsize / (ctx->lnx[l] - 2);
+    x.h2 = h1 * h1;
+    x.h2i = 1.0 / (h1 * h1);
+    x.npre = ctx->s.npre;
+    x.npost = ctx->s.npost;
+    x.cycles = ctx->cfg.cycles;
+  }
+  // first coarsest solve with lengthscale in place of lengthsize (main.f:3686-3689)
+  const double h1 = ctx->s.lengthscale / (ctx->lnx[1] - 2);
+  G.h2_first = h1 * h1;
+  G.ntop = ctx->s.ntop;
+  G.omega = ctx->cfg.omega;
+  G.tri = 0;
+  G.fmg = fmg ? 1 : 0;
+  DSG_CK(ctx, dsg::cluster64(G, fp64_fma(ctx), ctx->stream));
+  return DSG_OK;
+}
+
 // One V-cycle from level j down to 1 and back (main.f:3705-3759).
 int vcycle(dsg_ctx *ctx, int j) {
   const double ls = ctx->s.lengthsize;
   cudaStream_t st = ctx->stream;
-  for (int jj = j; jj >= 2; jj--) {
+  const int jt = ctx->tail64_top;  // levels 1..jt in one cluster launch (0: pass by pass)
+  for (int jj = j; jj >= 2 && jj > jt; jj--) {
     double **L = ctx->lv[jj];
     const Dims d = ctx->level(jj);
     DSG_CK(ctx, relax_level(ctx, ctx->s.npre, jj, ls));
     DSG_CK(ctx, dsg::resid(ls, L[2], L[1], L[3], L[4], L[5], L[6], d, st, fp64_fma(ctx)));
     const Dims dc = ctx->level(jj - 1);
     DSG_CK(ctx, dsg::rstrct(ctx->lv[jj - 1][3], L[2], dc, st));
-    DSG_CK(ctx, dsg::fill_zero(ctx->lv[jj - 1][1], dc.count(), st));
+    if (jj - 1 != jt) DSG_CK(ctx, dsg::fill_zero(ctx->lv[jj - 1][1], dc.count(), st));
   }
-  DSG_CK(ctx, relax_level(ctx, ctx->s.ntop, 1, ls));
-  for (int jj = 2; jj <= j; jj++) {
+  if (jt >= 1) {
+    int rc = coarse64(ctx, false);
+    if (rc) return rc;
+  } else {
+    DSG_CK(ctx, relax_level(ctx, ctx->s.ntop, 1, ls));
+  }
+  for (int jj = jt >= 1 ? jt + 1 : 2; jj <= j; jj++) {
     double **L = ctx->lv[jj];
     const Dims d = ctx->level(jj);
     DSG_CK(ctx, dsg::addint(L[1], ctx->lv[jj - 1][1], L[2], d, st));
@@ -258,13 +295,41 @@ cudaError_t relax32_level(dsg_ctx *ctx, int n, int l) {
   return e;
 }
 
+// FP32 levels 1..tail_top in one cluster launch: the full multigrid up to
+// that level (fmg), or one V-cycle.
+int coarse32(dsg_ctx *ctx, bool fmg) {
+  dsg::mgc::Args<float> &G = ctx->cl32;
+  for (int l = 1; l <= G.top; l++) {
+    float **L = ctx->lv32[l];
+    dsg::mgc::Level<float> &x = G.lv[l];
+    x.u = L[U32];
+    x.rhs = L[RHS32];
+    x.a = L[A32];
+    x.b = L[B32];
+    x.c = L[C32];
+    x.ei = L[EI32];
+    x.h2 = level_h2(ctx, l);
+    x.h2i = 1.0f / level_h2(ctx, l);
+    x.npre = pre32(ctx, l);
+    x.npost = post32(ctx, l);
+    x.cycles = fmg32_cycles(ctx, l);
+  }
+  G.h2_first = level_h2(ctx, 1);
+  G.ntop = ctx->s.ntop;
+  G.omega = omega32(ctx);
+  G.tri = tri32(ctx);
+  G.fmg = fmg ? 1 : 0;
+  DSG_CK(ctx, dsg::cluster32(G, ctx->stream));
+  return DSG_OK;
+}
+
 int vcycle32(dsg_ctx *ctx, int j) {
   cudaStream_t st = ctx->stream;
   const int ng = ctx->ng;
   float r1, r2;
   phase_coefs(ctx, &r1, &r2);
-  // levels 1..jt in one single-block launch (0: every level pass by pass)
-  const int jt = ctx->tail_top < j ? ctx->tail_top : j;
+  // levels 1..jt in one cluster launch (0: every level pass by pass)
+  const int jt = ctx->tail_top;
   for (int jj = j; jj >= 2 && jj > jt; jj--) {
     float **L = ctx->lv32[jj];
     float **Lc = ctx->lv32[jj - 1];
@@ -279,9 +344,8 @@ int vcycle32(dsg_ctx *ctx, int j) {
     }
   }
   if (jt >= 1) {
-    dsg::TailArgs A;
-    tail_args(ctx, jt, &A);
-    DSG_CK(ctx, dsg::vtail32(A, st));
+    int rc = coarse32(ctx, false);
+    if (rc) return rc;
   } else {
     DSG_CK(ctx, relax32_level(ctx, ctx->s.ntop, 1));
   }
@@ -441,9 +505,14 @@ int fmg32(dsg_ctx *ctx) {
   if (ng >= 2) DSG_CK(ctx, dsg::restrict32_split(ctx->lv32[ng - 1][RHS32], f.r, ctx->level(ng - 1), st));
   for (int g = ng - 2; g >= 1; g--)
     DSG_CK(ctx, dsg::restrict32(ctx->lv32[g][RHS32], ctx->lv32[g + 1][RHS32], ctx->level(g), st));
-  DSG_CK(ctx, cudaMemsetAsync(ctx->lv32[1][U32], 0, ctx->level(1).count() * sizeof(float), st));
-  DSG_CK(ctx, relax32_level(ctx, ctx->s.ntop, 1));
-  for (int j = 2; j <= ng; j++) {
+  if (ctx->tail_top >= 1) {
+    int rc = coarse32(ctx, true);
+    if (rc) return rc;
+  } else {
+    DSG_CK(ctx, cudaMemsetAsync(ctx->lv32[1][U32], 0, ctx->level(1).count() * sizeof(float), st));
+    DSG_CK(ctx, relax32_level(ctx, ctx->s.ntop, 1));
+  }
+  for (int j = ctx->tail_top >= 1 ? ctx->tail_top + 1 : 2; j <= ng; j++) {
     if (j == ng)
       DSG_CK(ctx, dsg::prolong32_split(f.u, ctx->lv32[j - 1][U32], ctx->level(j), 0, tri32(ctx), st));
     else
@@ -692,12 +761,17 @@ int mglin(dsg_ctx *ctx, dsg_mg_stats *stats) {
     DSG_CK(ctx, dsg::acfromac(ctx->lv[g][4], ctx->lv[g][5], ctx->lv[g][6], ctx->lv[g][7], ctx->lv[g + 1][4],
                               ctx->lv[g + 1][5], ctx->lv[g + 1][6], dc, st));
   }
-  double **L1 = ctx->lv[1];
-  DSG_CK(ctx, dsg::fill_zero(L1[1], ctx->level(1).count(), st));
-  // First coarse solve with lengthscale in place of lengthsize (main.f:3686-3689).
-  DSG_CK(ctx, dsg::relax_n(ctx->s.ntop, L1[1], ctx->s.lengthscale, L1[3], L1[4], L1[5], L1[6], L1[7],
-                           ctx->level(1), om, st, fp64_fma(ctx)));
-  for (int j = 2; j <= ng; j++) {
+  if (ctx->tail64_top >= 1) {
+    int rc = coarse64(ctx, true);
+    if (rc) return rc;
+  } else {
+    double **L1 = ctx->lv[1];
+    DSG_CK(ctx, dsg::fill_zero(L1[1], ctx->level(1).count(), st));
+    // First coarse solve with lengthscale in place of lengthsize (main.f:3686-3689).
+    DSG_CK(ctx, dsg::relax_n(ctx->s.ntop, L1[1], ctx->s.lengthscale, L1[3], L1[4], L1[5], L1[6], L1[7],
+                             ctx->level(1), om, st, fp64_fma(ctx)));
+  }
+  for (int j = ctx->tail64_top >= 1 ? ctx->tail64_top + 1 : 2; j <= ng; j++) {
     DSG_CK(ctx, dsg::interp(ctx->lv[j][1], ctx->lv[j - 1][1], ctx->level(j), st));
     for (int c = 0; c < ctx->cfg.cycles; c++) {
       int rc = vcycle(ctx, j);
@@ -745,6 +819,34 @@ int mglin(dsg_ctx *ctx, dsg_mg_stats *stats) {
     return dsg::set_error(ctx, DSG_E_NOT_CONVERGED, "multigrid reached %d V-cycles at relres %.3e > tol %.3e",
                           s.vcycles, s.relres, ctx->cfg.tol);
   return DSG_OK;
+}
+
+// Which levels the cluster kernels run.  FP32: every level below the finest
+// that fits a cluster's shared memory and registers (about 40^3 cells), or of
+// at most tail_nodes nodes when the configuration says so.
+void cluster_plan(dsg_ctx *ctx) {
+  const long long cap = ctx->cfg.tail_nodes;
+  const int c32 = cap >= 0 ? dsg::cluster32_size() : 0, c64 = dsg::cluster64_size();
+  auto extents = [&](auto &G, int top) {
+    for (int l = 1; l <= top; l++) {
+      G.lv[l].nx = ctx->lnx[l] - 2;
+      G.lv[l].ny = ctx->lny[l] - 2;
+      G.lv[l].nz = ctx->lnz[l] - 2;
+    }
+  };
+  const int most = ctx->ng - 1 < dsg::mgc::kMaxLevels ? ctx->ng - 1 : dsg::mgc::kMaxLevels;
+  memset(&ctx->cl32, 0, sizeof ctx->cl32);
+  memset(&ctx->cl64, 0, sizeof ctx->cl64);
+  ctx->tail_top = ctx->tail64_top = 0;
+  for (int l = most; l >= 1 && c32 > 0 && ctx->tail_top == 0; l--) {
+    if (cap > 0 && (long long)ctx->lnx[l] * ctx->lny[l] * ctx->lnz[l] > cap) continue;
+    extents(ctx->cl32, l);
+    if (dsg::mgc::layout(ctx->cl32, l, c32, 1024, dsg::kCluster32Cells)) ctx->tail_top = l;
+  }
+  for (int l = most; l >= 1 && c64 > 0 && ctx->tail64_top == 0; l--) {
+    extents(ctx->cl64, l);
+    if (dsg::mgc::layout(ctx->cl64, l, c64, 128, dsg::kCluster64Cells)) ctx->tail64_top = l;
+  }
 }
 
 }  // namespace
@@ -860,12 +962,7 @@ int dsg_create(const dsg_config *cfg, dsg_ctx **out) {
   ctx->s.cycles = cfg->cycles;
   ctx->s.ng = ng;
   ctx->s.last_epsdiv = -1.0;
-  {
-    const long long cap = cfg->tail_nodes == 0 ? 18LL * 18 * 18 : cfg->tail_nodes;
-    ctx->tail_top = 0;
-    for (int l = 1; l < ng && l <= dsg::kTailMaxLevels; l++)
-      if ((long long)ctx->lnx[l] * ctx->lny[l] * ctx->lnz[l] <= cap) ctx->tail_top = l;
-  }
+  cluster_plan(ctx);
   nondim(ctx);
   *out = ctx;
   return DSG_OK;

@@ -25,6 +25,12 @@ inline void count_launch() {
 }
 #define DSG_COUNT dsg::count_launch(),
 
+}  // namespace dsg
+
+#include "mgcluster.cuh"
+
+namespace dsg {
+
 // Column-major, 1-based (i,j,k) -> linear offset of an (nx,ny,nz) array.
 struct Dims {
   int nx, ny, nz;
@@ -200,7 +206,14 @@ struct TailArgs {
   float omega;
   int tri;  // trilinear prolongation (else injection)
 };
-cudaError_t vtail32(const TailArgs &args, cudaStream_t st);
+// coarse levels in one cluster launch (mgcluster.cuh).  cluster*_size: blocks
+// of the largest cluster the current device runs (0: none), with the kernel's
+// attributes set; cells per thread of a colour a block may have.
+constexpr int kCluster32Cells = 10, kCluster64Cells = 4;
+int cluster32_size();
+int cluster64_size();
+cudaError_t cluster32(const mgc::Args<float> &args, cudaStream_t st);
+cudaError_t cluster64(const mgc::Args<double> &args, bool fma, cudaStream_t st);
 // finest level in colour-split storage ({even, odd} arrays of (nx-2)/2 x (ny-2) x (nz-2))
 cudaError_t relax32_split_n(int n, float *const u[2], float *const rhs[2], const float *cc, Dims d, float h2,
                             float omega, float r1, float r2, cudaStream_t st);
@@ -274,7 +287,10 @@ struct dsg_ctx {
   dsg_scalars s;
   int nx, ny, nz, ng;
   int device = 0;             // CUDA device the context was created on
-  int tail_top = 0;           // FP32 levels 1..tail_top run in the single-block tail kernel (0: none)
+  int tail_top = 0;           // FP32 levels 1..tail_top run in the cluster kernel (0: none)
+  int tail64_top = 0;         // the same for the FP64 multigrid
+  dsg::mgc::Args<float> cl32;    // their slabs and shared-memory layout
+  dsg::mgc::Args<double> cl64;
   int lnx[32], lny[32], lnz[32];
   double *lv[32][8];          // [level][CC,P,RES,RHS,A,B,C,EI], level 1..ng
   float *lv32[32][6];         // FP32 hierarchy [level][U,RHS,A,B,C,EI] of the mixed mode;
@@ -437,7 +453,8 @@ inline void phase_coefs(dsg_ctx *ctx, float *r1, float *r2) {
   *r2 = (float)ctx->s.rho2;
 }
 
-// Arguments of the coarse-tail kernel for FP32 levels 1..top of ctx.
+// Arguments of the single-block coarse tail for FP32 levels 1..top of ctx (the
+// batched ensemble solve).
 inline void tail_args(dsg_ctx *ctx, int top, dsg::TailArgs *A) {
   memset(A, 0, sizeof *A);
   for (int l = 1; l <= top; l++) {

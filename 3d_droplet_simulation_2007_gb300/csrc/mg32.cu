@@ -69,7 +69,53 @@ __global__ void k_prolong32(float *__restrict__ uf, const float *__restrict__ uc
   b_prolong32<TRI>(blockIdx, gridDim, uf, uc, df, dc, add);
 }
 
-__global__ void __launch_bounds__(kTailThreads, 1) k_vtail32(TailArgs A) { tail_body(A); }
+// Arithmetic of the cluster kernel on the FP32 levels.
+struct Cluster32 {
+  typedef float T;
+  static constexpr int kMaxCells = kCluster32Cells;
+  static __device__ __forceinline__ float relax(float uc, float xp, float xm, float yp, float ym, float zp, float zm,
+                                                float ae, float aw, float bn, float bs, float ct, float cb, float ei,
+                                                float rhs, float h2, float omega) {
+    return relax32_value(uc, Nb{xp, xm, yp, ym, zp, zm}, ae, aw, bn, bs, ct, cb, ei, rhs, h2, omega);
+  }
+  static __device__ __forceinline__ float resid(float uc, float xp, float xm, float yp, float ym, float zp, float zm,
+                                                float ae, float aw, float bn, float bs, float ct, float cb, float rhs,
+                                                float h2i) {
+    return resid32_value(uc, Nb{xp, xm, yp, ym, zp, zm}, ae, aw, bn, bs, ct, cb, rhs, h2i);
+  }
+  static __device__ __forceinline__ float mean8(float r0, float r1, float r2, float r3, float r4, float r5, float r6,
+                                                float r7) {
+    float acc = 0.f;
+    acc += r0;
+    acc += r1;
+    acc += r2;
+    acc += r3;
+    acc += r4;
+    acc += r5;
+    acc += r6;
+    acc += r7;
+    return 0.125f * acc;
+  }
+  // Coarse planes c0, c0 + 1 .. of `buf` at fine cell (x, y, k), 0-based.
+  static __device__ __forceinline__ float prolong(const float *buf, int nx, int ny, int nz, int c0, int x, int y,
+                                                  int k, int tri) {
+    const int px = x >> 1, py = y >> 1, pk = k >> 1, P = nx * ny;
+    const float *p = buf + (pk - c0) * P + py * nx;
+    if (!tri) return p[px];
+    int dy = (y & 1) ? 1 : -1, dk = (k & 1) ? 1 : -1;
+    if (py + dy < 0 || py + dy == ny) dy = 0;
+    if (pk + dk < 0 || pk + dk == nz) dk = 0;
+    const float *pb = p + dy * nx, *pc = p + dk * P, *pe = pc + dy * nx;
+    const int xn = px + ((x & 1) ? 1 : -1);
+    const float yp = tri_yz_value(p[px], pb[px], pc[px], pe[px]);
+    const float yn = xn == nx ? 0.f : (xn < 0 ? yp : tri_yz_value(p[xn], pb[xn], pc[xn], pe[xn]));
+    return tri_x(yp, yn);
+  }
+};
+
+__global__ void __launch_bounds__(mgc::kThreads, 1) k_cluster32(const __grid_constant__ mgc::Args<float> G) {
+  mgc::cluster_mg<Cluster32>(G);
+}
 
 __global__ void k_restrict32(float *__restrict__ uc, const float *__restrict__ uf, Dims dc, Dims df) {
   b_restrict32(blockIdx, gridDim, uc, uf, dc, df);
@@ -400,11 +446,11 @@ cudaError_t resid_restrict32(float *rhs_c, float *u_c, const float *u, const flo
   return cudaGetLastError();
 }
 
-cudaError_t vtail32(const TailArgs &args, cudaStream_t st) {
-  DSG_COUNT k_vtail32<<<1, kTailThreads, 0, st>>>(args);
-  return cudaGetLastError();
-}
+int cluster32_size() { return mgc::cluster_size(k_cluster32); }
 
+cudaError_t cluster32(const mgc::Args<float> &args, cudaStream_t st) {
+  return mgc::launch(k_cluster32, args, st);
+}
 
 cudaError_t prolong32(float *uf, const float *uc, Dims df, int add, int tri, cudaStream_t st) {
   const Dims dc{df.nx / 2 + 1, df.ny / 2 + 1, df.nz / 2 + 1};

@@ -96,12 +96,18 @@ __device__ __forceinline__ float split_get(const float *__restrict__ ev, const f
 // fixes the rounding, so that every kernel that interpolates gives the same
 // bits.
 
+// Bilinear y-z combination of the parent row's value (a) and its neighbours'
+// along y (b), z (c) and both (e).
+__device__ __forceinline__ float tri_yz_value(float a, float b, float c, float e) {
+  return fmaf(0.0625f, e, fmaf(0.1875f, c, fmaf(0.1875f, b, 0.5625f * a)));
+}
+
 // Bilinear y-z combination at coarse x-index x (parent row pj, pk; neighbours nj, nk).
 __device__ __forceinline__ float tri_yz(const float *__restrict__ uc, Dims dc, int x, int pj, int nj, int pk,
                                         int nk) {
   const float a = uc[ix32(dc, x, pj, pk)], b = uc[ix32(dc, x, nj, pk)];
   const float c = uc[ix32(dc, x, pj, nk)], e = uc[ix32(dc, x, nj, nk)];
-  return fmaf(0.0625f, e, fmaf(0.1875f, c, fmaf(0.1875f, b, 0.5625f * a)));
+  return tri_yz_value(a, b, c, e);
 }
 
 // Coarse neighbour of parent p on the side of fine index f (odd f: +1, even:
@@ -318,7 +324,22 @@ __device__ __forceinline__ void b_split_from64(const uint3 B, const uint3 G, flo
 // The per-cell operations are shared by the one-launch-per-pass kernels and by
 // the single-block tail kernel below, so both give the same bits.
 
-// One red-black update of cell (i,j,k) (relax, main.f:3956-3997).
+// Red-black update of a cell with value uc from its neighbours and face
+// coefficients (relax, main.f:3956-3997), and its residual.
+__device__ __forceinline__ float relax32_value(float uc, const Nb &n, float ae, float aw, float bn, float bs, float ct,
+                                               float cb, float ei, float rhs, float h2, float omega) {
+  // the explicit fmaf keeps its rounding where h2 * rhs is loop-invariant
+  const float s = fmaf(-h2, rhs, ae * n.xp + aw * n.xm + bn * n.yp + bs * n.ym + ct * n.zp + cb * n.zm);
+  return omega * (s * ei) + (1.f - omega) * uc;
+}
+__device__ __forceinline__ float resid32_value(float uc, const Nb &n, float ae, float aw, float bn, float bs, float ct,
+                                               float cb, float rhs, float h2i) {
+  const float lap = ae * (n.xp - uc) + aw * (n.xm - uc) + bn * (n.yp - uc) + bs * (n.ym - uc) + ct * (n.zp - uc) +
+                    cb * (n.zm - uc);
+  return rhs - h2i * lap;
+}
+
+// One red-black update of cell (i,j,k).
 __device__ __forceinline__ void relax32_cell(float *u, const float *rhs, const float *a, const float *b,
                                              const float *c, const float *ei, Dims d, int i, int j, int k,
                                              float h2, float omega) {
@@ -326,9 +347,7 @@ __device__ __forceinline__ void relax32_cell(float *u, const float *rhs, const f
   const unsigned sy = (unsigned)d.nx, sz = (unsigned)d.nx * d.ny;
   const float uc = u[q];
   const Nb n = neighbours(u, q, i, j, k, d, uc);
-  const float s = a[q] * n.xp + a[q - 1] * n.xm + b[q] * n.yp + b[q - sy] * n.ym + c[q] * n.zp + c[q - sz] * n.zm -
-                  h2 * rhs[q];
-  u[q] = omega * (s * ei[q]) + (1.f - omega) * uc;
+  u[q] = relax32_value(uc, n, a[q], a[q - 1], b[q], b[q - sy], c[q], c[q - sz], ei[q], rhs[q], h2, omega);
 }
 
 // Coarse rhs of coarse cell (ic,jc,kc) = mean of its 8 fine residuals (resid +
@@ -348,9 +367,7 @@ __device__ __forceinline__ void resid_restrict32_cell(float *rhs_c, float *u_c, 
         const unsigned q = ix32(df, i, j, k);
         const float uc = u[q];
         const Nb n = neighbours(u, q, i, j, k, df, uc);
-        const float lap = a[q] * (n.xp - uc) + a[q - 1] * (n.xm - uc) + b[q] * (n.yp - uc) +
-                          b[q - sy] * (n.ym - uc) + c[q] * (n.zp - uc) + c[q - sz] * (n.zm - uc);
-        acc += rhs[q] - h2i * lap;
+        acc += resid32_value(uc, n, a[q], a[q - 1], b[q], b[q - sy], c[q], c[q - sz], rhs[q], h2i);
       }
   const unsigned qc = ix32(dc, ic, jc, kc);
   rhs_c[qc] = 0.125f * acc;
@@ -396,8 +413,9 @@ __device__ __forceinline__ void b_prolong32(const uint3 B, const uint3 G, float 
 
 // ---- coarse tail: every level at or below `top` in one thread block ---------
 //
-// On levels of a few thousand cells a launch costs more than its work.  The
-// tail kernel runs the rest of a V-cycle from level `top` down to the coarsest
+// The batched ensemble solve's form of the coarse levels (a standalone solve
+// runs them in a cluster, mgcluster.cuh; here each member's block must fit
+// beside the other members').  The tail runs the rest of a V-cycle from level `top` down to the coarsest
 // grid and back (pre-sweeps, residual restriction, NTOP coarsest sweeps,
 // prolongation, post-sweeps: mglin's recursion, main.f:3703-3759) inside one
 // block, with a block barrier between passes in place of a launch boundary.

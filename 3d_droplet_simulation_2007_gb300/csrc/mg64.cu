@@ -127,6 +127,59 @@ __global__ void k_relax_colour(double *__restrict__ u, const double *__restrict_
   u[q] = omega * temp + (1.0 - omega) * uc;
 }
 
+// Arithmetic of the cluster kernel on the FP64 levels: the two forms of
+// k_relax_colour and k_resid, and rstrct's and interp's transfers.
+template <bool FMA>
+struct Cluster64 {
+  typedef double T;
+  static constexpr int kMaxCells = kCluster64Cells;
+  static __device__ __forceinline__ double relax(double uc, double xp, double xm, double yp, double ym, double zp,
+                                                 double zm, double ae, double aw, double bn, double bs, double ct,
+                                                 double cb, double ei, double rhs, double h2, double omega) {
+    if (FMA) {
+      double t = ae * xp;
+      t = __fma_rn(aw, xm, t);
+      t = __fma_rn(bn, yp, t);
+      t = __fma_rn(bs, ym, t);
+      t = __fma_rn(ct, zp, t);
+      t = __fma_rn(cb, zm, t);
+      t = __fma_rn(-h2, rhs, t) * ei;
+      return __fma_rn(omega, t - uc, uc);
+    }
+    const double temp = (ae * xp + aw * xm + bn * yp + bs * ym + ct * zp + cb * zm - h2 * rhs) * ei;
+    return omega * temp + (1.0 - omega) * uc;
+  }
+  static __device__ __forceinline__ double resid(double uc, double xp, double xm, double yp, double ym, double zp,
+                                                 double zm, double ae, double aw, double bn, double bs, double ct,
+                                                 double cb, double rhs, double h2i) {
+    if (FMA) {
+      double t = ae * (xp - uc);
+      t = __fma_rn(aw, xm - uc, t);
+      t = __fma_rn(bn, yp - uc, t);
+      t = __fma_rn(bs, ym - uc, t);
+      t = __fma_rn(ct, zp - uc, t);
+      t = __fma_rn(cb, zm - uc, t);
+      return __fma_rn(-h2i, t, rhs);
+    }
+    return -h2i * (ae * (xp - uc) + aw * (xm - uc) + bn * (yp - uc) + bs * (ym - uc) + ct * (zp - uc) +
+                   cb * (zm - uc)) +
+           rhs;
+  }
+  static __device__ __forceinline__ double mean8(double r0, double r1, double r2, double r3, double r4, double r5,
+                                                 double r6, double r7) {
+    return 0.125 * (r0 + r1 + r2 + r3 + r4 + r5 + r6 + r7);
+  }
+  static __device__ __forceinline__ double prolong(const double *buf, int nx, int ny, int, int c0, int x, int y, int k,
+                                                   int) {
+    return buf[((k >> 1) - c0) * nx * ny + (y >> 1) * nx + (x >> 1)];
+  }
+};
+
+template <bool FMA>
+__global__ void __launch_bounds__(mgc::kThreads, 1) k_cluster64(const __grid_constant__ mgc::Args<double> G) {
+  mgc::cluster_mg<Cluster64<FMA>>(G);
+}
+
 // Residual of one interior cell, rhs - (1/h^2) sum a_nb (u_nb - u) (main.f:3912-3925),
 // in the reference's order or as a fused multiply-add chain.
 template <bool FMA>
@@ -575,6 +628,15 @@ static void relax_passes(double *u, double h2, const double *rhs, const double *
     else
       DSG_COUNT k_relax_colour<false><<<grid, kBlk, 0, st>>>(u, rhs, a, b, c, ei, d, h2, omega, colour);
   }
+}
+
+int cluster64_size() {
+  const int n = mgc::cluster_size(k_cluster64<false>);
+  return mgc::cluster_size(k_cluster64<true>) < n ? 0 : n;
+}
+
+cudaError_t cluster64(const mgc::Args<double> &args, bool fma, cudaStream_t st) {
+  return fma ? mgc::launch(k_cluster64<true>, args, st) : mgc::launch(k_cluster64<false>, args, st);
 }
 
 cudaError_t relax(double *u, double lengthsize, const double *rhs, const double *a, const double *b,

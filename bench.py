@@ -73,7 +73,7 @@ def parse():
     ap.add_argument("--fmg32-fine", type=int, default=None,
                     help="V-cycles of the FP32 FMG start on the finest level (default: as on the others)")
     ap.add_argument("--tail-nodes", type=int, default=0,
-                    help="largest FP32 level (nodes) of the single-block coarse tail (0: default, -1: off)")
+                    help="largest FP32 level (nodes) run in the cluster launch (0: all that fit, -1: off)")
     ap.add_argument("--e2e-steps", type=int, default=6)
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")

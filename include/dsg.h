@@ -88,8 +88,9 @@ typedef struct dsg_config {
   int inner_vcycles;   /* FP32 V-cycles per FP64 defect evaluation in the mixed modes (<= 0: as many
                           as the measured reduction per V-cycle predicts to reach tol, at most 8) */
   int use_graphs;      /* capture the mixed-mode iterations in CUDA graphs (1) or launch directly (0) */
-  int tail_nodes;      /* mixed modes: FP32 levels of at most this many nodes run in one single-block
-                          launch per V-cycle (0: 18^3 = 5832; < 0: one launch per pass on every level) */
+  int tail_nodes;      /* mixed modes: FP32 levels of at most this many nodes run in one launch of a
+                          thread-block cluster per V-cycle, as far as they fit one (0: every level below
+                          the finest that fits, about 40^3 cells; < 0: one launch per pass on every level) */
   int warm_start;      /* DSG_MODE_TOL_MIXED initial guess: 0 = FP32 full multigrid, 1 = previous-step
                           pressure, 2 = zero */
   double mg32_omega;   /* relaxation factor of the FP32 V-cycles of the mixed modes (<= 0: omega) */
