@@ -133,7 +133,8 @@ cudaError_t fill_zero(double *f, size_t n, cudaStream_t st);
 
 // vof.cu
 cudaError_t bc_c(double *cc, Dims d, cudaStream_t st);
-// list/count: scratch of the interface-cell list (>= interior cells) and its length
+// list/count: scratch of the interface-cell list and the cells' bits (a fine
+// field) and the list's length, zero before the call and after it
 cudaError_t swp(const double *us, double *cc, double *vof1, double *vof2, double *vof3, int dir, Dims d,
                 double tauh, unsigned *list, unsigned *count, cudaStream_t st);
 cudaError_t calcrho(double *rhon, double *mun, const double *cc, Dims d, double rho1, double rho2,

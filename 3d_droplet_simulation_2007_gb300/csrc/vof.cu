@@ -2,16 +2,25 @@
 // the plane/volume relations AL3D/FL3D (main.f:4562-4698), bc_flux
 // (main.f:4496-4539), bc_c (main.f:4331-4396) and calcrho (main.f:2177-2190).
 //
-// One sweep = flux kernel (per cell: left-out, stay, right-out volumes written
-// to the three scratch arrays the reference uses: z(iei), z(ires), z(irhs) of
-// the finest level) -> bc_flux -> update kernel (c = vof3(i-1)+vof2(i)+vof1(i+1)
-// clipped to [0,1]) -> bc_c.  Most cells are empty or full and take the cheap
-// branches; interface cells evaluate the Youngs normal, AL3D and up to three
-// FL3D calls in FP64.
+// One sweep = scan kernel (a bit per cell: not empty; the fluxes of the full
+// cells, the list of the interface cells) -> flux kernel of the listed cells
+// (left-out, stay, right-out volumes in the three scratch arrays the reference
+// uses: z(iei), z(ires), z(irhs) of the finest level) -> update kernel
+// (c = vof3(i-1)+vof2(i)+vof1(i+1) clipped to [0,1]) -> bc_c.  A cell whose own
+// and two neighbours' bits are clear stays at zero, so the update and the flux
+// arrays touch the liquid and its rim only: most of a sweep's traffic is the
+// scan's one read of c.
 #include "dsg_internal.cuh"
 
 namespace dsg {
 namespace {
+
+// The lanes of a warp take different branches of AL3D and FL3D, and a warp
+// executes every branch that one of its lanes takes, at 16 cycles of the SM's
+// FP64 pipe per instruction.  The branches below therefore only pick operands;
+// the divisions, square roots and acos/cos that several of them share stand
+// behind the branches and are executed once (same operations per cell;
+// 64^3: 36 -> 30 us).
 
 // AL3D: plane constant alpha of m1 x1 + m2 x2 + m3 x3 = alpha cutting volume cc
 // from the unit cube (m1+m2+m3 = 1, all >= 0).  Scardovelli-Zaleski analytic
@@ -27,40 +36,35 @@ __device__ double al3d(double b1, double b2, double b3, double cc) {
   const double pr = dmax1(6.0 * m1 * m2 * m3, 1.0e-50);
   const double V1 = m1 * m1 * m1 / pr;
   const double V2 = V1 + 0.5 * (m2 - m1) / m3;
-  double mm, V3;
-  if (m3 < m12) {
-    mm = m3;
-    V3 = (m3 * m3 * (3.0 * m12 - m3) + m1 * m1 * (m1 - 3.0 * m3) + m2 * m2 * (m2 - 3.0 * m3)) / pr;
-  } else {
-    mm = m12;
-    V3 = 0.5 * mm / m3;
+  const bool five = m3 < m12;  // regimes 3 and 5 up to m3, else 3 and 4 up to m12
+  const double mm = five ? m3 : m12;
+  double num = 0.5 * mm, den = m3;
+  if (five) {
+    num = m3 * m3 * (3.0 * m12 - m3) + m1 * m1 * (m1 - 3.0 * m3) + m2 * m2 * (m2 - 3.0 * m3);
+    den = pr;
   }
+  const double V3 = num / den;
   const double ch = dmin1(cc, 1.0 - cc);
   double res;
   if (ch < V1) {
     res = pow(pr * ch, 1.0 / 3.0);
   } else if (ch < V2) {
     res = 0.5 * (m1 + sqrt(m1 * m1 + 8.0 * m2 * m3 * (ch - V1)));
-  } else if (ch < V3) {
-    const double p = 2.0 * m1 * m2;
-    const double q = 1.5 * m1 * m2 * (m12 - 2.0 * m3 * ch);
-    const double p12 = sqrt(p);
-    double cst = q / (p * p12);
-    if (cst > 1.0) cst = 1.0;
-    if (cst < -1.0) cst = -1.0;
-    const double cs = cos(acos(cst) / 3.0);
-    res = p12 * (sqrt(3.0 * (1.0 - cs * cs)) - cs) + m12;
-  } else if (mm == m12) {
+  } else if (ch >= V3 && mm == m12) {
     res = m3 * ch + 0.5 * mm;
   } else {
-    const double p = m1 * (m2 + m3) + m2 * m3 - 0.25;
-    const double q = 1.5 * m1 * m2 * m3 * (0.5 - ch);
+    double p = 2.0 * m1 * m2, q = 1.5 * m1 * m2 * (m12 - 2.0 * m3 * ch), add = m12;
+    if (!(ch < V3)) {
+      p = m1 * (m2 + m3) + m2 * m3 - 0.25;
+      q = 1.5 * m1 * m2 * m3 * (0.5 - ch);
+      add = 0.5;
+    }
     const double p12 = sqrt(p);
     double cst = q / (p * p12);
     if (cst > 1.0) cst = 1.0;
     if (cst < -1.0) cst = -1.0;
     const double cs = cos(acos(cst) / 3.0);
-    res = p12 * (sqrt(3.0 * (1.0 - cs * cs)) - cs) + 0.5;
+    res = p12 * (sqrt(3.0 * (1.0 - cs * cs)) - cs) + add;
   }
   if (cc > 0.5) res = 1.0 - res;
   return res;
@@ -83,18 +87,24 @@ __device__ double fl3d(double m1, double m2, double m3, double alpha, double r0,
   const double b12 = b1 + b2;
   const double bm = dmin1(b12, b3);
   const double pr = dmax1(6.0 * b1 * b2 * b3, 1.0e-50);
+  double num, den = pr;
+  const bool two = !(al0 < b1) && al0 < b2;  // the regime with a second term, b1^3 / pr
   if (al0 < b1) {
-    tmp = al0 * al0 * al0 / pr;
+    num = al0 * al0 * al0;
   } else if (al0 < b2) {
-    tmp = 0.5 * al0 * (al0 - b1) / (b2 * b3) + b1 * b1 * b1 / pr;
+    num = 0.5 * al0 * (al0 - b1);
+    den = b2 * b3;
   } else if (al0 < bm) {
-    tmp = (al0 * al0 * (3.0 * b12 - al0) + b1 * b1 * (b1 - 3.0 * al0) + b2 * b2 * (b2 - 3.0 * al0)) / pr;
+    num = al0 * al0 * (3.0 * b12 - al0) + b1 * b1 * (b1 - 3.0 * al0) + b2 * b2 * (b2 - 3.0 * al0);
   } else if (bm == b12) {
-    tmp = (al0 - 0.5 * bm) / b3;
+    num = al0 - 0.5 * bm;
+    den = b3;
   } else {
-    tmp = (al0 * al0 * (3.0 - 2.0 * al0) + b1 * b1 * (b1 - 3.0 * al0) + b2 * b2 * (b2 - 3.0 * al0) +
-           b3 * b3 * (b3 - 3.0 * al0)) / pr;
+    num = al0 * al0 * (3.0 - 2.0 * al0) + b1 * b1 * (b1 - 3.0 * al0) + b2 * b2 * (b2 - 3.0 * al0) +
+          b3 * b3 * (b3 - 3.0 * al0);
   }
+  tmp = num / den;
+  if (two) tmp = tmp + b1 * b1 * b1 / pr;
   return al <= 0.5 ? tmp * dr0 : (1.0 - tmp) * dr0;
 }
 
@@ -160,59 +170,80 @@ __device__ void iface_flux(size_t q, const double *__restrict__ us, const double
   else { n1 = mz; n2 = mx; n3 = my; }
   n1 = n1 / (1.0 - a1 + a2);
   alpha = alpha + n1 * a1;
-  if (a1 < 0.0) f1 = fl3d(n1, n2, n3, alpha, a1, -a1);
-  if (a2 > 0.0) f3 = fl3d(n1, n2, n3, alpha, 1.0, a2);
+  // The outflow at either end: in most cells there is one at most, so lanes
+  // with an outflow to the left and lanes with one to the right share a call.
+  const bool left = a1 < 0.0, right = a2 > 0.0;
+  if (left || right) {
+    const double f = fl3d(n1, n2, n3, alpha, left ? a1 : 1.0, left ? -a1 : a2);
+    if (left) f1 = f;
+    else f3 = f;
+  }
+  if (left && right) f3 = fl3d(n1, n2, n3, alpha, 1.0, a2);
   f2 = fl3d(n1, n2, n3, alpha, mm1, mm2);
   vof1[q] = f1;
   vof2[q] = f2;
   vof3[q] = f3;
 }
 
-// Sweep fluxes, pass 1: full and empty cells directly (the reference's
-// c == 1 and c == 0 branches); interface cells are appended to `list`
-// (one atomic per warp) for pass 2, so that the PLIC geometry runs on full
-// warps instead of one busy lane per warp.
+// Bits of the cells with c != +0, one word per 32 cells along x: word w of row
+// (j, k) at (k - 2) * (ny - 2) + (j - 2) rows of wpr = ceil((nx - 2) / 32).
+__host__ __device__ __forceinline__ int words_per_row(Dims d) { return (d.nx - 2 + 31) / 32; }
+
+constexpr int kScanRows = 4;  // rows a warp scans, all loaded before the first is used
+
+// Sweep, pass 1: the bits, the fluxes of full cells (the reference's c == 1
+// branch; zero for values that are neither positive nor +0) and the list of
+// interface cells (one atomic per warp), so that the PLIC geometry runs on
+// full warps instead of one busy lane per warp.
 template <int D>
-__global__ void k_swp_flux(const double *__restrict__ us, const double *__restrict__ cc,
-                           double *__restrict__ vof1, double *__restrict__ vof2, double *__restrict__ vof3, Dims d,
-                           double tauh, unsigned *__restrict__ list, unsigned *__restrict__ count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  const bool inside = i <= d.nx - 1 && j <= d.ny - 1;
-  const size_t q = inside ? d.ix(i, j, k) : 0;
-  const double c0 = inside ? cc[q] : 0.0;
-  const bool iface = inside && positive_bits(c0) && !is_one_bits(c0);
-  // warp-aggregated append (a warp is one x-row of the block)
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned mask = __ballot_sync(0xffffffffu, iface);
-  if (mask) {
-    unsigned base = 0;
-    const int leader = __ffs(mask) - 1;
-    if ((int)lane == leader) base = atomicAdd(count, (unsigned)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (iface) list[base + __popc(mask & ((1u << lane) - 1u))] = (unsigned)q;
+__global__ void k_swp_scan(const double *__restrict__ us, const double *__restrict__ cc, double *__restrict__ vof1,
+                           double *__restrict__ vof2, double *__restrict__ vof3, Dims d, double tauh,
+                           unsigned *__restrict__ bits, unsigned *__restrict__ list, unsigned *__restrict__ count) {
+  const int i = blockIdx.x * 32 + threadIdx.x + 2, k = blockIdx.z + 2;
+  const int j0 = (blockIdx.y * blockDim.y + threadIdx.y) * kScanRows + 2;
+  const unsigned lane = threadIdx.x;
+  double c[kScanRows];
+#pragma unroll
+  for (int r = 0; r < kScanRows; r++)
+    c[r] = i <= d.nx - 1 && j0 + r <= d.ny - 1 ? cc[d.ix(i, j0 + r, k)] : 0.0;
+  unsigned mask[kScanRows], total = 0, some = 0;
+#pragma unroll
+  for (int r = 0; r < kScanRows; r++) {
+    const unsigned any = __ballot_sync(0xffffffffu, !is_zero_bits(c[r]));
+    mask[r] = __ballot_sync(0xffffffffu, positive_bits(c[r]) && !is_one_bits(c[r]));
+    total += __popc(mask[r]);
+    some |= any;
+    if (lane == 0 && j0 + r <= d.ny - 1)
+      bits[((size_t)(k - 2) * (d.ny - 2) + (j0 + r - 2)) * words_per_row(d) + blockIdx.x] = any;
   }
-  if (!inside || iface) return;
-  if (!is_one_bits(c0)) {
-    // empty cell: no flux.  It returns before the velocity loads and the
-    // FP64 arithmetic of full cells, which the compiler otherwise if-converts
-    // so that every cell executes them (measured: 9 FP64 operations per cell
-    // and 279 us per y/z sweep at 256^3, against 101 us).
-    vof1[q] = 0.0;
-    vof2[q] = 0.0;
-    vof3[q] = 0.0;
-    return;
+  if (!some) return;
+  unsigned base = 0;
+  if (total) {
+    if (lane == 0) base = atomicAdd(count, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
   }
-  const long sd = D == 1 ? 1 : (D == 2 ? (long)d.sy() : (long)d.sz());
-  const double a1 = us[q] * tauh;
-  const double a2 = us[q + sd] * tauh;
-  vof1[q] = dmax1(-a1, 0.0);
-  vof2[q] = 1.0 - dmax1(a1, 0.0) + dmin1(a2, 0.0);
-  vof3[q] = dmax1(a2, 0.0);
+#pragma unroll
+  for (int r = 0; r < kScanRows; r++) {
+    const size_t q = d.ix(i, j0 + r, k);
+    const bool iface = mask[r] >> lane & 1u;
+    if (iface) list[base + __popc(mask[r] & ((1u << lane) - 1u))] = (unsigned)q;
+    base += __popc(mask[r]);
+    if (iface || is_zero_bits(c[r])) continue;  // lanes past the grid's end hold zeros
+    double f1 = 0.0, f2 = 0.0, f3 = 0.0;
+    if (is_one_bits(c[r])) {
+      const long sd = D == 1 ? 1 : (D == 2 ? (long)d.sy() : (long)d.sz());
+      const double a1 = us[q] * tauh, a2 = us[q + sd] * tauh;
+      f1 = dmax1(-a1, 0.0);
+      f2 = 1.0 - dmax1(a1, 0.0) + dmin1(a2, 0.0);
+      f3 = dmax1(a2, 0.0);
+    }
+    vof1[q] = f1;
+    vof2[q] = f2;
+    vof3[q] = f3;
+  }
 }
 
-// Sweep fluxes, pass 2: the listed interface cells, one per thread.
+// Pass 2: the listed interface cells, one per thread.
 template <int D>
 __global__ void k_swp_flux_iface(const unsigned *__restrict__ list, const unsigned *__restrict__ count,
                                  const double *__restrict__ us, const double *__restrict__ cc,
@@ -223,67 +254,104 @@ __global__ void k_swp_flux_iface(const unsigned *__restrict__ list, const unsign
     iface_flux<D>(list[t], us, cc, vof1, vof2, vof3, d, tauh);
 }
 
-// bc_flux: zero the ghost fluxes entering the domain along D.
+// Pass 3: c = vof3(-1) + vof2 + vof1(+1) along D clipped to [0,1], a missing
+// bit's fluxes being zero, and so those that enter through the domain's faces
+// (bc_flux, main.f:4496-4539).  A warp takes wpw words of the bits,
+// and its 32 lanes go together through those that have something to do.  The
+// list's length is reset for the next sweep.
 template <int D>
-__global__ void k_bc_flux(double *__restrict__ vof1, double *__restrict__ vof3, Dims d) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int q = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  if (D == 1) {
-    if (p > d.ny - 1 || q > d.nz - 1) return;
-    vof3[d.ix(1, p, q)] = 0.0;
-    vof1[d.ix(d.nx, p, q)] = 0.0;
-  } else if (D == 2) {
-    if (p > d.nx - 1 || q > d.nz - 1) return;
-    vof3[d.ix(p, 1, q)] = 0.0;
-    vof1[d.ix(p, d.ny, q)] = 0.0;
-  } else {
-    if (p > d.nx - 1 || q > d.ny - 1) return;
-    vof3[d.ix(p, q, 1)] = 0.0;
-    vof1[d.ix(p, q, d.nz)] = 0.0;
+__global__ void k_swp_update(double *__restrict__ cc, const double *__restrict__ vof1,
+                             const double *__restrict__ vof2, const double *__restrict__ vof3,
+                             const unsigned *__restrict__ bits, unsigned *__restrict__ count, Dims d, int wpw) {
+  const int wpr = words_per_row(d), ny2 = d.ny - 2;
+  const long long rows = (long long)ny2 * (d.nz - 2), words = rows * wpr;
+  const unsigned lane = threadIdx.x & 31;
+  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 32 * wpw, w = w0 + lane;
+  if (w == 0) *count = 0u;
+  unsigned own = 0, lo = 0, hi = 0;  // bits of a cell, its lower and its upper neighbour
+  if ((int)lane < wpw && w < words) {
+    own = bits[w];
+    const long long row = w / wpr;
+    const int x = (int)(w - row * wpr), j = (int)(row % ny2);
+    if (D == 1) {
+      lo = own << 1 | (x > 0 ? bits[w - 1] >> 31 : 0u);
+      hi = own >> 1 | (x + 1 < wpr ? bits[w + 1] << 31 : 0u);
+    } else if (D == 2) {
+      lo = j > 0 ? bits[w - wpr] : 0u;
+      hi = j + 1 < ny2 ? bits[w + wpr] : 0u;
+    } else {
+      lo = row >= ny2 ? bits[w - (long long)ny2 * wpr] : 0u;
+      hi = row + ny2 < rows ? bits[w + (long long)ny2 * wpr] : 0u;
+    }
+  }
+  const size_t sd = D == 1 ? 1 : (D == 2 ? d.sy() : d.sz());
+  unsigned busy = __ballot_sync(0xffffffffu, (own | lo | hi) != 0u);
+  while (busy) {
+    const int b = __ffs(busy) - 1;
+    busy &= busy - 1;
+    const unsigned o = __shfl_sync(0xffffffffu, own, b), l = __shfl_sync(0xffffffffu, lo, b),
+                   h = __shfl_sync(0xffffffffu, hi, b);
+    const long long row = (w0 + b) / wpr;
+    const int i = (int)(w0 + b - row * wpr) * 32 + (int)lane + 2;
+    if (i > d.nx - 1 || !((o | l | h) >> lane & 1u)) continue;
+    const size_t q = d.ix(i, (int)(row % ny2) + 2, (int)(row / ny2) + 2);
+    const double x = (l >> lane & 1u ? vof3[q - sd] : 0.0) + (o >> lane & 1u ? vof2[q] : 0.0) +
+                     (h >> lane & 1u ? vof1[q + sd] : 0.0);
+    // dmax1(0, dmin1(1, x)) on the bit patterns (same result for every non-NaN x)
+    const double y = __double_as_longlong(x) >= 0x3FF0000000000000LL ? 1.0 : x;
+    cc[q] = __double_as_longlong(y) <= 0LL ? 0.0 : y;
   }
 }
 
-template <int D>
-__global__ void k_swp_update(double *__restrict__ cc, const double *__restrict__ vof1,
-                             const double *__restrict__ vof2, const double *__restrict__ vof3, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  if (i > d.nx - 1 || j > d.ny - 1) return;
-  const size_t q = d.ix(i, j, k);
-  const size_t sd = D == 1 ? 1 : (D == 2 ? d.sy() : d.sz());
-  const double x = vof3[q - sd] + vof2[q] + vof1[q + sd];
-  // dmax1(0, dmin1(1, x)) on the bit patterns (same result for every non-NaN x)
-  const double y = __double_as_longlong(x) >= 0x3FF0000000000000LL ? 1.0 : x;
-  cc[q] = __double_as_longlong(y) <= 0LL ? 0.0 : y;
-}
-
-// bc_c, three ordered steps (main.f:4340-4395 without the dead filter block).
-__global__ void k_bc_c_x(double *__restrict__ cc, Dims d) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (j > d.ny || k > d.nz) return;
-  cc[d.ix(2, j, k)] = cc[d.ix(1, j, k)];
-  cc[d.ix(d.nx, j, k)] = cc[d.ix(d.nx - 1, j, k)];
-}
-
-__global__ void k_bc_c_y(double *__restrict__ cc, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  if (i > d.nx - 1 || k > d.nz - 1) return;
-  double x = cc[d.ix(i, 2, k)];
-  if (x > 1.0) x = 1.0;
-  if (x < 0.0) x = 0.0;
-  cc[d.ix(i, 1, k)] = x;
-  cc[d.ix(i, d.ny, k)] = cc[d.ix(i, d.ny - 1, k)];
-}
-
-__global__ void k_bc_c_z(double *__restrict__ cc, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (i > d.nx - 1 || j > d.ny) return;
-  cc[d.ix(i, j, 1)] = cc[d.ix(i, j, 2)];
-  cc[d.ix(i, j, d.nz)] = cc[d.ix(i, j, d.nz - 1)];
+// bc_c (main.f:4340-4395 without the dead filter block).  Its three ordered
+// steps -- x: plane 2 = plane 1, plane nx = plane nx-1; y: ghosts of i in
+// 2..nx-1 (the lower one clipped); z: likewise over all j -- in one launch: a
+// y or z ghost is a function of cells that no step writes (plane 1 in place of
+// plane 2).  The x step copies the old y and z ghosts of plane nx-1 to plane
+// nx; the threads that overwrite them do that first.
+__global__ void k_bc_c(double *__restrict__ cc, Dims d) {
+  const int face = blockIdx.z;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y * blockDim.y + threadIdx.y;
+  auto src = [&](int i, int j, int k) { return cc[d.ix(i == 2 ? 1 : i, j, k)]; };
+  if (face == 0) {  // p -> j, q -> k
+    const int j = p + 2, k = q + 2;
+    if (j > d.ny - 1 || k > d.nz - 1) return;
+    cc[d.ix(2, j, k)] = cc[d.ix(1, j, k)];
+    cc[d.ix(d.nx, j, k)] = cc[d.ix(d.nx - 1, j, k)];
+    return;
+  }
+  const int i = p + 2;
+  if (i > d.nx - 1) return;
+  const bool last = i == d.nx - 1;
+  if (face == 1) {  // q -> k
+    const int k = q + 2;
+    if (k > d.nz - 1) return;
+    if (last) {
+      cc[d.ix(d.nx, 1, k)] = cc[d.ix(i, 1, k)];
+      cc[d.ix(d.nx, d.ny, k)] = cc[d.ix(i, d.ny, k)];
+    }
+    double x = src(i, 2, k);
+    if (x > 1.0) x = 1.0;
+    if (x < 0.0) x = 0.0;
+    cc[d.ix(i, 1, k)] = x;
+    cc[d.ix(i, d.ny, k)] = src(i, d.ny - 1, k);
+    return;
+  }
+  const int j = q + 1;  // q -> j, ghost rows included
+  if (j > d.ny) return;
+  for (int s = 0; s < 2; s++) {
+    const int k = s ? d.nz : 1, kin = s ? d.nz - 1 : 2;
+    if (last) cc[d.ix(d.nx, j, k)] = cc[d.ix(i, j, k)];
+    double x;
+    if (j == 1) {
+      x = src(i, 2, kin);
+      if (x > 1.0) x = 1.0;
+      if (x < 0.0) x = 0.0;
+    } else {
+      x = src(i, j == d.ny ? d.ny - 1 : j, kin);
+    }
+    cc[d.ix(i, j, k)] = x;
+  }
 }
 
 // calcrho (main.f:2177-2190); for c = 0 and c = 1 the same operations are
@@ -311,22 +379,28 @@ const dim3 kBlk(32, 4, 1);
 template <int D>
 void sweep(const double *us, double *cc, double *v1, double *v2, double *v3, Dims d, double tauh, unsigned *list,
            unsigned *count, cudaStream_t st) {
-  cudaMemsetAsync(count, 0, sizeof(unsigned), st);
-  DSG_COUNT k_swp_flux<D><<<interior_grid(d, kBlk), kBlk, 0, st>>>(us, cc, v1, v2, v3, d, tauh, list, count);
-  DSG_COUNT k_swp_flux_iface<D><<<kRedBlocks, 128, 0, st>>>(list, count, us, cc, v1, v2, v3, d, tauh);
-  const dim3 b2(32, 8);
-  int p = D == 1 ? d.ny : d.nx, q = D == 3 ? d.ny : d.nz;
-  DSG_COUNT k_bc_flux<D><<<dim3((p + 31) / 32, (q + 7) / 8), b2, 0, st>>>(v1, v3, d);
-  DSG_COUNT k_swp_update<D><<<interior_grid(d, kBlk), kBlk, 0, st>>>(cc, v1, v2, v3, d);
+  unsigned *bits = list + (size_t)(d.nx - 2) * (d.ny - 2) * (d.nz - 2);
+  const int wpr = words_per_row(d), rows = 4 * kScanRows;
+  DSG_COUNT k_swp_scan<D><<<dim3((unsigned)wpr, (unsigned)((d.ny - 2 + rows - 1) / rows), (unsigned)(d.nz - 2)), kBlk,
+                            0, st>>>(us, cc, v1, v2, v3, d, tauh, bits, list, count);
+  // One warp per block: a cell is some thousand FP64 operations in sequence,
+  // and warps on one SM share its FP64 pipe, so a short list goes to as many
+  // SMs as it has warps (64^3 droplet: 36 us, 40 us with four warps per block).
+  DSG_COUNT k_swp_flux_iface<D><<<4 * kRedBlocks, 32, 0, st>>>(list, count, us, cc, v1, v2, v3, d, tauh);
+  const size_t words = (size_t)wpr * (d.ny - 2) * (d.nz - 2);
+  // Words per warp: on small grids few, because a warp goes through its busy
+  // words one after the other (64^3: 4 us with 4, 12 us with 32); on large ones
+  // more, because most warps find nothing to do (256^3: 19 us with 4, 13 with 32).
+  const int wpw = words < ((size_t)1 << 17) ? 4 : 16;
+  DSG_COUNT k_swp_update<D><<<(unsigned)((words + 4 * wpw - 1) / (4 * wpw)), 128, 0, st>>>(cc, v1, v2, v3, bits, count,
+                                                                                          d, wpw);
 }
 
 }  // namespace
 
 cudaError_t bc_c(double *cc, Dims d, cudaStream_t st) {
-  const dim3 b2(32, 8);
-  DSG_COUNT k_bc_c_x<<<dim3((d.ny + 31) / 32, (d.nz + 7) / 8), b2, 0, st>>>(cc, d);
-  DSG_COUNT k_bc_c_y<<<dim3((d.nx + 31) / 32, (d.nz + 7) / 8), b2, 0, st>>>(cc, d);
-  DSG_COUNT k_bc_c_z<<<dim3((d.nx + 31) / 32, (d.ny + 7) / 8), b2, 0, st>>>(cc, d);
+  const int p = d.nx > d.ny ? d.nx : d.ny, q = d.ny > d.nz ? d.ny : d.nz;
+  DSG_COUNT k_bc_c<<<dim3((p + 31) / 32, (q + 7) / 8, 3), dim3(32, 8), 0, st>>>(cc, d);
   return cudaGetLastError();
 }
 
