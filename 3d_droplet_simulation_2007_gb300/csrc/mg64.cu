@@ -39,48 +39,49 @@ __global__ void k_bc_scalar(double *__restrict__ s, Dims d) {
   s[d.ix(i, j, k)] = s[d.ix(ci, cj, ck)];
 }
 
-// bc_resid step 1 (main.f:4441-4446): x faces over all j,k, reading cell 2 / nx-1.
-__global__ void k_bc_xcopy(double *__restrict__ s, Dims d) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (j > d.ny || k > d.nz) return;
-  s[d.ix(1, j, k)] = s[d.ix(2, j, k)];
-  s[d.ix(d.nx, j, k)] = s[d.ix(d.nx - 1, j, k)];
-}
-
-// bc_resid steps 2-3 (main.f:4450-4461): y and z ghosts of interior i set to 0.
-__global__ void k_bc_resid_yz(double *__restrict__ s, Dims d) {
-  const int face = blockIdx.z;  // 0: y (i, k in 2..nz-1), 1: z (i, all j)
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int q = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (i > d.nx - 1) return;
-  if (face == 0) {
-    if (q < 2 || q > d.nz - 1) return;
-    s[d.ix(i, 1, q)] = 0.0;
-    s[d.ix(i, d.ny, q)] = 0.0;
-  } else {
-    if (q > d.ny) return;
-    s[d.ix(i, q, 1)] = 0.0;
-    s[d.ix(i, q, d.nz)] = 0.0;
+// bc_resid (main.f:4441-4461: plane 1 = plane 2 and plane nx = plane nx-1 over
+// all j, k, then the y and z ghosts of interior i = 0) and bc_out
+// (main.f:4406-4427: the same x step, then every y ghost, all i, and the z
+// ghosts of interior i from the adjacent cell), their ordered steps in one
+// launch.  The x step copies old ghosts of planes 2 and nx-1 that the z step
+// (bc_resid: and the y step) overwrites; the threads that overwrite them copy
+// them first.
+template <bool ZERO>
+__global__ void k_bc_copy(double *__restrict__ s, Dims d) {
+  const int face = blockIdx.z;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y * blockDim.y + threadIdx.y;
+  if (face == 0) {  // p -> j, q -> k
+    const int j = p + 2, k = q + 2;
+    if (j > d.ny - 1 || k > d.nz - 1) return;
+    s[d.ix(1, j, k)] = s[d.ix(2, j, k)];
+    s[d.ix(d.nx, j, k)] = s[d.ix(d.nx - 1, j, k)];
+    return;
   }
-}
-
-// bc_out step 2 (main.f:4413-4418): y faces, all i, interior k.
-__global__ void k_bc_out_y(double *__restrict__ s, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  if (i > d.nx || k > d.nz - 1) return;
-  s[d.ix(i, 1, k)] = s[d.ix(i, 2, k)];
-  s[d.ix(i, d.ny, k)] = s[d.ix(i, d.ny - 1, k)];
-}
-
-// bc_out step 3 (main.f:4422-4427): z faces, interior i, all j.
-__global__ void k_bc_out_z(double *__restrict__ s, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  auto put = [&](int i, int j, int k, double x) {
+    const size_t n = d.ix(i, j, k);
+    const double old = s[n];
+    if (i == 2) s[n - 1] = old;
+    if (i == d.nx - 1) s[n + 1] = old;
+    s[n] = x;
+  };
+  if (face == 1) {  // p -> i, q -> k
+    const int i = p + (ZERO ? 2 : 1), k = q + 2;
+    if (i > d.nx - (ZERO ? 1 : 0) || k > d.nz - 1) return;
+    if (ZERO) {
+      put(i, 1, k, 0.0);
+      put(i, d.ny, k, 0.0);
+    } else {
+      const int ci = i == 1 ? 2 : (i == d.nx ? d.nx - 1 : i);
+      s[d.ix(i, 1, k)] = s[d.ix(ci, 2, k)];
+      s[d.ix(i, d.ny, k)] = s[d.ix(ci, d.ny - 1, k)];
+    }
+    return;
+  }
+  const int i = p + 2, j = q + 1;  // ghost rows included
   if (i > d.nx - 1 || j > d.ny) return;
-  s[d.ix(i, j, 1)] = s[d.ix(i, j, 2)];
-  s[d.ix(i, j, d.nz)] = s[d.ix(i, j, d.nz - 1)];
+  const int cj = j == 1 ? 2 : (j == d.ny ? d.ny - 1 : j);
+  put(i, j, 1, ZERO ? 0.0 : s[d.ix(i, cj, 2)]);
+  put(i, j, d.nz, ZERO ? 0.0 : s[d.ix(i, cj, d.nz - 1)]);
 }
 
 // ---- relax: one colour pass (main.f:3973-3992) ----------------------------
@@ -601,19 +602,18 @@ cudaError_t bc_scalar(double *s, Dims d, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+static dim3 bc_grid(Dims d) {
+  const int p = d.nx > d.ny ? d.nx : d.ny, q = d.ny > d.nz ? d.ny : d.nz;
+  return dim3((unsigned)((p + 31) / 32), (unsigned)((q + 7) / 8), 3);
+}
+
 cudaError_t bc_resid(double *s, Dims d, cudaStream_t st) {
-  const dim3 blk(32, 8);
-  DSG_COUNT k_bc_xcopy<<<dim3((d.ny + 31) / 32, (d.nz + 7) / 8), blk, 0, st>>>(s, d);
-  const int m = d.ny > d.nz ? d.ny : d.nz;
-  DSG_COUNT k_bc_resid_yz<<<dim3((d.nx + 31) / 32, (m + 7) / 8, 2), blk, 0, st>>>(s, d);
+  DSG_COUNT k_bc_copy<true><<<bc_grid(d), dim3(32, 8), 0, st>>>(s, d);
   return cudaGetLastError();
 }
 
 cudaError_t bc_out(double *s, Dims d, cudaStream_t st) {
-  const dim3 blk(32, 8);
-  DSG_COUNT k_bc_xcopy<<<dim3((d.ny + 31) / 32, (d.nz + 7) / 8), blk, 0, st>>>(s, d);
-  DSG_COUNT k_bc_out_y<<<dim3((d.nx + 31) / 32, (d.nz + 7) / 8), blk, 0, st>>>(s, d);
-  DSG_COUNT k_bc_out_z<<<dim3((d.nx + 31) / 32, (d.ny + 7) / 8), blk, 0, st>>>(s, d);
+  DSG_COUNT k_bc_copy<false><<<bc_grid(d), dim3(32, 8), 0, st>>>(s, d);
   return cudaGetLastError();
 }
 

@@ -157,60 +157,76 @@ __global__ void k_project(double *__restrict__ u, double *__restrict__ v, double
 }
 
 // ---- bc_v (main.f:4064-4141) ---------------------------------------------------
-__global__ void k_bcv_1(double *__restrict__ u, double *__restrict__ v, double *__restrict__ w, Dims d,
-                        double xvel2) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (j > d.ny || k > d.nz) return;
-  const int jj = j == 1 ? 2 : j;
-  const double x = (jj * 1.0 - 1.5) / (d.ny * 1.0 - 1.5) - 1.0;
-  const double val = xvel2 * (-(x * x) + 1.0);
-  u[d.ix(1, j, k)] = j == 1 ? -val : val;
-  v[d.ix(d.nx, j, k)] = v[d.ix(d.nx - 1, j, k)];
-  w[d.ix(d.nx, j, k)] = w[d.ix(d.nx - 1, j, k)];
+//
+// The ordered steps of bc_v and bc_w (x planes, y planes, z planes) in one
+// launch each.  A y or z ghost is a function of interior cells that no step
+// writes or of constants; where the x step copies a value that a later step
+// overwrites (plane nx-1's ghosts and zero planes into plane nx), the thread
+// that overwrites it copies it first.  Their fourth step, plane 2 from plane 1,
+// comes with the outlet sums, because y and z ghosts are formed from plane 2
+// before it.
+__global__ void k_bcv(double *__restrict__ u, double *__restrict__ v, double *__restrict__ w, Dims d, double xvel2) {
+  const int face = blockIdx.z;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y * blockDim.y + threadIdx.y;
+  if (face == 0) {  // p -> j, q -> k, all of them for the inflow
+    const int j = p + 1, k = q + 1;
+    if (j > d.ny || k > d.nz) return;
+    const int jj = j == 1 ? 2 : j;
+    const double x = (jj * 1.0 - 1.5) / (d.ny * 1.0 - 1.5) - 1.0;
+    const double val = xvel2 * (-(x * x) + 1.0);
+    u[d.ix(1, j, k)] = j == 1 ? -val : val;
+    const bool kin = k >= 2 && k <= d.nz - 1;
+    // v: rows 1, 2 and ny and planes 1 and nz of plane nx-1 change below; w:
+    // rows 1 and ny and planes 2 and nz
+    if (j >= 3 && j <= d.ny - 1 && kin) v[d.ix(d.nx, j, k)] = v[d.ix(d.nx - 1, j, k)];
+    if (j >= 2 && j <= d.ny - 1 && (k == 1 || (k >= 3 && k <= d.nz - 1)))
+      w[d.ix(d.nx, j, k)] = w[d.ix(d.nx - 1, j, k)];
+    if ((j == 1 || j == d.ny) && k == 1) w[d.ix(d.nx, j, k)] = w[d.ix(d.nx - 1, j, k)];
+    return;
+  }
+  const int i = p + 2;
+  if (i > d.nx - 1) return;
+  const bool last = i == d.nx - 1;
+  auto put = [&](double *f, int j, int k, double x) {
+    const size_t n = d.ix(i, j, k);
+    if (last) f[n + 1] = f[n];
+    f[n] = x;
+  };
+  if (face == 1) {  // q -> k
+    const int k = q + 2;
+    if (k > d.nz - 1) return;
+    u[d.ix(i, 1, k)] = -u[d.ix(i, 2, k)];
+    u[d.ix(i, d.ny, k)] = u[d.ix(i, d.ny - 1, k)];
+    put(v, 2, k, 0.0);
+    put(v, 1, k, 0.0);
+    put(v, d.ny, k, 0.0);
+    if (k == 2) return;  // w's plane 2 is the z step's
+    put(w, 1, k, -w[d.ix(i, 2, k)]);
+    put(w, d.ny, k, w[d.ix(i, d.ny - 1, k)]);
+    return;
+  }
+  const int j = q + 1;  // q -> j, ghost rows included
+  if (j > d.ny) return;
+  for (int s = 0; s < 2; s++) {
+    const int k = s ? d.nz : 1, kin = s ? d.nz - 1 : 2;
+    u[d.ix(i, j, k)] = j == 1 ? -u[d.ix(i, 2, kin)] : u[d.ix(i, j == d.ny ? d.ny - 1 : j, kin)];
+    put(v, j, k, j <= 2 || j == d.ny ? 0.0 : v[d.ix(i, j, kin)]);
+  }
+  put(w, j, 2, 0.0);
+  put(w, j, d.nz, 0.0);
 }
 
-__global__ void k_bcv_2(double *__restrict__ u, double *__restrict__ v, double *__restrict__ w, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  if (i > d.nx - 1 || k > d.nz - 1) return;
-  u[d.ix(i, 1, k)] = -u[d.ix(i, 2, k)];
-  u[d.ix(i, d.ny, k)] = u[d.ix(i, d.ny - 1, k)];
-  v[d.ix(i, 2, k)] = 0.0;
-  v[d.ix(i, 1, k)] = 0.0;
-  v[d.ix(i, d.ny, k)] = 0.0;
-  w[d.ix(i, 1, k)] = -w[d.ix(i, 2, k)];
-  w[d.ix(i, d.ny, k)] = w[d.ix(i, d.ny - 1, k)];
-}
-
-__global__ void k_bcv_3(double *__restrict__ u, double *__restrict__ v, double *__restrict__ w, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (i > d.nx - 1 || j > d.ny) return;
-  u[d.ix(i, j, 1)] = u[d.ix(i, j, 2)];
-  u[d.ix(i, j, d.nz)] = u[d.ix(i, j, d.nz - 1)];
-  v[d.ix(i, j, 1)] = v[d.ix(i, j, 2)];
-  v[d.ix(i, j, d.nz)] = v[d.ix(i, j, d.nz - 1)];
-  w[d.ix(i, j, 2)] = 0.0;
-  w[d.ix(i, j, d.nz)] = 0.0;
-}
-
-// x2(2,j,k) = x1(1,j,k) over interior j,k (bc_v/bc_w step 4 copies).
-__global__ void k_copy_inflow(double *__restrict__ dst, const double *__restrict__ src, int dst_i, Dims d) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  if (j > d.ny - 1 || k > d.nz - 1) return;
-  dst[d.ix(dst_i, j, k)] = src[d.ix(1, j, k)];
-}
-
-// Sums of f0(1,j,k) and f1(nx-1,j,k) over interior j,k (deterministic order).
-__global__ void k_outlet_partial(double *__restrict__ partials, const double *__restrict__ f0,
-                                 const double *__restrict__ f1, Dims d) {
+// Sums of f0(1,j,k) and f1(nx-1,j,k) over interior j,k (deterministic order),
+// and f1's planes 2 (and with `one` 1) = f0's plane 1 there.
+__global__ void k_outlet_partial(double *__restrict__ partials, const double *f0, double *f1, bool one, Dims d) {
   const size_t n = (size_t)(d.ny - 2) * (d.nz - 2);
   double s0 = 0.0, s1 = 0.0;
   for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
     const int j = (int)(t % (size_t)(d.ny - 2)) + 2, k = (int)(t / (size_t)(d.ny - 2)) + 2;
-    s0 += f0[d.ix(1, j, k)];
+    const double in = f0[d.ix(1, j, k)];
+    if (one) f1[d.ix(1, j, k)] = in;
+    f1[d.ix(2, j, k)] = in;
+    s0 += in;
     s1 += f1[d.ix(d.nx - 1, j, k)];
   }
   __shared__ double sh0[256], sh1[256];
@@ -254,43 +270,47 @@ __global__ void k_outlet_apply(double *__restrict__ x, const double *__restrict_
 }
 
 // ---- bc_w (main.f:4143-4220) ---------------------------------------------------
-__global__ void k_bcw_1(double *__restrict__ w2, double *__restrict__ w3, const double *__restrict__ v,
-                        const double *__restrict__ w, Dims d) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  if (j > d.ny - 1 || k > d.nz - 1) return;
-  const double v1 = v[d.ix(1, j, k)], wv1 = w[d.ix(1, j, k)];
-  w2[d.ix(1, j, k)] = v1;
-  w2[d.ix(2, j, k)] = v1;
-  w2[d.ix(d.nx, j, k)] = v[d.ix(d.nx, j, k)];
-  w3[d.ix(1, j, k)] = wv1;
-  w3[d.ix(2, j, k)] = wv1;
-  w3[d.ix(d.nx, j, k)] = w[d.ix(d.nx, j, k)];
-}
-
-__global__ void k_bcw_2(double *__restrict__ w1, double *__restrict__ w2, double *__restrict__ w3,
-                        const double *__restrict__ v, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int k = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  if (i > d.nx - 1 || k > d.nz - 1) return;
-  w1[d.ix(i, 1, k)] = -w1[d.ix(i, 2, k)];
-  w1[d.ix(i, d.ny, k)] = w1[d.ix(i, d.ny - 1, k)];
-  w2[d.ix(i, 1, k)] = 0.0;
-  w2[d.ix(i, 2, k)] = 0.0;
-  w2[d.ix(i, d.ny, k)] = v[d.ix(i, d.ny, k)];
-  w3[d.ix(i, 1, k)] = -w3[d.ix(i, 2, k)];
-  w3[d.ix(i, d.ny, k)] = w3[d.ix(i, d.ny - 1, k)];
-}
-
-__global__ void k_bcw_3(double *__restrict__ w1, double *__restrict__ w2, double *__restrict__ w3,
-                        const double *__restrict__ w, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  if (i > d.nx - 1 || j > d.ny) return;
-  w1[d.ix(i, j, 1)] = w1[d.ix(i, j, 2)];
-  w1[d.ix(i, j, d.nz)] = w1[d.ix(i, j, d.nz - 1)];
-  w2[d.ix(i, j, 1)] = w2[d.ix(i, j, 2)];
-  w2[d.ix(i, j, d.nz)] = w2[d.ix(i, j, d.nz - 1)];
+__global__ void k_bcw(double *__restrict__ w1, double *__restrict__ w2, double *__restrict__ w3,
+                      const double *__restrict__ v, const double *__restrict__ w, Dims d) {
+  const int face = blockIdx.z;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y * blockDim.y + threadIdx.y;
+  if (face == 0) {  // p -> j, q -> k
+    const int j = p + 2, k = q + 2;
+    if (j > d.ny - 1 || k > d.nz - 1) return;
+    const double v1 = v[d.ix(1, j, k)], wv1 = w[d.ix(1, j, k)];
+    w2[d.ix(1, j, k)] = v1;
+    if (j > 2) w2[d.ix(2, j, k)] = v1;  // row 2 is the y step's
+    w2[d.ix(d.nx, j, k)] = v[d.ix(d.nx, j, k)];
+    w3[d.ix(1, j, k)] = wv1;
+    if (k > 2) w3[d.ix(2, j, k)] = wv1;  // plane 2 is the z step's
+    w3[d.ix(d.nx, j, k)] = w[d.ix(d.nx, j, k)];
+    return;
+  }
+  const int i = p + 2;
+  if (i > d.nx - 1) return;
+  // w2 and w3 of an interior cell after the x step
+  auto in2 = [&](int j, int k) { return i == 2 ? v[d.ix(1, j, k)] : w2[d.ix(i, j, k)]; };
+  auto in3 = [&](int j, int k) { return i == 2 ? w[d.ix(1, j, k)] : w3[d.ix(i, j, k)]; };
+  if (face == 1) {  // q -> k
+    const int k = q + 2;
+    if (k > d.nz - 1) return;
+    w1[d.ix(i, 1, k)] = -w1[d.ix(i, 2, k)];
+    w1[d.ix(i, d.ny, k)] = w1[d.ix(i, d.ny - 1, k)];
+    w2[d.ix(i, 1, k)] = 0.0;
+    w2[d.ix(i, 2, k)] = 0.0;
+    w2[d.ix(i, d.ny, k)] = v[d.ix(i, d.ny, k)];
+    if (k == 2) return;
+    w3[d.ix(i, 1, k)] = -in3(2, k);
+    w3[d.ix(i, d.ny, k)] = in3(d.ny - 1, k);
+    return;
+  }
+  const int j = q + 1;  // q -> j, ghost rows included
+  if (j > d.ny) return;
+  for (int s = 0; s < 2; s++) {
+    const int k = s ? d.nz : 1, kin = s ? d.nz - 1 : 2;
+    w1[d.ix(i, j, k)] = j == 1 ? -w1[d.ix(i, 2, kin)] : w1[d.ix(i, j == d.ny ? d.ny - 1 : j, kin)];
+    w2[d.ix(i, j, k)] = j <= 2 ? 0.0 : (j == d.ny ? v[d.ix(i, d.ny, kin)] : in2(j, kin));
+  }
   const double wb = w[d.ix(i, j, 1)];
   w3[d.ix(i, j, 1)] = wb;
   w3[d.ix(i, j, 2)] = wb;
@@ -302,32 +322,30 @@ const dim3 kFace(32, 8, 1);
 
 inline dim3 fgrid(int p, int q) { return dim3((unsigned)((p + 31) / 32), (unsigned)((q + 7) / 8)); }
 
+inline dim3 fgrid3(Dims d) {
+  const int p = d.nx > d.ny ? d.nx : d.ny, q = d.ny > d.nz ? d.ny : d.nz;
+  return dim3((unsigned)((p + 31) / 32), (unsigned)((q + 7) / 8), 3);
+}
+
 // Outlet flux balance shared by bc_v and bc_w: x(nx,j,k) = x(nx-1,j,k) + vout - vout2
 // with vout the mean of u(1,j,k) and vout2 the mean of x(nx-1,j,k).
-void outlet(double *x, const double *u, double *partials, Dims d, cudaStream_t st) {
-  DSG_COUNT k_outlet_partial<<<kOutletBlocks, 256, 0, st>>>(partials, u, x, d);
+void outlet(double *x, const double *u, bool one, double *partials, Dims d, cudaStream_t st) {
+  DSG_COUNT k_outlet_partial<<<kOutletBlocks, 256, 0, st>>>(partials, u, x, one, d);
   DSG_COUNT k_outlet_apply<<<fgrid(d.ny, d.nz), kFace, 0, st>>>(x, partials, d);
 }
 
 }  // namespace
 
 cudaError_t bc_v(double *u, double *v, double *w, double *partials, Dims d, double xvel2, cudaStream_t st) {
-  DSG_COUNT k_bcv_1<<<fgrid(d.ny, d.nz), kFace, 0, st>>>(u, v, w, d, xvel2);
-  DSG_COUNT k_bcv_2<<<fgrid(d.nx, d.nz), kFace, 0, st>>>(u, v, w, d);
-  DSG_COUNT k_bcv_3<<<fgrid(d.nx, d.ny), kFace, 0, st>>>(u, v, w, d);
-  DSG_COUNT k_copy_inflow<<<fgrid(d.ny, d.nz), kFace, 0, st>>>(u, u, 2, d);
-  outlet(u, u, partials, d, st);
+  DSG_COUNT k_bcv<<<fgrid3(d), kFace, 0, st>>>(u, v, w, d, xvel2);
+  outlet(u, u, false, partials, d, st);
   return cudaGetLastError();
 }
 
 cudaError_t bc_w(double *w1, double *w2, double *w3, const double *u, const double *v, const double *w,
                  double *partials, Dims d, cudaStream_t st) {
-  DSG_COUNT k_bcw_1<<<fgrid(d.ny, d.nz), kFace, 0, st>>>(w2, w3, v, w, d);
-  DSG_COUNT k_bcw_2<<<fgrid(d.nx, d.nz), kFace, 0, st>>>(w1, w2, w3, v, d);
-  DSG_COUNT k_bcw_3<<<fgrid(d.nx, d.ny), kFace, 0, st>>>(w1, w2, w3, w, d);
-  DSG_COUNT k_copy_inflow<<<fgrid(d.ny, d.nz), kFace, 0, st>>>(w1, u, 1, d);
-  DSG_COUNT k_copy_inflow<<<fgrid(d.ny, d.nz), kFace, 0, st>>>(w1, u, 2, d);
-  outlet(w1, u, partials, d, st);
+  DSG_COUNT k_bcw<<<fgrid3(d), kFace, 0, st>>>(w1, w2, w3, v, w, d);
+  outlet(w1, u, true, partials, d, st);
   return cudaGetLastError();
 }
 
