@@ -197,10 +197,8 @@ int vcycle(dsg_ctx *ctx, int j) {
     double **L = ctx->lv[jj];
     const Dims d = ctx->level(jj);
     DSG_CK(ctx, relax_level(ctx, ctx->s.npre, jj, ls));
-    DSG_CK(ctx, dsg::resid(ls, L[2], L[1], L[3], L[4], L[5], L[6], d, st, fp64_fma(ctx)));
-    const Dims dc = ctx->level(jj - 1);
-    DSG_CK(ctx, dsg::rstrct(ctx->lv[jj - 1][3], L[2], dc, st));
-    if (jj - 1 != jt) DSG_CK(ctx, dsg::fill_zero(ctx->lv[jj - 1][1], dc.count(), st));
+    DSG_CK(ctx, dsg::resid_rstrct(ls, ctx->lv[jj - 1][3], ctx->lv[jj - 1][1], L[1], L[3], L[4], L[5], L[6], d, st,
+                                  fp64_fma(ctx)));
   }
   if (jt >= 1) {
     int rc = coarse64(ctx, false);
@@ -211,7 +209,9 @@ int vcycle(dsg_ctx *ctx, int j) {
   for (int jj = jt >= 1 ? jt + 1 : 2; jj <= j; jj++) {
     double **L = ctx->lv[jj];
     const Dims d = ctx->level(jj);
-    DSG_CK(ctx, dsg::addint(L[1], ctx->lv[jj - 1][1], L[2], d, st));
+    // the finest level's residual array keeps addint's values: its ghosts
+    // are read in the next step's momentum phase
+    DSG_CK(ctx, dsg::addint(L[1], ctx->lv[jj - 1][1], jj == ctx->ng ? L[2] : nullptr, d, st));
     DSG_CK(ctx, relax_level(ctx, ctx->s.npost, jj, ls));
   }
   return DSG_OK;

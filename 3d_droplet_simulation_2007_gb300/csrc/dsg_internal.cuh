@@ -107,6 +107,9 @@ cudaError_t relax_n(int n, double *u, double lengthsize, const double *rhs, cons
                     cudaStream_t st, bool fma = false);
 cudaError_t resid(double lengthsize, double *res, const double *u, const double *rhs, const double *a,
                   const double *b, const double *c, Dims d, cudaStream_t st, bool fma = false);
+// resid (virtual ghosts) and rstrct in one pass, the coarse correction zeroed
+cudaError_t resid_rstrct(double lengthsize, double *rhs_c, double *u_c, const double *u, const double *rhs,
+                         const double *a, const double *b, const double *c, Dims df, cudaStream_t st, bool fma);
 cudaError_t rstrct(double *uc, const double *uf, Dims dc, cudaStream_t st);
 cudaError_t interp(double *uf, const double *uc, Dims df, cudaStream_t st);
 cudaError_t addint(double *uf, const double *uc, double *res, Dims df, cudaStream_t st);

@@ -72,6 +72,7 @@ __global__ void k_prolong32(float *__restrict__ uf, const float *__restrict__ uc
 // Arithmetic of the cluster kernel on the FP32 levels.
 struct Cluster32 {
   typedef float T;
+  typedef Cluster32 First;  // of the first coarsest solve
   static constexpr int kMaxCells = kCluster32Cells;
   static __device__ __forceinline__ float relax(float uc, float xp, float xm, float yp, float ym, float zp, float zm,
                                                 float ae, float aw, float bn, float bs, float ct, float cb, float ei,

@@ -11,6 +11,8 @@
 // All arithmetic keeps the reference's operation order; this file is built
 // without FMA contraction so results are bit-identical to a non-contracting
 // Fortran build.
+#include <cmath>
+
 #include "dsg_internal.cuh"
 
 namespace dsg {
@@ -85,14 +87,70 @@ __global__ void k_bc_copy(double *__restrict__ s, Dims d) {
 }
 
 // ---- relax: one colour pass (main.f:3973-3992) ----------------------------
+// How an update is rounded.
+// REF: the reference's operation order, no contraction (17 FP64 operations
+// per cell, bit-identical to the oracle).
+// REF2: the same bits in 15 operations, where h2 and 1 - omega are plus or
+// minus powers of two (2^k cells along x; the reference's omega = 1.5): their
+// products are exact, so a fused multiply-add rounds exactly once where the
+// separate multiply and add did.
+// FMA: the same sum as a fused multiply-add chain and the update written as
+// u + omega*(temp - u) (10 operations).
+// GB300's FP64 pipe bounds the REF forms, so the operation count sets their
+// speed (128^3 pass: 39.1 us with 17, 34.6 with 15).
+enum Round { REF, REF2, FMA };
+
+template <Round R>
+__device__ __forceinline__ double relax_value(double uc, double xp, double xm, double yp, double ym, double zp,
+                                              double zm, double ae, double aw, double bn, double bs, double ct,
+                                              double cb, double ei, double rhs, double h2, double omega) {
+  if (R == FMA) {
+    double t = ae * xp;
+    t = __fma_rn(aw, xm, t);
+    t = __fma_rn(bn, yp, t);
+    t = __fma_rn(bs, ym, t);
+    t = __fma_rn(ct, zp, t);
+    t = __fma_rn(cb, zm, t);
+    t = __fma_rn(-h2, rhs, t) * ei;
+    return __fma_rn(omega, t - uc, uc);
+  }
+  const double sum = ae * xp + aw * xm + bn * yp + bs * ym + ct * zp + cb * zm;
+  if (R == REF2) return __fma_rn(1.0 - omega, uc, omega * (__fma_rn(-h2, rhs, sum) * ei));
+  return omega * ((sum - h2 * rhs) * ei) + (1.0 - omega) * uc;
+}
+
+// Residual of a cell, rhs - (1/h^2) sum a_nb (u_nb - u) (main.f:3912-3925).
+template <Round R>
+__device__ __forceinline__ double resid_value(double uc, double xp, double xm, double yp, double ym, double zp,
+                                              double zm, double ae, double aw, double bn, double bs, double ct,
+                                              double cb, double rhs, double h2i) {
+  if (R == FMA) {
+    double t = ae * (xp - uc);
+    t = __fma_rn(aw, xm - uc, t);
+    t = __fma_rn(bn, yp - uc, t);
+    t = __fma_rn(bs, ym - uc, t);
+    t = __fma_rn(ct, zp - uc, t);
+    t = __fma_rn(cb, zm - uc, t);
+    return __fma_rn(-h2i, t, rhs);
+  }
+  const double sum = ae * (xp - uc) + aw * (xm - uc) + bn * (yp - uc) + bs * (ym - uc) + ct * (zp - uc) +
+                     cb * (zm - uc);
+  if (R == REF2) return __fma_rn(-h2i, sum, rhs);
+  return -h2i * sum + rhs;
+}
+
+// |x| is a power of two in the range where its product with a value of the
+// fields stays exact (no overflow or underflow for magnitudes in 2^+-600).
+bool power_of_two(double x) {
+  int e;
+  return std::isfinite(x) && x != 0.0 && std::fabs(std::frexp(x, &e)) == 0.5 && e > -300 && e < 300;
+}
+
 // colour 0 updates i+j+k even (first pass), colour 1 odd.  Thread (t, j, k)
 // updates i = i0 + 2t.  Ghost neighbours are virtual (see file header).
-// FMA = false: the reference's operation order, no contraction (17 FP64
-// operations per cell, bit-identical to the oracle).  FMA = true: the same
-// sum as a fused multiply-add chain and the update written as
-// u + omega*(temp - u) (10 FP64 operations); GB300's FP64 pipe, not HBM,
-// bounds this kernel, so the operation count sets its speed.
-template <bool FMA>
+// GHOSTS: the cells at the boundary also write the ghosts they determine (the
+// last sweep of a block, in place of a bc_scalar launch).
+template <Round R, bool GHOSTS>
 __global__ void k_relax_colour(double *__restrict__ u, const double *__restrict__ rhs,
                                const double *__restrict__ a, const double *__restrict__ b,
                                const double *__restrict__ c, const double *__restrict__ ei, Dims d,
@@ -105,66 +163,44 @@ __global__ void k_relax_colour(double *__restrict__ u, const double *__restrict_
   const size_t q = d.ix(i, j, k);
   const size_t sy = d.sy(), sz = d.sz();
   const double uc = u[q];
-  const double uxp = (i + 1 == d.nx) ? 0.0 : u[q + 1];
-  const double uxm = (i - 1 == 1) ? uc : u[q - 1];
-  const double uyp = (j + 1 == d.ny) ? uc : u[q + sy];
-  const double uym = (j - 1 == 1) ? uc : u[q - sy];
-  const double uzp = (k + 1 == d.nz) ? uc : u[q + sz];
-  const double uzm = (k - 1 == 1) ? uc : u[q - sz];
-  if (FMA) {
-    double t = a[q] * uxp;
-    t = __fma_rn(a[q - 1], uxm, t);
-    t = __fma_rn(b[q], uyp, t);
-    t = __fma_rn(b[q - sy], uym, t);
-    t = __fma_rn(c[q], uzp, t);
-    t = __fma_rn(c[q - sz], uzm, t);
-    t = __fma_rn(-h2, rhs[q], t) * ei[q];
-    u[q] = __fma_rn(omega, t - uc, uc);
-    return;
+  const double xp = (i + 1 == d.nx) ? 0.0 : u[q + 1];
+  const double xm = (i - 1 == 1) ? uc : u[q - 1];
+  const double yp = (j + 1 == d.ny) ? uc : u[q + sy];
+  const double ym = (j - 1 == 1) ? uc : u[q - sy];
+  const double zp = (k + 1 == d.nz) ? uc : u[q + sz];
+  const double zm = (k - 1 == 1) ? uc : u[q - sz];
+  const double v = relax_value<R>(uc, xp, xm, yp, ym, zp, zm, a[q], a[q - 1], b[q], b[q - sy], c[q], c[q - sz], ei[q],
+                                  rhs[q], h2, omega);
+  u[q] = v;
+  if (GHOSTS) {
+    // ghosts whose nearest interior cell this is: 1 = v, nx = 0 along x; the
+    // cell's own value along y and z
+    const int i0 = i == 2 ? 1 : i, i1 = i == d.nx - 1 ? d.nx : i;
+    const int j0 = j == 2 ? 1 : j, j1 = j == d.ny - 1 ? d.ny : j;
+    const int k0 = k == 2 ? 1 : k, k1 = k == d.nz - 1 ? d.nz : k;
+    if (i0 == i1 && j0 == j1 && k0 == k1) return;
+    for (int kk = k0; kk <= k1; kk++)
+      for (int jj = j0; jj <= j1; jj++)
+        for (int ii = i0; ii <= i1; ii++)
+          if (ii != i || jj != j || kk != k) u[d.ix(ii, jj, kk)] = ii == d.nx ? 0.0 : v;
   }
-  const double temp = (a[q] * uxp + a[q - 1] * uxm + b[q] * uyp + b[q - sy] * uym + c[q] * uzp +
-                       c[q - sz] * uzm - h2 * rhs[q]) *
-                      ei[q];
-  u[q] = omega * temp + (1.0 - omega) * uc;
 }
 
 // Arithmetic of the cluster kernel on the FP64 levels: the two forms of
 // k_relax_colour and k_resid, and rstrct's and interp's transfers.
-template <bool FMA>
+template <Round R>
 struct Cluster64 {
   typedef double T;
+  // the first coarsest solve has lengthscale for its spacing, no power of two
+  typedef Cluster64<R == REF2 ? REF : R> First;
   static constexpr int kMaxCells = kCluster64Cells;
-  static __device__ __forceinline__ double relax(double uc, double xp, double xm, double yp, double ym, double zp,
-                                                 double zm, double ae, double aw, double bn, double bs, double ct,
-                                                 double cb, double ei, double rhs, double h2, double omega) {
-    if (FMA) {
-      double t = ae * xp;
-      t = __fma_rn(aw, xm, t);
-      t = __fma_rn(bn, yp, t);
-      t = __fma_rn(bs, ym, t);
-      t = __fma_rn(ct, zp, t);
-      t = __fma_rn(cb, zm, t);
-      t = __fma_rn(-h2, rhs, t) * ei;
-      return __fma_rn(omega, t - uc, uc);
-    }
-    const double temp = (ae * xp + aw * xm + bn * yp + bs * ym + ct * zp + cb * zm - h2 * rhs) * ei;
-    return omega * temp + (1.0 - omega) * uc;
+  template <class... X>
+  static __device__ __forceinline__ double relax(X... x) {
+    return relax_value<R>(x...);
   }
-  static __device__ __forceinline__ double resid(double uc, double xp, double xm, double yp, double ym, double zp,
-                                                 double zm, double ae, double aw, double bn, double bs, double ct,
-                                                 double cb, double rhs, double h2i) {
-    if (FMA) {
-      double t = ae * (xp - uc);
-      t = __fma_rn(aw, xm - uc, t);
-      t = __fma_rn(bn, yp - uc, t);
-      t = __fma_rn(bs, ym - uc, t);
-      t = __fma_rn(ct, zp - uc, t);
-      t = __fma_rn(cb, zm - uc, t);
-      return __fma_rn(-h2i, t, rhs);
-    }
-    return -h2i * (ae * (xp - uc) + aw * (xm - uc) + bn * (yp - uc) + bs * (ym - uc) + ct * (zp - uc) +
-                   cb * (zm - uc)) +
-           rhs;
+  template <class... X>
+  static __device__ __forceinline__ double resid(X... x) {
+    return resid_value<R>(x...);
   }
   static __device__ __forceinline__ double mean8(double r0, double r1, double r2, double r3, double r4, double r5,
                                                  double r6, double r7) {
@@ -176,35 +212,23 @@ struct Cluster64 {
   }
 };
 
-template <bool FMA>
+template <Round R>
 __global__ void __launch_bounds__(mgc::kThreads, 1) k_cluster64(const __grid_constant__ mgc::Args<double> G) {
-  mgc::cluster_mg<Cluster64<FMA>>(G);
+  mgc::cluster_mg<Cluster64<R>>(G);
 }
 
-// Residual of one interior cell, rhs - (1/h^2) sum a_nb (u_nb - u) (main.f:3912-3925),
-// in the reference's order or as a fused multiply-add chain.
-template <bool FMA>
+// Residual of an interior cell, its neighbours' values from memory.
+template <Round R>
 __device__ __forceinline__ double cell_resid(const double *__restrict__ u, const double *__restrict__ rhs,
                                              const double *__restrict__ a, const double *__restrict__ b,
                                              const double *__restrict__ c, size_t q, size_t sy, size_t sz,
                                              double h2i) {
-  const double uc = u[q];
-  if (FMA) {
-    double t = a[q] * (u[q + 1] - uc);
-    t = __fma_rn(a[q - 1], u[q - 1] - uc, t);
-    t = __fma_rn(b[q], u[q + sy] - uc, t);
-    t = __fma_rn(b[q - sy], u[q - sy] - uc, t);
-    t = __fma_rn(c[q], u[q + sz] - uc, t);
-    t = __fma_rn(c[q - sz], u[q - sz] - uc, t);
-    return __fma_rn(-h2i, t, rhs[q]);
-  }
-  return -h2i * (a[q] * (u[q + 1] - uc) + a[q - 1] * (u[q - 1] - uc) + b[q] * (u[q + sy] - uc) +
-                 b[q - sy] * (u[q - sy] - uc) + c[q] * (u[q + sz] - uc) + c[q - sz] * (u[q - sz] - uc)) +
-         rhs[q];
+  return resid_value<R>(u[q], u[q + 1], u[q - 1], u[q + sy], u[q - sy], u[q + sz], u[q - sz], a[q], a[q - 1], b[q],
+                        b[q - sy], c[q], c[q - sz], rhs[q], h2i);
 }
 
 // ---- resid (main.f:3912-3925), reads the ghosts from memory ----------------
-template <bool FMA>
+template <Round R>
 __global__ void k_resid(double *__restrict__ res, const double *__restrict__ u,
                         const double *__restrict__ rhs, const double *__restrict__ a,
                         const double *__restrict__ b, const double *__restrict__ c, Dims d,
@@ -214,7 +238,44 @@ __global__ void k_resid(double *__restrict__ res, const double *__restrict__ u,
   const int k = blockIdx.z + 2;
   if (i > d.nx - 1 || j > d.ny - 1) return;
   const size_t q = d.ix(i, j, k);
-  res[q] = cell_resid<FMA>(u, rhs, a, b, c, q, d.sy(), d.sz(), h2i);
+  res[q] = cell_resid<R>(u, rhs, a, b, c, q, d.sy(), d.sz(), h2i);
+}
+
+// ---- resid and rstrct in one pass (main.f:3718-3726) -----------------------
+// Coarse right-hand side = mean of the 8 fine residuals, coarse correction = 0
+// (interiors; the sweeps read ghosts virtually).  The residual itself is not
+// stored.  A thread forms the four residuals of fine column i in a coarse
+// cell's y-z square, and the even lane of a pair adds the pair's eight in
+// rstrct's order (128^3: 83 us, one pass where resid, its ghosts, rstrct and
+// the zeroing took 79 + 6 + 20 us and a residual array).
+template <Round R>
+__global__ void k_resid_rstrct(double *__restrict__ rhs_c, double *__restrict__ u_c, const double *__restrict__ u,
+                               const double *__restrict__ rhs, const double *__restrict__ a,
+                               const double *__restrict__ b, const double *__restrict__ c, Dims dc, Dims df,
+                               double h2i) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;  // fine column; blockDim.x = 32
+  const int jc = blockIdx.y * blockDim.y + threadIdx.y + 2, kc = blockIdx.z + 2;
+  if (jc > dc.ny - 1) return;
+  const size_t sy = df.sy(), sz = df.sz();
+  double r[4] = {0.0, 0.0, 0.0, 0.0};
+  if (i <= df.nx - 1) {
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int j = 2 * jc - 2 + (m & 1), k = 2 * kc - 2 + (m >> 1);
+      const size_t q = df.ix(i, j, k);
+      const double uc = u[q];
+      r[m] = resid_value<R>(uc, i + 1 == df.nx ? 0.0 : u[q + 1], i == 2 ? uc : u[q - 1], j + 1 == df.ny ? uc : u[q + sy],
+                            j == 2 ? uc : u[q - sy], k + 1 == df.nz ? uc : u[q + sz], k == 2 ? uc : u[q - sz], a[q],
+                            a[q - 1], b[q], b[q - sy], c[q], c[q - sz], rhs[q], h2i);
+    }
+  }
+  double o[4];
+#pragma unroll
+  for (int m = 0; m < 4; m++) o[m] = __shfl_down_sync(0xffffffffu, r[m], 1);
+  if ((i & 1) || i > df.nx - 1) return;
+  const size_t qc = dc.ix(i / 2 + 1, jc, kc);
+  rhs_c[qc] = 0.125 * (r[0] + o[0] + r[1] + o[1] + r[2] + o[2] + r[3] + o[3]);
+  u_c[qc] = 0.0;
 }
 
 // ---- rstrct fused with the coarse bc_scalar (main.f:3765-3791) ------------
@@ -255,6 +316,7 @@ __global__ void k_interp(double *__restrict__ uf, const double *__restrict__ uc,
 }
 
 // ---- addint: res = interp(uc) (+bc_scalar); uf += res everywhere ----------
+// (res may be null where no one reads it)
 __global__ void k_addint(double *__restrict__ uf, double *__restrict__ res, const double *__restrict__ uc,
                          Dims df, Dims dc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
@@ -269,7 +331,7 @@ __global__ void k_addint(double *__restrict__ uf, double *__restrict__ res, cons
     x = uc[dc.ix((ci >> 1) + 1, (cj >> 1) + 1, (ck >> 1) + 1)];
   }
   const size_t q = df.ix(i, j, k);
-  res[q] = x;
+  if (res) res[q] = x;
   uf[q] = uf[q] + x;
 }
 
@@ -517,7 +579,7 @@ __device__ __forceinline__ long long abs_bits(double x) {
   return __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFLL;
 }
 
-template <bool FMA>
+template <bool F>
 __global__ void k_relres_partial(double *__restrict__ partials, const double *__restrict__ u,
                                  const double *__restrict__ rhs, const double *__restrict__ a,
                                  const double *__restrict__ b, const double *__restrict__ c, Dims d,
@@ -528,8 +590,8 @@ __global__ void k_relres_partial(double *__restrict__ partials, const double *__
   for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
     int i, j, k;
     const size_t q = interior_cell(t, d, i, j, k);
-    const double r = cell_resid<FMA>(u, rhs, a, b, c, q, sy, sz, h2i);
-    if (FMA) {
+    const double r = cell_resid<F ? FMA : REF>(u, rhs, a, b, c, q, sy, sz, h2i);
+    if (F) {
       v[0] = __fma_rn(r, r, v[0]);
       v[1] = __fma_rn(rhs[q], rhs[q], v[1]);
     } else {
@@ -617,26 +679,37 @@ cudaError_t bc_out(double *s, Dims d, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-static void relax_passes(double *u, double h2, const double *rhs, const double *a, const double *b,
-                         const double *c, const double *ei, Dims d, double omega, bool fma, cudaStream_t st) {
+// The form of the sweeps and residuals on spacing h2: the fused multiply-add
+// chain, or the reference's rounding in as few operations as h2 and omega allow.
+static Round rounding(bool fma, double h2, double omega) {
+  return fma ? FMA : (power_of_two(h2) && power_of_two(1.0 - omega) ? REF2 : REF);
+}
+
+template <Round R>
+static void relax_passes(int n, double *u, double h2, const double *rhs, const double *a, const double *b,
+                         const double *c, const double *ei, Dims d, double omega, cudaStream_t st) {
   const int half = (d.nx - 2 + 1) / 2;
   const dim3 grid((unsigned)((half + kBlk.x - 1) / kBlk.x), (unsigned)((d.ny - 2 + kBlk.y - 1) / kBlk.y),
                   (unsigned)(d.nz - 2));
-  for (int colour = 0; colour < 2; colour++) {
-    if (fma)
-      DSG_COUNT k_relax_colour<true><<<grid, kBlk, 0, st>>>(u, rhs, a, b, c, ei, d, h2, omega, colour);
-    else
-      DSG_COUNT k_relax_colour<false><<<grid, kBlk, 0, st>>>(u, rhs, a, b, c, ei, d, h2, omega, colour);
-  }
+  for (int q = 0; q < n; q++)
+    for (int colour = 0; colour < 2; colour++) {
+      if (q == n - 1)
+        DSG_COUNT k_relax_colour<R, true><<<grid, kBlk, 0, st>>>(u, rhs, a, b, c, ei, d, h2, omega, colour);
+      else
+        DSG_COUNT k_relax_colour<R, false><<<grid, kBlk, 0, st>>>(u, rhs, a, b, c, ei, d, h2, omega, colour);
+    }
 }
 
 int cluster64_size() {
-  const int n = mgc::cluster_size(k_cluster64<false>);
-  return mgc::cluster_size(k_cluster64<true>) < n ? 0 : n;
+  const int n = mgc::cluster_size(k_cluster64<REF>);
+  return mgc::cluster_size(k_cluster64<REF2>) < n || mgc::cluster_size(k_cluster64<FMA>) < n ? 0 : n;
 }
 
 cudaError_t cluster64(const mgc::Args<double> &args, bool fma, cudaStream_t st) {
-  return fma ? mgc::launch(k_cluster64<true>, args, st) : mgc::launch(k_cluster64<false>, args, st);
+  Round r = rounding(fma, args.lv[1].h2, args.omega);
+  for (int l = 2; l <= args.top && r == REF2; l++) r = rounding(fma, args.lv[l].h2, args.omega);
+  return r == FMA ? mgc::launch(k_cluster64<FMA>, args, st)
+                  : (r == REF2 ? mgc::launch(k_cluster64<REF2>, args, st) : mgc::launch(k_cluster64<REF>, args, st));
 }
 
 cudaError_t relax(double *u, double lengthsize, const double *rhs, const double *a, const double *b,
@@ -650,19 +723,38 @@ cudaError_t relax_n(int n, double *u, double lengthsize, const double *rhs, cons
   if (n <= 0) return cudaSuccess;
   const double h1 = lengthsize / (d.nx - 2);
   const double h2 = h1 * h1;
-  for (int q = 0; q < n; q++) relax_passes(u, h2, rhs, a, b, c, ei, d, omega, fma, st);
-  return bc_scalar(u, d, st);
+  switch (rounding(fma, h2, omega)) {
+    case FMA: relax_passes<FMA>(n, u, h2, rhs, a, b, c, ei, d, omega, st); break;
+    case REF2: relax_passes<REF2>(n, u, h2, rhs, a, b, c, ei, d, omega, st); break;
+    default: relax_passes<REF>(n, u, h2, rhs, a, b, c, ei, d, omega, st);
+  }
+  return cudaGetLastError();
 }
 
 cudaError_t resid(double lengthsize, double *res, const double *u, const double *rhs, const double *a,
                   const double *b, const double *c, Dims d, cudaStream_t st, bool fma) {
   const double h1 = lengthsize / (d.nx - 2);
   const double h2i = 1.0 / (h1 * h1);
-  if (fma)
-    DSG_COUNT k_resid<true><<<interior_grid(d, kBlk), kBlk, 0, st>>>(res, u, rhs, a, b, c, d, h2i);
-  else
-    DSG_COUNT k_resid<false><<<interior_grid(d, kBlk), kBlk, 0, st>>>(res, u, rhs, a, b, c, d, h2i);
+  switch (rounding(fma, h2i, 1.5)) {
+    case FMA: DSG_COUNT k_resid<FMA><<<interior_grid(d, kBlk), kBlk, 0, st>>>(res, u, rhs, a, b, c, d, h2i); break;
+    case REF2: DSG_COUNT k_resid<REF2><<<interior_grid(d, kBlk), kBlk, 0, st>>>(res, u, rhs, a, b, c, d, h2i); break;
+    default: DSG_COUNT k_resid<REF><<<interior_grid(d, kBlk), kBlk, 0, st>>>(res, u, rhs, a, b, c, d, h2i);
+  }
   return bc_resid(res, d, st);
+}
+
+cudaError_t resid_rstrct(double lengthsize, double *rhs_c, double *u_c, const double *u, const double *rhs,
+                         const double *a, const double *b, const double *c, Dims df, cudaStream_t st, bool fma) {
+  const double h1 = lengthsize / (df.nx - 2);
+  const double h2i = 1.0 / (h1 * h1);
+  const Dims dc{df.nx / 2 + 1, df.ny / 2 + 1, df.nz / 2 + 1};
+  const dim3 grid((unsigned)((df.nx - 2 + 31) / 32), (unsigned)((dc.ny - 2 + 3) / 4), (unsigned)(dc.nz - 2));
+  switch (rounding(fma, h2i, 1.5)) {
+    case FMA: DSG_COUNT k_resid_rstrct<FMA><<<grid, kBlk, 0, st>>>(rhs_c, u_c, u, rhs, a, b, c, dc, df, h2i); break;
+    case REF2: DSG_COUNT k_resid_rstrct<REF2><<<grid, kBlk, 0, st>>>(rhs_c, u_c, u, rhs, a, b, c, dc, df, h2i); break;
+    default: DSG_COUNT k_resid_rstrct<REF><<<grid, kBlk, 0, st>>>(rhs_c, u_c, u, rhs, a, b, c, dc, df, h2i);
+  }
+  return cudaGetLastError();
 }
 
 cudaError_t rstrct(double *uc, const double *uf, Dims dc, cudaStream_t st) {

@@ -577,7 +577,7 @@ __device__ void cluster_mg(const Args<typename A::T> &params) {
   zero_u(G.lv[G.fmg ? 1 : G.top]);
   cluster_barrier();
   if (G.fmg) {
-    smooth_level<A>(1, rank, G.ntop, G.h2_first, false, p);
+    smooth_level<typename A::First>(1, rank, G.ntop, G.h2_first, false, p);
     for (int j = 2; j <= G.top; j++) {
       phase_barrier(G.lv[j], G.lv[j - 1]);
       prolong_level<A>(G.lv[j], G.lv[j - 1], rank, G.o_buf, 0, G.tri);
