@@ -56,11 +56,12 @@ struct Entry {
 };
 
 // Argument sets of the batched passes (the parameters of the block bodies).
-struct ARelaxSplit { float *u[2]; float *r[2]; const float *cc; Dims d; Split sp; float h2, omega, r1, r2; };
+struct ARelaxSplit { float *u[2]; float *r[2]; const float *cc; const unsigned char *flags; Dims d; Split sp; float h2, omega, r1, r2; };
 struct ARelax { float *u; const float *rhs, *a, *b, *c, *ei; Dims d; float h2, omega; };
 struct ARRSplit {
   float *rhs_c, *u_c;
   const float *ue, *uo, *re, *ro, *cc;
+  const unsigned char *flags;
   Dims df;
   Split sp;
   Dims dc;
@@ -80,7 +81,8 @@ struct ADefect {
 };
 struct AFold { const double *partials; double *out; };
 struct AZero { float *p; size_t n; };
-struct ATo32 { float *dst; const double *src; size_t n; };
+struct ACodes { float *dst; unsigned char *codes; const double *src; Dims d; };
+struct AFlags { unsigned char *flags; const unsigned char *codes; Dims d; };
 struct AAcf64 { float *a, *b, *c, *ei; const double *a2, *b2, *c2; Dims dc, df; };
 struct AAcf32 { float *a, *b, *c, *ei; const float *a2, *b2, *c2; Dims dc, df; };
 struct ASplit64 { float *ev, *od; const double *src; Dims d; Split sp; };
@@ -145,8 +147,12 @@ unsigned launch_grid(unsigned total, unsigned threads) {
 
 __global__ void kb_relax32_split(BATCH_PARAMS(ARelaxSplit), int colour) {
   FOR_MEMBER_BLOCKS(ARelaxSplit) {
-    b_relax32_split(B, G, a.u[colour], a.u[1 - colour], a.r[colour], a.cc, a.d, a.sp, colour, a.h2, a.omega, a.r1,
-                    a.r2);
+    float *self = a.u[colour];
+    const float *other = a.u[1 - colour];
+    if (split_vec(a.sp))
+      b_relax32_split<true>(B, G, self, other, a.r[colour], a.cc, a.flags, a.d, a.sp, colour, a.h2, a.omega, a.r1, a.r2);
+    else
+      b_relax32_split<false>(B, G, self, other, a.r[colour], a.cc, a.flags, a.d, a.sp, colour, a.h2, a.omega, a.r1, a.r2);
   });
 }
 
@@ -156,8 +162,12 @@ __global__ void kb_relax32(BATCH_PARAMS(ARelax), int colour) {
 
 __global__ void kb_resid_restrict32_split(BATCH_PARAMS(ARRSplit)) {
   FOR_MEMBER_BLOCKS(ARRSplit) {
-    b_resid_restrict32_split(B, G, a.rhs_c, a.u_c, a.ue, a.uo, a.re, a.ro, a.cc, a.df, a.sp, a.dc, a.h2i, a.r1,
-                             a.r2);
+    if (split_vec(a.sp))
+      b_resid_restrict32_split<true>(B, G, a.rhs_c, a.u_c, a.ue, a.uo, a.re, a.ro, a.cc, a.flags, a.df, a.sp, a.dc,
+                                     a.h2i, a.r1, a.r2);
+    else
+      b_resid_restrict32_split<false>(B, G, a.rhs_c, a.u_c, a.ue, a.uo, a.re, a.ro, a.cc, a.flags, a.df, a.sp, a.dc,
+                                      a.h2i, a.r1, a.r2);
   });
 }
 
@@ -206,8 +216,12 @@ __global__ void kb_zero32(BATCH_PARAMS(AZero)) {
   });
 }
 
-__global__ void kb_to32(BATCH_PARAMS(ATo32)) {
-  FOR_MEMBER_BLOCKS(ATo32) { b_to32(B, G, a.dst, a.src, a.n); });
+__global__ void kb_codes(BATCH_PARAMS(ACodes)) {
+  FOR_MEMBER_BLOCKS(ACodes) { b_codes(B, G, a.dst, a.codes, a.src, a.d); });
+}
+
+__global__ void kb_flags(BATCH_PARAMS(AFlags)) {
+  FOR_MEMBER_BLOCKS(AFlags) { b_flags(B, G, a.flags, a.codes, a.d); });
 }
 
 __global__ void kb_acfromac64to32(BATCH_PARAMS(AAcf64)) {
@@ -243,7 +257,7 @@ static_assert(sizeof(Table<ARelaxSplit>) <= 32000 && sizeof(Table<ARRSplit>) <= 
 
 enum Kind {
   K_RELAX_SPLIT, K_RELAX, K_RR_SPLIT, K_RR, K_PRO_SPLIT, K_PRO, K_TAIL, K_CORRECT, K_DEFECT, K_FOLD, K_ZERO,
-  K_TO32, K_ACF64, K_ACF32, K_SPLIT64, K_RESTR_SPLIT, K_RESTR, K_KINDS
+  K_CODES, K_FLAGS, K_ACF64, K_ACF32, K_SPLIT64, K_RESTR_SPLIT, K_RESTR, K_KINDS
 };
 
 // Kinds whose block shape the autotuner may change (independent cells).
@@ -336,8 +350,8 @@ struct TableBuilder {
 dim3 grid_of(int k, const Dims &d, dim3 blk) {
   switch (k) {
     case K_RELAX_SPLIT: {
-      const int hx = (d.nx - 2) >> 1;
-      return dim3(cdiv(hx, 2 * blk.x), cdiv(d.ny - 2, blk.y), d.nz - 2);
+      const Split sp{(d.nx - 2) >> 1, d.ny - 2, d.nz - 2};
+      return dim3(cdiv(sp.hx, split_cells(sp, blk.x)), cdiv(d.ny - 2, blk.y), d.nz - 2);
     }
     case K_RELAX: {
       const int half = (d.nx - 2 + 1) / 2;
@@ -424,7 +438,7 @@ struct Planner {
         FineSplit f = fine_split(c);
         float r1, r2;
         phase_coefs(c, &r1, &r2);
-        ARelaxSplit a{{f.u[0], f.u[1]}, {f.r[0], f.r[1]}, c->lv32[l][A32], d,
+        ARelaxSplit a{{f.u[0], f.u[1]}, {f.r[0], f.r[1]}, c->lv32[l][A32], c->seg_flags, d,
                       Split{(d.nx - 2) >> 1, d.ny - 2, d.nz - 2}, level_h2(c, l), omega32(c), r1, r2};
         ts.add((int)i, grid_of(K_RELAX_SPLIT, d, bs), nsw[i], a);
       } else {
@@ -458,7 +472,7 @@ struct Planner {
         FineSplit f = fine_split(c);
         float r1, r2;
         phase_coefs(c, &r1, &r2);
-        ARRSplit a{Lc[RHS32], Lc[U32], f.u[0], f.u[1], f.r[0], f.r[1], L[A32], df,
+        ARRSplit a{Lc[RHS32], Lc[U32], f.u[0], f.u[1], f.r[0], f.r[1], L[A32], c->seg_flags, df,
                    Split{(df.nx - 2) >> 1, df.ny - 2, df.nz - 2}, dc, 1.0f / level_h2(c, l), r1, r2};
         ts.add((int)i, grid_of(K_RR_SPLIT, dc, bs), 1, a);
       } else {
@@ -572,13 +586,17 @@ struct Planner {
     int maxng = 0;
     for (auto &x : mp) maxng = std::max(maxng, x.ng);
     {  // FP32 fine cc, coarse coefficients
-      TableBuilder<ATo32> t;
+      TableBuilder<ACodes> t;
+      TableBuilder<AFlags> tf;
       for (size_t i = 0; i < n; i++) {
         dsg_ctx *c = mp[i].c;
-        const size_t cnt = c->fine().count();
-        t.add((int)i, dim3(std::min(cdiv(cnt, 256), 8192u)), 1, ATo32{c->lv32[c->ng][A32], c->lv[c->ng][0], cnt});
+        const Dims d = c->fine();
+        t.add((int)i, dim3(std::min(cdiv(32 * segment_codes(d), 256), 8192u)), 1,
+              ACodes{c->lv32[c->ng][A32], c->seg_codes, c->lv[c->ng][0], d});
+        tf.add((int)i, dim3(std::min(cdiv(segment_flags(d), 256), 8192u)), 1, AFlags{c->seg_flags, c->seg_codes, d});
       }
-      emit(out, K_TO32, t, dim3(256), 0, 0, 0, 0, 0, -1);
+      emit(out, K_CODES, t, dim3(256), 0, 0, 0, 0, 0, -1);
+      emit(out, K_FLAGS, tf, dim3(256), 0, 0, 0, 0, 0, -1);
     }
     {
       TableBuilder<AAcf64> t;
@@ -737,7 +755,8 @@ cudaError_t launch(const BatchSolve &b, const Launch &L, cudaStream_t st) {
     case K_DEFECT: return launch_table<ADefect>(kb_defect64, L, gate, st);
     case K_FOLD: return launch_table<AFold>(kb_fold2, L, gate, st);
     case K_ZERO: return launch_table<AZero>(kb_zero32, L, gate, st);
-    case K_TO32: return launch_table<ATo32>(kb_to32, L, gate, st);
+    case K_CODES: return launch_table<ACodes>(kb_codes, L, gate, st);
+    case K_FLAGS: return launch_table<AFlags>(kb_flags, L, gate, st);
     case K_ACF64: return launch_table<AAcf64>(kb_acfromac64to32, L, gate, st);
     case K_ACF32: return launch_table<AAcf32>(kb_acfromac32, L, gate, st);
     case K_SPLIT64: return launch_table<ASplit64>(kb_split_from64, L, gate, st);

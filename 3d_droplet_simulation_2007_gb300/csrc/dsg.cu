@@ -256,7 +256,8 @@ cudaError_t relax32_level(dsg_ctx *ctx, int n, int l) {
     float r1, r2;
     phase_coefs(ctx, &r1, &r2);
     cudaError_t e =
-        dsg::relax32_split_n(n, f.u, f.r, L[A32], d, level_h2(ctx, l), omega32(ctx), r1, r2, ctx->stream);
+        dsg::relax32_split_n(n, f.u, f.r, L[A32], ctx->seg_flags, d, level_h2(ctx, l), omega32(ctx), r1, r2,
+                             ctx->stream);
     if (e != cudaSuccess) return e;
     return cudaEventRecordWithFlags(e1, ctx->stream, cudaEventRecordExternal);
   }
@@ -277,7 +278,8 @@ cudaError_t relax32_level(dsg_ctx *ctx, int n, int l) {
     FineSplit f = fine_split(ctx);
     float r1, r2;
     phase_coefs(ctx, &r1, &r2);
-    e = dsg::relax32_split_n(n, f.u, f.r, L[A32], d, level_h2(ctx, l), omega32(ctx), r1, r2, ctx->stream);
+    e = dsg::relax32_split_n(n, f.u, f.r, L[A32], ctx->seg_flags, d, level_h2(ctx, l), omega32(ctx), r1, r2,
+                             ctx->stream);
   } else {
     e = dsg::relax32_n(n, L[U32], level_h2(ctx, l), L[RHS32], L[A32], L[B32], L[C32], L[EI32], d,
                        omega32(ctx), ctx->stream);
@@ -336,7 +338,7 @@ int vcycle32(dsg_ctx *ctx, int j) {
     DSG_CK(ctx, relax32_level(ctx, pre32(ctx, jj), jj));
     if (jj == ng) {
       FineSplit f = fine_split(ctx);
-      DSG_CK(ctx, dsg::resid_restrict32_split(Lc[RHS32], Lc[U32], f.u, f.r, L[A32], ctx->level(jj),
+      DSG_CK(ctx, dsg::resid_restrict32_split(Lc[RHS32], Lc[U32], f.u, f.r, L[A32], ctx->seg_flags, ctx->level(jj),
                                               1.0f / level_h2(ctx, jj), r1, r2, st));
     } else {
       DSG_CK(ctx, dsg::resid_restrict32(Lc[RHS32], Lc[U32], L[U32], L[RHS32], L[A32], L[B32], L[C32],
@@ -464,7 +466,7 @@ bool graph_matches(const GraphRec &g, const int key[6]) {
 int coef_hierarchy32(dsg_ctx *ctx, cudaStream_t st) {
   const int ng = ctx->ng;
   double **F = ctx->lv[ng];
-  DSG_CK(ctx, dsg::to32(ctx->lv32[ng][A32], F[0], ctx->fine().count(), st));
+  DSG_CK(ctx, dsg::to32_flags(ctx->lv32[ng][A32], ctx->seg_flags, ctx->seg_codes, F[0], ctx->fine(), st));
   if (ng >= 2) {
     float **C = ctx->lv32[ng - 1];
     DSG_CK(ctx, dsg::acfromac64to32(C[A32], C[B32], C[C32], C[EI32], F[4], F[5], F[6], ctx->level(ng - 1), st));
@@ -905,6 +907,8 @@ int dsg_create(const dsg_config *cfg, dsg_ctx **out) {
   total += nextra * fine;
   total += up(dsg::kRedBlocks * 4 * sizeof(double)) + up(16 * sizeof(double)) + up(sizeof(unsigned long long)) +
            up(sizeof(unsigned)) + up(dsg::kRedBlocks * 6 * sizeof(double)) + up(16 * sizeof(double));
+  const Dims fd{cfg->nx, cfg->ny, cfg->nz};
+  total += up(dsg::segment_flags(fd)) + up(dsg::segment_codes(fd));
   cudaError_t e = cudaMalloc(&ctx->arena, total);
   if (e != cudaSuccess) {
     int rc = dsg::cuda_fail(ctx, e, "cudaMalloc(arena)");
@@ -944,6 +948,10 @@ int dsg_create(const dsg_config *cfg, dsg_ctx **out) {
   ctx->gcr_partials = (double *)p;
   p += up(dsg::kRedBlocks * 6 * sizeof(double));
   ctx->gcr_coef = (double *)p;
+  p += up(16 * sizeof(double));
+  ctx->seg_flags = (unsigned char *)p;
+  p += up(dsg::segment_flags(fd));
+  ctx->seg_codes = (unsigned char *)p;
   e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->red_host, 16 * sizeof(double));
   if (e == cudaSuccess) e = cudaMemsetAsync(ctx->arena, 0, total, ctx->own_stream);

@@ -219,10 +219,13 @@ int cluster64_size();
 cudaError_t cluster32(const mgc::Args<float> &args, cudaStream_t st);
 cudaError_t cluster64(const mgc::Args<double> &args, bool fma, cudaStream_t st);
 // finest level in colour-split storage ({even, odd} arrays of (nx-2)/2 x (ny-2) x (nz-2))
-cudaError_t relax32_split_n(int n, float *const u[2], float *const rhs[2], const float *cc, Dims d, float h2,
-                            float omega, float r1, float r2, cudaStream_t st);
+// (flags: of the uniform segments, to32_flags)
+cudaError_t relax32_split_n(int n, float *const u[2], float *const rhs[2], const float *cc,
+                            const unsigned char *flags, Dims d, float h2, float omega, float r1, float r2,
+                            cudaStream_t st);
 cudaError_t resid_restrict32_split(float *rhs_c, float *u_c, float *const u[2], float *const rhs[2], const float *cc,
-                                   Dims df, float h2i, float r1, float r2, cudaStream_t st);
+                                   const unsigned char *flags, Dims df, float h2i, float r1, float r2,
+                                   cudaStream_t st);
 cudaError_t prolong32_split(float *const u[2], const float *uc, Dims df, int add, int tri, cudaStream_t st);
 cudaError_t restrict32_split(float *uc, float *const rhs[2], Dims dc, cudaStream_t st);
 cudaError_t split_from64(float *const dst[2], const double *src, Dims d, cudaStream_t st);
@@ -230,7 +233,12 @@ cudaError_t defect64(float *const r32[2], double *out2, double *partials, const 
                      const double *a, const double *b, const double *c, const double *diag, Dims d,
                      double lengthsize, cudaStream_t st);
 cudaError_t correct64(double *p, float *const e[2], Dims d, int init, cudaStream_t st);
-cudaError_t to32(float *dst, const double *src, size_t n, cudaStream_t st);
+// FP32 volume fraction of all nodes, and the flags of the finest level's
+// uniform segments (codes: scratch), segment_flags / segment_codes bytes
+size_t segment_codes(Dims d);
+size_t segment_flags(Dims d);
+cudaError_t to32_flags(float *dst, unsigned char *flags, unsigned char *codes, const double *src, Dims d,
+                       cudaStream_t st);
 // One GCR iteration of the mixed solve on the finest level, after the V-cycle
 // that left z = M r in the split correction arrays: w = A z, the step
 // lengths, then (not last) d, q, r and p updated, or (last) p += alpha d.
@@ -303,6 +311,8 @@ struct dsg_ctx {
   double *f[DSG_NFIELDS];     // fine fields; 0..7 alias lv[ng]
   double *ccf;                // csf filtered volume fraction (local array of csf)
   double *diag64;             // sum of the six fine face coefficients (the mixed solve's defect)
+  unsigned char *seg_flags;   // uniform segments of the finest FP32 level, and the codes they come from
+  unsigned char *seg_codes;
   bool diag_fresh = false;    // diag64 was formed from the current coefficients (this step's abcei)
   // The mixed solve's FP32 coefficient hierarchy, launched on `side` right
   // after this step's abcei so that it overlaps the rest of the momentum

@@ -22,17 +22,21 @@ namespace {
 
 using namespace mg32;
 
+template <bool VEC>
 __global__ void k_relax32_split(float *__restrict__ self, const float *__restrict__ other,
-                                const float *__restrict__ rhs_self, const float *__restrict__ cc, Dims d, Split sp,
-                                int c, float h2, float omega, float r1, float r2) {
-  b_relax32_split(blockIdx, gridDim, self, other, rhs_self, cc, d, sp, c, h2, omega, r1, r2);
+                                const float *__restrict__ rhs_self, const float *__restrict__ cc,
+                                const unsigned char *__restrict__ flags, Dims d, Split sp, int c, float h2, float omega,
+                                float r1, float r2) {
+  b_relax32_split<VEC>(blockIdx, gridDim, self, other, rhs_self, cc, flags, d, sp, c, h2, omega, r1, r2);
 }
 
+template <bool VEC>
 __global__ void k_resid_restrict32_split(float *__restrict__ rhs_c, float *__restrict__ u_c, const float *__restrict__ ue,
                                          const float *__restrict__ uo, const float *__restrict__ re,
-                                         const float *__restrict__ ro, const float *__restrict__ cc, Dims df,
-                                         Split sp, Dims dc, float h2i, float r1, float r2) {
-  b_resid_restrict32_split(blockIdx, gridDim, rhs_c, u_c, ue, uo, re, ro, cc, df, sp, dc, h2i, r1, r2);
+                                         const float *__restrict__ ro, const float *__restrict__ cc,
+                                         const unsigned char *__restrict__ flags, Dims df, Split sp, Dims dc, float h2i,
+                                         float r1, float r2) {
+  b_resid_restrict32_split<VEC>(blockIdx, gridDim, rhs_c, u_c, ue, uo, re, ro, cc, flags, df, sp, dc, h2i, r1, r2);
 }
 
 template <bool TRI>
@@ -145,8 +149,13 @@ __global__ void k_correct64(double *__restrict__ p, const float *__restrict__ ev
   b_correct64(blockIdx, gridDim, p, ev, od, d, sp, init);
 }
 
-__global__ void k_to32(float *__restrict__ dst, const double *__restrict__ src, size_t n) {
-  b_to32(blockIdx, gridDim, dst, src, n);
+__global__ void k_codes(float *__restrict__ dst, unsigned char *__restrict__ codes, const double *__restrict__ src,
+                        Dims d) {
+  b_codes(blockIdx, gridDim, dst, codes, src, d);
+}
+
+__global__ void k_flags(unsigned char *__restrict__ flags, const unsigned char *__restrict__ codes, Dims d) {
+  b_flags(blockIdx, gridDim, flags, codes, d);
 }
 
 __global__ void k_acfromac64to32(float *__restrict__ a, float *__restrict__ b, float *__restrict__ c,
@@ -394,24 +403,50 @@ cudaError_t relax32_n(int n, float *u, float h2, const float *rhs, const float *
   return cudaGetLastError();
 }
 
+// Block of the finest sweep: 64 split indices x 8 rows, or where a thread has
+// four neighbours a row's hx / 4 threads and as many rows as make whole warps
+// of them, up to about 256 threads: warps run on from one row into the next.
+static dim3 split_block(Split sp) {
+  if (!split_vec(sp)) return dim3(32, 8, 1);
+  const int x = sp.hx / 4;
+  int step = 1;
+  while (x * step % 32) step *= 2;
+  if (x > 256 || x * step > 512) return dim3(32, 8, 1);
+  const int rows = 256 / (x * step) * step;
+  return dim3((unsigned)x, (unsigned)(rows > step ? rows : step), 1);
+}
+
 // Finest level, colour-split storage: u = {even, odd}, rhs = {even, odd}.
-cudaError_t relax32_split_n(int n, float *const u[2], float *const rhs[2], const float *cc, Dims d, float h2,
-                            float omega, float r1, float r2, cudaStream_t st) {
+cudaError_t relax32_split_n(int n, float *const u[2], float *const rhs[2], const float *cc,
+                            const unsigned char *flags, Dims d, float h2, float omega, float r1, float r2,
+                            cudaStream_t st) {
   const Split sp{(d.nx - 2) >> 1, d.ny - 2, d.nz - 2};
-  const dim3 blk(32, 8, 1);  // a block covers 64 split indices x 8 rows
-  const dim3 grid((unsigned)((sp.hx + 63) / 64), (unsigned)((d.ny - 2 + 7) / 8), (unsigned)(d.nz - 2));
+  const dim3 blk = split_block(sp);
+  const dim3 grid((unsigned)((sp.hx + split_cells(sp, blk.x) - 1) / split_cells(sp, blk.x)),
+                  (unsigned)((d.ny - 2 + blk.y - 1) / blk.y), (unsigned)(d.nz - 2));
   for (int q = 0; q < n; q++)
-    for (int c = 0; c < 2; c++)
-      DSG_COUNT k_relax32_split<<<grid, blk, 0, st>>>(u[c], u[1 - c], rhs[c], cc, d, sp, c, h2, omega, r1, r2);
+    for (int c = 0; c < 2; c++) {
+      if (split_vec(sp))
+        DSG_COUNT k_relax32_split<true><<<grid, blk, 0, st>>>(u[c], u[1 - c], rhs[c], cc, flags, d, sp, c, h2, omega,
+                                                             r1, r2);
+      else
+        DSG_COUNT k_relax32_split<false><<<grid, blk, 0, st>>>(u[c], u[1 - c], rhs[c], cc, flags, d, sp, c, h2, omega,
+                                                              r1, r2);
+    }
   return cudaGetLastError();
 }
 
 cudaError_t resid_restrict32_split(float *rhs_c, float *u_c, float *const u[2], float *const rhs[2], const float *cc,
-                                   Dims df, float h2i, float r1, float r2, cudaStream_t st) {
+                                   const unsigned char *flags, Dims df, float h2i, float r1, float r2,
+                                   cudaStream_t st) {
   const Dims dc{df.nx / 2 + 1, df.ny / 2 + 1, df.nz / 2 + 1};
   const Split sp{(df.nx - 2) >> 1, df.ny - 2, df.nz - 2};
-  DSG_COUNT k_resid_restrict32_split<<<interior_grid(dc, kBlk), kBlk, 0, st>>>(rhs_c, u_c, u[0], u[1], rhs[0], rhs[1],
-                                                                            cc, df, sp, dc, h2i, r1, r2);
+  if (split_vec(sp))
+    DSG_COUNT k_resid_restrict32_split<true><<<interior_grid(dc, kBlk), kBlk, 0, st>>>(
+        rhs_c, u_c, u[0], u[1], rhs[0], rhs[1], cc, flags, df, sp, dc, h2i, r1, r2);
+  else
+    DSG_COUNT k_resid_restrict32_split<false><<<interior_grid(dc, kBlk), kBlk, 0, st>>>(
+        rhs_c, u_c, u[0], u[1], rhs[0], rhs[1], cc, flags, df, sp, dc, h2i, r1, r2);
   return cudaGetLastError();
 }
 
@@ -504,8 +539,13 @@ cudaError_t correct64(double *p, float *const e[2], Dims d, int init, cudaStream
   return cudaGetLastError();
 }
 
-cudaError_t to32(float *dst, const double *src, size_t n, cudaStream_t st) {
-  DSG_COUNT k_to32<<<flat_blocks(n), 256, 0, st>>>(dst, src, n);
+size_t segment_codes(Dims d) { return (size_t)segments(d) * d.ny * d.nz; }
+size_t segment_flags(Dims d) { return (size_t)segments(d) * (d.ny - 2) * (d.nz - 2); }
+
+cudaError_t to32_flags(float *dst, unsigned char *flags, unsigned char *codes, const double *src, Dims d,
+                       cudaStream_t st) {
+  DSG_COUNT k_codes<<<flat_blocks(32 * segment_codes(d)), 256, 0, st>>>(dst, codes, src, d);
+  if (split_vec(Split{(d.nx - 2) >> 1, d.ny - 2, d.nz - 2})) DSG_COUNT k_flags<<<flat_blocks(segment_flags(d)), 256, 0, st>>>(flags, codes, d);
   return cudaGetLastError();
 }
 

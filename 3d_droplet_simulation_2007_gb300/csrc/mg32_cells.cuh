@@ -72,8 +72,87 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return r;
 }
 
+// Sum over the six faces of coefficient times neighbour minus h2 * rhs, with
+// every rounding spelled out: the compiler's own choice of fused operations
+// differs between kernels (which product of the first sum it rounds, whether a
+// loop-invariant h2 * rhs is formed on its own).
+__device__ __forceinline__ float face_sum(float ae, float xp, float aw, float xm, float bn, float yp, float bs, float ym,
+                                          float ct, float zp, float cb, float zm, float h2, float rhs) {
+  float t = fmaf(ae, xp, aw * xm);
+  t = fmaf(bn, yp, t);
+  t = fmaf(bs, ym, t);
+  t = fmaf(ct, zp, t);
+  t = fmaf(cb, zm, t);
+  return fmaf(-h2, rhs, t);
+}
+// omega * t + (1 - omega) * u
+__device__ __forceinline__ float over_relax(float omega, float t, float u) {
+  return fmaf(1.f - omega, u, omega * t);
+}
+
 __device__ __forceinline__ float face_coef(float x, float y, float r1, float r2) {
   return rcp_approx(r1 * (x + y) + r2);
+}
+
+// ---- uniform segments ---------------------------------------------------------
+//
+// Most of the domain is pure gas or pure liquid.  A segment is 32 split
+// indices of one row, both colours (i = 2 + 64 s .. 65 + 64 s): what one warp
+// updates.  Where the volume fractions that a segment's cells read (theirs and
+// their six neighbours') are all exactly 0 or all exactly 1, its flag is 1 or
+// 2, every face coefficient is face_coef of that value twice, and a sweep
+// reads neither cc nor forms seven reciprocals per cell: 16 instead of 24
+// bytes and a third of the instructions, with the same bits.  The flag is read
+// before anything depends on it, so that no load waits for a vote (a vote over
+// the seven loaded fractions lost more than the reciprocals cost).  Else the
+// flag is 0.  Only the grids that split_vec names use them (b_relax32_split).
+constexpr int kVecCells = 200000;
+__host__ __device__ __forceinline__ bool split_vec(Split sp) { return (sp.hx & 3) == 0 && (long long)sp.hx * sp.ny2 * sp.nz2 >= kVecCells; }
+__host__ __device__ __forceinline__ int segments(Dims d) { return (((d.nx - 2) >> 1) + 31) / 32; }
+
+__device__ __forceinline__ const unsigned char *seg_flag(const unsigned char *flags, Dims d, int j, int k) {
+  return flags + ((unsigned)(j - 2) + (unsigned)(d.ny - 2) * (unsigned)(k - 2)) * (unsigned)segments(d);
+}
+
+// FP64 -> FP32 volume fraction of all nodes, and a code per segment and row
+// (ghost rows included): 1 or 2 if the row's fractions from one cell before
+// the segment to one after it (within 2..nx) are all 0 or all 1, else 0.  One
+// warp per segment.
+__device__ __forceinline__ void b_codes(const uint3 B, const uint3 G, float *__restrict__ dst,
+                                        unsigned char *__restrict__ codes, const double *__restrict__ src, Dims d) {
+  const unsigned ns = segments(d), total = ns * (unsigned)d.ny * (unsigned)d.nz, lane = threadIdx.x & 31;
+  for (unsigned t = (B.x * blockDim.x + threadIdx.x) >> 5; t < total; t += G.x * blockDim.x >> 5) {
+    const unsigned row = t / ns, s = t - row * ns;
+    const double *in = src + (size_t)row * d.nx - 1;  // in[i]: node i of the row
+    float *out = dst + (size_t)row * d.nx - 1;
+    const int i0 = 2 + 64 * (int)s, ia = i0 + (int)lane, ib = ia + 32;
+    const int before = i0 > 2 ? i0 - 1 : 2, after = i0 + 64 < d.nx ? i0 + 64 : d.nx;
+    const float first = (float)in[i0];
+    const float a = ia <= d.nx ? (float)in[ia] : first, b = ib <= d.nx ? (float)in[ib] : first;
+    const float e = (float)in[lane == 0 ? before : after];
+    if (ia <= d.nx) out[ia] = a;
+    if (ib <= d.nx) out[ib] = b;
+    if (s == 0 && lane == 0) out[1] = (float)in[1];
+    if (s == ns - 1)
+      for (int i = i0 + 64 + (int)lane; i <= d.nx; i += 32) out[i] = (float)in[i];
+    const unsigned f = __float_as_uint(first);
+    const bool same = __float_as_uint(a) == f && __float_as_uint(b) == f && __float_as_uint(e) == f;
+    const bool all = __all_sync(0xffffffffu, same);
+    if (lane == 0) codes[t] = !all ? 0 : (f == 0u ? 1 : (f == 0x3F800000u ? 2 : 0));
+  }
+}
+
+// The flag of each interior segment: its row's code if the four rows around it
+// have the same one.
+__device__ __forceinline__ void b_flags(const uint3 B, const uint3 G, unsigned char *__restrict__ flags,
+                                        const unsigned char *__restrict__ codes, Dims d) {
+  const unsigned ns = segments(d), ny2 = d.ny - 2, total = ns * ny2 * (unsigned)(d.nz - 2);
+  for (unsigned t = B.x * blockDim.x + threadIdx.x; t < total; t += G.x * blockDim.x) {
+    const unsigned row = t / ns, s = t - row * ns, k = row / ny2, j = row - k * ny2;
+    const unsigned sy = ns, sz = ns * (unsigned)d.ny, q = s + sy * (j + 1) + sz * (k + 1);
+    const unsigned char c = codes[q];
+    flags[t] = codes[q - sy] == c && codes[q + sy] == c && codes[q - sz] == c && codes[q + sz] == c ? c : 0;
+  }
 }
 
 // Value of cell (i,j,k) of a colour-split pair {even, odd}.
@@ -139,11 +218,12 @@ __device__ __forceinline__ float coarse_at(const float *__restrict__ uc, Dims dc
 // One colour-c update (0 = i+j+k even) of the finest-level cell at split
 // index (m, j, k).  Offsets are 32-bit (grids stay below 2^31 nodes) and
 // taken from one base pointer per array, which cut the pass from 51.3 to
-// 47.2 us at 258^3 against 64-bit indexing, with the same bits.
+// 47.2 us at 258^3 against 64-bit indexing, with the same bits.  flag: of the
+// cell's segment.
 __device__ __forceinline__ void relax32_split_cell(float *__restrict__ self, const float *__restrict__ other,
                                                    const float *__restrict__ rhs_self, const float *__restrict__ cc,
                                                    Dims d, Split sp, int c, float h2, float omega, float r1, float r2,
-                                                   int m, int j, int k) {
+                                                   int m, int j, int k, unsigned flag) {
   const int p = (j + k + c) & 1;
   const int i = 2 + 2 * m + p;
   const int row = sp.hx, plane = sp.hx * sp.ny2;
@@ -156,19 +236,25 @@ __device__ __forceinline__ void relax32_split_cell(float *__restrict__ self, con
   const float yp = (j == d.ny - 1) ? uc : o[row];
   const float zm = (k == 2) ? uc : o[-plane];
   const float zp = (k == d.nz - 1) ? uc : o[plane];
-  const unsigned q = (unsigned)(i - 1) + (unsigned)d.nx * ((unsigned)(j - 1) + (unsigned)d.ny * (unsigned)(k - 1));
-  const float *cq = cc + q;
-  const int sy = d.nx, sz = d.nx * d.ny;
-  const float c0 = cq[0];
-  const float ae = face_coef(c0, cq[1], r1, r2);
-  const float aw = (i == 2) ? ae : face_coef(cq[-1], c0, r1, r2);
-  const float bn = face_coef(c0, cq[sy], r1, r2);
-  const float bs = face_coef(cq[-sy], c0, r1, r2);
-  const float ct = face_coef(c0, cq[sz], r1, r2);
-  const float cb = face_coef(cq[-sz], c0, r1, r2);
+  const float f = rhs_self[qs];
+  float ae, aw, bn, bs, ct, cb;
+  if (flag) {
+    const float c0 = flag == 1 ? 0.f : 1.f;
+    ae = aw = bn = bs = ct = cb = face_coef(c0, c0, r1, r2);
+  } else {
+    const unsigned q = (unsigned)(i - 1) + (unsigned)d.nx * ((unsigned)(j - 1) + (unsigned)d.ny * (unsigned)(k - 1));
+    const float *cq = cc + q;
+    const int sy = d.nx, sz = d.nx * d.ny;
+    const float c0 = cq[0];
+    ae = face_coef(c0, cq[1], r1, r2);
+    aw = (i == 2) ? ae : face_coef(cq[-1], c0, r1, r2);
+    bn = face_coef(c0, cq[sy], r1, r2);
+    bs = face_coef(cq[-sy], c0, r1, r2);
+    ct = face_coef(c0, cq[sz], r1, r2);
+    cb = face_coef(cq[-sz], c0, r1, r2);
+  }
   const float ei = rcp_approx(ae + aw + bn + bs + ct + cb);
-  const float temp = (ae * xp + aw * xm + bn * yp + bs * ym + ct * zp + cb * zm - h2 * rhs_self[qs]) * ei;
-  self[qs] = omega * temp + (1.f - omega) * uc;
+  self[qs] = over_relax(omega, face_sum(ae, xp, aw, xm, bn, yp, bs, ym, ct, zp, cb, zm, h2, f) * ei, uc);
 }
 
 // Operator of the finest-level FP32 correction equation at the colour-c cell of
@@ -202,31 +288,88 @@ __device__ __forceinline__ float lap32_split_cell(const float *__restrict__ self
   return ae * (xp - uc) + aw * (xm - uc) + bn * (yp - uc) + bs * (ym - uc) + ct * (zp - uc) + cb * (zm - uc);
 }
 
-// One colour pass on the finest level: each thread updates split indices m
-// and m + blockDim.x of its row (two independent cells in flight; 45.7 against
-// 47.2 us per pass with one).
+// One colour pass on the finest level.  Rows of a multiple of four split
+// indices: a thread updates four neighbours; a warp whose cells all lie in
+// uniform segments reads and writes them as 16-byte vectors, any other warp one
+// by one (256^3: 28.6 us per pass, 45.4 with two cells per thread, uniform or
+// not: that form issues 110 instructions per cell; 160^3: 7.6 against 12.9).
+// Other rows, and grids of fewer than kVecCells cells per colour, which have
+// too few threads that way (64^3: 3.3 us with two cells per thread, 3.7 with
+// four): split indices m and m + blockDim.x.  split_cells: the split indices
+// a block covers along a row.  VEC = split_vec(sp).
+__host__ __device__ __forceinline__ int split_cells(Split sp, int blk_x) { return (split_vec(sp) ? 4 : 2) * blk_x; }
+
+template <bool VEC>
 __device__ __forceinline__ void b_relax32_split(const uint3 B, const uint3 G, float *__restrict__ self, const float *__restrict__ other,
-                                const float *__restrict__ rhs_self, const float *__restrict__ cc, Dims d, Split sp,
-                                int c, float h2, float omega, float r1, float r2) {
-  const int m = B.x * 2 * blockDim.x + threadIdx.x;
+                                const float *__restrict__ rhs_self, const float *__restrict__ cc,
+                                const unsigned char *__restrict__ flags, Dims d, Split sp, int c, float h2, float omega,
+                                float r1, float r2) {
   const int j = B.y * blockDim.y + threadIdx.y + 2;
   const int k = B.z + 2;
-  if (j > d.ny - 1) return;
-  if (m < sp.hx) relax32_split_cell(self, other, rhs_self, cc, d, sp, c, h2, omega, r1, r2, m, j, k);
-  if (m + (int)blockDim.x < sp.hx)
-    relax32_split_cell(self, other, rhs_self, cc, d, sp, c, h2, omega, r1, r2, m + blockDim.x, j, k);
+  if (!VEC) {
+    const int m = B.x * 2 * blockDim.x + threadIdx.x, m2 = m + (int)blockDim.x;
+    if (j > d.ny - 1) return;
+    if (m < sp.hx) relax32_split_cell(self, other, rhs_self, cc, d, sp, c, h2, omega, r1, r2, m, j, k, 0);
+    if (m2 < sp.hx) relax32_split_cell(self, other, rhs_self, cc, d, sp, c, h2, omega, r1, r2, m2, j, k, 0);
+    return;
+  }
+  const int m = 4 * (int)(B.x * blockDim.x + threadIdx.x);
+  const bool in = j <= d.ny - 1 && m < sp.hx;
+  const unsigned f = in ? seg_flag(flags, d, j, k)[m >> 5] : 1;  // the four cells lie in one segment
+  if (!__all_sync(0xffffffffu, f != 0)) {
+    if (in)
+      for (int q = 0; q < 4; q++)
+        relax32_split_cell(self, other, rhs_self, cc, d, sp, c, h2, omega, r1, r2, m + q, j, k, f);
+    return;
+  }
+  if (!in) return;
+  const int p = (j + k + c) & 1;
+  const unsigned row = sp.hx, plane = sp.hx * sp.ny2;
+  const unsigned q = (unsigned)m + row * (unsigned)(j - 2) + plane * (unsigned)(k - 2);
+  auto vec = [](const float *x) { return *reinterpret_cast<const float4 *>(x); };
+  const float *o = other + q;
+  const float4 u = vec(self + q), x = vec(o), f4 = vec(rhs_self + q);
+  const float4 ym = (j == 2) ? u : vec(o - row), yp = (j == d.ny - 1) ? u : vec(o + row);
+  const float4 zm = (k == 2) ? u : vec(o - plane), zp = (k == d.nz - 1) ? u : vec(o + plane);
+  // along x: the cell before (p = 0) or after (p = 1) the vector x as well
+  const float side = p ? (m + 4 == sp.hx ? 0.f : o[4]) : (m == 0 ? u.x : o[-1]);
+  const float4 xm = p ? x : make_float4(side, x.x, x.y, x.z);
+  const float4 xp = p ? make_float4(x.y, x.z, x.w, side) : x;
+  const float c0 = f == 1 ? 0.f : 1.f;
+  const float kf = face_coef(c0, c0, r1, r2);
+  const float ei = rcp_approx(kf + kf + kf + kf + kf + kf);
+  auto upd = [&](float uc, float e, float w, float n, float s, float t, float b, float f) {
+    return over_relax(omega, face_sum(kf, e, kf, w, kf, n, kf, s, kf, t, kf, b, h2, f) * ei, uc);
+  };
+  *reinterpret_cast<float4 *>(self + q) =
+      make_float4(upd(u.x, xp.x, xm.x, yp.x, ym.x, zp.x, zm.x, f4.x), upd(u.y, xp.y, xm.y, yp.y, ym.y, zp.y, zm.y, f4.y),
+                  upd(u.z, xp.z, xm.z, yp.z, ym.z, zp.z, zm.z, f4.z), upd(u.w, xp.w, xm.w, yp.w, ym.w, zp.w, zm.w, f4.w));
 }
 
 // Finest-level residual (cc-derived operator, virtual ghosts) restricted to the
 // coarse rhs: mean of the 8 fine residuals of each coarse cell.
+template <bool VEC>
 __device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const uint3 G, float *__restrict__ rhs_c, float *__restrict__ u_c, const float *__restrict__ ue,
                                          const float *__restrict__ uo, const float *__restrict__ re,
-                                         const float *__restrict__ ro, const float *__restrict__ cc, Dims df,
-                                         Split sp, Dims dc, float h2i, float r1, float r2) {
+                                         const float *__restrict__ ro, const float *__restrict__ cc,
+                                         const unsigned char *__restrict__ flags, Dims df, Split sp, Dims dc, float h2i,
+                                         float r1, float r2) {
   const int ic = B.x * blockDim.x + threadIdx.x + 2;
   const int jc = B.y * blockDim.y + threadIdx.y + 2;
   const int kc = B.z + 2;
   if (ic > dc.nx - 1 || jc > dc.ny - 1) return;
+  // the warp's 32 coarse cells lie in one segment of each of the four rows
+  unsigned f00 = 0;
+  bool uniform = false;
+  if (VEC) {
+    const int seg = (ic - 2) >> 5;
+    f00 = seg_flag(flags, df, 2 * jc - 2, 2 * kc - 2)[seg];
+    const unsigned f10 = seg_flag(flags, df, 2 * jc - 1, 2 * kc - 2)[seg],
+                   f01 = seg_flag(flags, df, 2 * jc - 2, 2 * kc - 1)[seg],
+                   f11 = seg_flag(flags, df, 2 * jc - 1, 2 * kc - 1)[seg];
+    uniform = f00 && f00 == f10 && f00 == f01 && f00 == f11;
+  }
+  const float cu = f00 == 2 ? 1.f : 0.f, ku = face_coef(cu, cu, r1, r2);
   float acc = 0.f;
 #pragma unroll
   for (int dk = 0; dk < 2; dk++)
@@ -242,15 +385,18 @@ __device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const ui
         const float ym = (j == 2) ? uc : split_get(ue, uo, sp, i, j - 1, k);
         const float zp = (k + 1 == df.nz) ? uc : split_get(ue, uo, sp, i, j, k + 1);
         const float zm = (k == 2) ? uc : split_get(ue, uo, sp, i, j, k - 1);
-        const float *cq = cc + ix32(df, i, j, k);
-        const int sy = df.nx, sz = df.nx * df.ny;
-        const float c0 = cq[0];
-        const float ae = face_coef(c0, cq[1], r1, r2);
-        const float aw = (i == 2) ? ae : face_coef(cq[-1], c0, r1, r2);
-        const float bn = face_coef(c0, cq[sy], r1, r2);
-        const float bs = face_coef(cq[-sy], c0, r1, r2);
-        const float ct = face_coef(c0, cq[sz], r1, r2);
-        const float cb = face_coef(cq[-sz], c0, r1, r2);
+        float ae = ku, aw = ku, bn = ku, bs = ku, ct = ku, cb = ku;
+        if (!uniform) {
+          const float *cq = cc + ix32(df, i, j, k);
+          const int sy = df.nx, sz = df.nx * df.ny;
+          const float c0 = cq[0];
+          ae = face_coef(c0, cq[1], r1, r2);
+          aw = (i == 2) ? ae : face_coef(cq[-1], c0, r1, r2);
+          bn = face_coef(c0, cq[sy], r1, r2);
+          bs = face_coef(cq[-sy], c0, r1, r2);
+          ct = face_coef(c0, cq[sz], r1, r2);
+          cb = face_coef(cq[-sz], c0, r1, r2);
+        }
         const float lap = ae * (xp - uc) + aw * (xm - uc) + bn * (yp - uc) + bs * (ym - uc) + ct * (zp - uc) +
                           cb * (zm - uc);
         acc += split_get(re, ro, sp, i, j, k) - h2i * lap;
@@ -328,9 +474,8 @@ __device__ __forceinline__ void b_split_from64(const uint3 B, const uint3 G, flo
 // coefficients (relax, main.f:3956-3997), and its residual.
 __device__ __forceinline__ float relax32_value(float uc, const Nb &n, float ae, float aw, float bn, float bs, float ct,
                                                float cb, float ei, float rhs, float h2, float omega) {
-  // the explicit fmaf keeps its rounding where h2 * rhs is loop-invariant
-  const float s = fmaf(-h2, rhs, ae * n.xp + aw * n.xm + bn * n.yp + bs * n.ym + ct * n.zp + cb * n.zm);
-  return omega * (s * ei) + (1.f - omega) * uc;
+  const float s = face_sum(ae, n.xp, aw, n.xm, bn, n.yp, bs, n.ym, ct, n.zp, cb, n.zm, h2, rhs);
+  return over_relax(omega, s * ei, uc);
 }
 __device__ __forceinline__ float resid32_value(float uc, const Nb &n, float ae, float aw, float bn, float bs, float ct,
                                                float cb, float rhs, float h2i) {
@@ -646,11 +791,6 @@ __device__ __forceinline__ void b_correct64(const uint3 B, const uint3 G, double
 }
 
 // Coarse FP32 coefficients (acfromac) straight from the FP64 fine ones.
-__device__ __forceinline__ void b_to32(const uint3 B, const uint3 G, float *__restrict__ dst, const double *__restrict__ src, size_t n) {
-  for (size_t q = (size_t)B.x * blockDim.x + threadIdx.x; q < n; q += (size_t)G.x * blockDim.x)
-    dst[q] = (float)src[q];
-}
-
 __device__ __forceinline__ void b_acfromac64to32(const uint3 B, const uint3 G, float *__restrict__ a, float *__restrict__ b, float *__restrict__ c,
                                  float *__restrict__ ei, const double *__restrict__ a2,
                                  const double *__restrict__ b2, const double *__restrict__ c2, Dims dc, Dims df) {
