@@ -188,14 +188,55 @@ int coarse64(dsg_ctx *ctx, bool fmg) {
   return DSG_OK;
 }
 
-// One V-cycle from level j down to 1 and back (main.f:3705-3759).
-int vcycle(dsg_ctx *ctx, int j) {
+// A smoothing phase of level l in one cooperative launch: n sweeps; down: the
+// residual restricted into level l - 1 at the end; up: level l - 1's correction
+// added (add) or set at the start.
+int phase64(dsg_ctx *ctx, int l, int n, bool down, bool up, bool add) {
+  dsg::mgg::Args<double> &G = ctx->gr64[l];
+  double **L = ctx->lv[l];
+  G.u = L[1];
+  G.rhs = L[3];
+  G.a = L[4];
+  G.b = L[5];
+  G.c = L[6];
+  G.ei = L[7];
+  const double h1 = ctx->s.lengthsize / (ctx->lnx[l] - 2);
+  G.h2 = h1 * h1;
+  G.h2i = 1.0 / (h1 * h1);
+  G.omega = ctx->cfg.omega;
+  G.n = n > 0 ? n : 0;
+  G.rhs_c = down ? ctx->lv[l - 1][3] : nullptr;
+  G.u_c = down ? ctx->lv[l - 1][1] : nullptr;
+  G.prolong = up ? ctx->lv[l - 1][1] : nullptr;
+  G.add = add ? 1 : 0;
+  G.ghosts = l == ctx->ng && n > 0;
+  DSG_CK(ctx, dsg::grid64(G, fp64_fma(ctx), ctx->stream));
+  return DSG_OK;
+}
+
+// Whether level l's phases are cooperative launches (the live profile times
+// the finest level's sweeps as launches of their own).
+template <class A>
+bool phases(const dsg_ctx *ctx, const A &level, int l) {
+  return level.g.blocks() > 0 && !(ctx->prof && l == ctx->ng);
+}
+
+// One V-cycle from level j down to 1 and back (main.f:3705-3759); init: level
+// j starts from level j - 1's u.
+int vcycle(dsg_ctx *ctx, int j, bool init) {
   const double ls = ctx->s.lengthsize;
   cudaStream_t st = ctx->stream;
   const int jt = ctx->tail64_top;  // levels 1..jt in one cluster launch (0: pass by pass)
   for (int jj = j; jj >= 2 && jj > jt; jj--) {
     double **L = ctx->lv[jj];
     const Dims d = ctx->level(jj);
+    if (init && jj == j && (jj == ctx->ng || !phases(ctx, ctx->gr64[jj], jj)))
+      DSG_CK(ctx, dsg::interp(L[1], ctx->lv[jj - 1][1], d, st));
+    if (phases(ctx, ctx->gr64[jj], jj)) {
+      int rc = phase64(ctx, jj, ctx->s.npre, true, init && jj == j && jj < ctx->ng, false);
+      if (rc) return rc;
+      continue;
+    }
     DSG_CK(ctx, relax_level(ctx, ctx->s.npre, jj, ls));
     DSG_CK(ctx, dsg::resid_rstrct(ls, ctx->lv[jj - 1][3], ctx->lv[jj - 1][1], L[1], L[3], L[4], L[5], L[6], d, st,
                                   fp64_fma(ctx)));
@@ -209,9 +250,19 @@ int vcycle(dsg_ctx *ctx, int j) {
   for (int jj = jt >= 1 ? jt + 1 : 2; jj <= j; jj++) {
     double **L = ctx->lv[jj];
     const Dims d = ctx->level(jj);
+    if (jj < ctx->ng && phases(ctx, ctx->gr64[jj], jj)) {
+      int rc = phase64(ctx, jj, ctx->s.npost, false, true, true);
+      if (rc) return rc;
+      continue;
+    }
     // the finest level's residual array keeps addint's values: its ghosts
     // are read in the next step's momentum phase
     DSG_CK(ctx, dsg::addint(L[1], ctx->lv[jj - 1][1], jj == ctx->ng ? L[2] : nullptr, d, st));
+    if (phases(ctx, ctx->gr64[jj], jj)) {
+      int rc = phase64(ctx, jj, ctx->s.npost, false, false, false);
+      if (rc) return rc;
+      continue;
+    }
     DSG_CK(ctx, relax_level(ctx, ctx->s.npost, jj, ls));
   }
   return DSG_OK;
@@ -325,7 +376,42 @@ int coarse32(dsg_ctx *ctx, bool fmg) {
   return DSG_OK;
 }
 
-int vcycle32(dsg_ctx *ctx, int j) {
+// phase64's counterpart on the FP32 levels.
+int phase32(dsg_ctx *ctx, int l, int n, bool down, bool up, bool add) {
+  dsg::mgg::Args<float> &G = ctx->gr32[l];
+  float **L = ctx->lv32[l];
+  if (l == ctx->ng) {
+    const FineSplit f = fine_split(ctx);
+    G.u = G.rhs = nullptr;
+    for (int c = 0; c < 2; c++) {
+      G.us[c] = f.u[c];
+      G.rs[c] = f.r[c];
+    }
+    G.cc = L[A32];
+    phase_coefs(ctx, &G.r1, &G.r2);
+  } else {
+    G.u = L[U32];
+    G.rhs = L[RHS32];
+    G.a = L[A32];
+    G.b = L[B32];
+    G.c = L[C32];
+    G.ei = L[EI32];
+  }
+  G.h2 = level_h2(ctx, l);
+  G.h2i = 1.0f / level_h2(ctx, l);
+  G.omega = omega32(ctx);
+  G.n = n > 0 ? n : 0;
+  G.rhs_c = down ? ctx->lv32[l - 1][RHS32] : nullptr;
+  G.u_c = down ? ctx->lv32[l - 1][U32] : nullptr;
+  G.prolong = up ? ctx->lv32[l - 1][U32] : nullptr;
+  G.add = add ? 1 : 0;
+  G.tri = tri32(ctx);
+  DSG_CK(ctx, dsg::grid32(G, ctx->stream));
+  return DSG_OK;
+}
+
+// One FP32 V-cycle from level j; init: level j starts from level j - 1's u.
+int vcycle32(dsg_ctx *ctx, int j, bool init) {
   cudaStream_t st = ctx->stream;
   const int ng = ctx->ng;
   float r1, r2;
@@ -335,6 +421,16 @@ int vcycle32(dsg_ctx *ctx, int j) {
   for (int jj = j; jj >= 2 && jj > jt; jj--) {
     float **L = ctx->lv32[jj];
     float **Lc = ctx->lv32[jj - 1];
+    const bool set = init && jj == j;
+    if (phases(ctx, ctx->gr32[jj], jj)) {
+      int rc = phase32(ctx, jj, pre32(ctx, jj), true, set, false);
+      if (rc) return rc;
+      continue;
+    }
+    if (set && jj == ng)
+      DSG_CK(ctx, dsg::prolong32_split(fine_split(ctx).u, Lc[U32], ctx->level(jj), 0, tri32(ctx), st));
+    else if (set)
+      DSG_CK(ctx, dsg::prolong32(L[U32], Lc[U32], ctx->level(jj), 0, tri32(ctx), st));
     DSG_CK(ctx, relax32_level(ctx, pre32(ctx, jj), jj));
     if (jj == ng) {
       FineSplit f = fine_split(ctx);
@@ -352,6 +448,11 @@ int vcycle32(dsg_ctx *ctx, int j) {
     DSG_CK(ctx, relax32_level(ctx, ctx->s.ntop, 1));
   }
   for (int jj = jt >= 1 ? jt + 1 : 2; jj <= j; jj++) {
+    if (phases(ctx, ctx->gr32[jj], jj)) {
+      int rc = phase32(ctx, jj, post32(ctx, jj), false, true, true);
+      if (rc) return rc;
+      continue;
+    }
     if (jj == ng) {
       FineSplit f = fine_split(ctx);
       DSG_CK(ctx, dsg::prolong32_split(f.u, ctx->lv32[jj - 1][U32], ctx->level(jj), 1, tri32(ctx), st));
@@ -515,13 +616,15 @@ int fmg32(dsg_ctx *ctx) {
     DSG_CK(ctx, relax32_level(ctx, ctx->s.ntop, 1));
   }
   for (int j = ctx->tail_top >= 1 ? ctx->tail_top + 1 : 2; j <= ng; j++) {
-    if (j == ng)
-      DSG_CK(ctx, dsg::prolong32_split(f.u, ctx->lv32[j - 1][U32], ctx->level(j), 0, tri32(ctx), st));
-    else
-      DSG_CK(ctx, dsg::prolong32(ctx->lv32[j][U32], ctx->lv32[j - 1][U32], ctx->level(j), 0, tri32(ctx), st));
     const int cycles = fmg32_cycles(ctx, j);
+    if (cycles <= 0) {
+      if (j == ng)
+        DSG_CK(ctx, dsg::prolong32_split(f.u, ctx->lv32[j - 1][U32], ctx->level(j), 0, tri32(ctx), st));
+      else
+        DSG_CK(ctx, dsg::prolong32(ctx->lv32[j][U32], ctx->lv32[j - 1][U32], ctx->level(j), 0, tri32(ctx), st));
+    }
     for (int c = 0; c < cycles; c++) {
-      int rc = vcycle32(ctx, j);
+      int rc = vcycle32(ctx, j, c == 0);
       if (rc) return rc;
     }
   }
@@ -577,7 +680,7 @@ int mixed_solve(dsg_ctx *ctx, dsg_mg_stats *s) {
     if (!ctx->cfg.mg32_krylov) {
       DSG_CK(ctx, cudaMemsetAsync(f.u[0], 0, fine_split_bytes(ctx), st));
       for (int q = 0; q < inner; q++) {
-        int e = vcycle32(ctx, ng);
+        int e = vcycle32(ctx, ng, false);
         if (e) return e;
       }
       DSG_CK(ctx, dsg::correct64(ctx->lv[ng][1], f.u, ctx->fine(), 0, st));
@@ -591,7 +694,7 @@ int mixed_solve(dsg_ctx *ctx, dsg_mg_stats *s) {
     phase_coefs(ctx, &r1, &r2);
     for (int q = 0; q < inner; q++) {
       DSG_CK(ctx, cudaMemsetAsync(f.u[0], 0, fine_split_bytes(ctx), st));
-      int e = vcycle32(ctx, ng);
+      int e = vcycle32(ctx, ng, false);
       if (e) return e;
       DSG_CK(ctx, dsg::gcr_step(q == 0, q == inner - 1, g, ctx->lv[ng][1], f.u, f.r, L[A32], ctx->fine(),
                                 1.0f / level_h2(ctx, ng), r1, r2, st));
@@ -774,9 +877,9 @@ int mglin(dsg_ctx *ctx, dsg_mg_stats *stats) {
                              ctx->level(1), om, st, fp64_fma(ctx)));
   }
   for (int j = ctx->tail64_top >= 1 ? ctx->tail64_top + 1 : 2; j <= ng; j++) {
-    DSG_CK(ctx, dsg::interp(ctx->lv[j][1], ctx->lv[j - 1][1], ctx->level(j), st));
+    if (ctx->cfg.cycles <= 0) DSG_CK(ctx, dsg::interp(ctx->lv[j][1], ctx->lv[j - 1][1], ctx->level(j), st));
     for (int c = 0; c < ctx->cfg.cycles; c++) {
-      int rc = vcycle(ctx, j);
+      int rc = vcycle(ctx, j, c == 0);
       if (rc) return rc;
       if (j == ng) fine_sweeps += ctx->s.npre + ctx->s.npost;
     }
@@ -797,7 +900,7 @@ int mglin(dsg_ctx *ctx, dsg_mg_stats *stats) {
     s.relres_init = r;
     int n = 0;
     while (r >= ctx->cfg.tol && n < ctx->cfg.max_vcycles) {
-      rc = vcycle(ctx, ng);
+      rc = vcycle(ctx, ng, false);
       if (rc) return rc;
       fine_sweeps += ctx->s.npre + ctx->s.npost;
       n++;
@@ -823,12 +926,26 @@ int mglin(dsg_ctx *ctx, dsg_mg_stats *stats) {
   return DSG_OK;
 }
 
-// Which levels the cluster kernels run.  FP32: every level below the finest
-// that fits a cluster's shared memory and registers (about 40^3 cells), or of
-// at most tail_nodes nodes when the configuration says so.
-void cluster_plan(dsg_ctx *ctx) {
+// Which levels run in the cluster kernel and which as cooperative phases.
+//
+// Cluster: every level below the finest that fits a cluster's shared memory
+// and registers (about 40^3 cells in FP32, 32^3 in FP64), or of at most
+// tail_nodes nodes when the configuration says so.  A context that has the
+// GPU for itself hands the largest of them to cooperative phases: beyond
+// 32^3 cells in FP32 and 16^3 in FP64 one cluster's 16 SMs take longer for a
+// pass than the exchange over the whole GPU (40^3 FP32: 0.92 against 0.78 us,
+// 32^3: 0.45 against 0.77; 32^3 FP64: 6.4 against 1.3).  An ensemble's members keep them in clusters,
+// which run side by side, and have no cooperative phases, which do not.
+//
+// Cooperative phases: every other level that fits the SMs' registers (about
+// 84^3 cells in FP32, 42^3 in FP64), the finest one among them.
+void level_plan(dsg_ctx *ctx) {
   const long long cap = ctx->cfg.tail_nodes;
+  const bool mixed = ctx->cfg.mode == DSG_MODE_TOL_MIXED || ctx->cfg.mode == DSG_MODE_LEARNED;
   const int c32 = cap >= 0 ? dsg::cluster32_size() : 0, c64 = dsg::cluster64_size();
+  const int g32 = ctx->alone && mixed && cap >= 0 ? dsg::grid32_blocks() : 0;
+  const int g64 = ctx->alone && !mixed ? dsg::grid64_blocks() : 0;
+  auto cells = [&](int l) { return (long long)(ctx->lnx[l] - 2) * (ctx->lny[l] - 2) * (ctx->lnz[l] - 2); };
   auto extents = [&](auto &G, int top) {
     for (int l = 1; l <= top; l++) {
       G.lv[l].nx = ctx->lnx[l] - 2;
@@ -839,15 +956,29 @@ void cluster_plan(dsg_ctx *ctx) {
   const int most = ctx->ng - 1 < dsg::mgc::kMaxLevels ? ctx->ng - 1 : dsg::mgc::kMaxLevels;
   memset(&ctx->cl32, 0, sizeof ctx->cl32);
   memset(&ctx->cl64, 0, sizeof ctx->cl64);
+  memset(ctx->gr32, 0, sizeof ctx->gr32);
+  memset(ctx->gr64, 0, sizeof ctx->gr64);
   ctx->tail_top = ctx->tail64_top = 0;
   for (int l = most; l >= 1 && c32 > 0 && ctx->tail_top == 0; l--) {
     if (cap > 0 && (long long)ctx->lnx[l] * ctx->lny[l] * ctx->lnz[l] > cap) continue;
+    if (g32 > 0 && cells(l) > 32 * 32 * 32) continue;
     extents(ctx->cl32, l);
     if (dsg::mgc::layout(ctx->cl32, l, c32, 1024, dsg::kCluster32Cells)) ctx->tail_top = l;
   }
   for (int l = most; l >= 1 && c64 > 0 && ctx->tail64_top == 0; l--) {
+    if (g64 > 0 && cells(l) > 16 * 16 * 16) continue;
     extents(ctx->cl64, l);
     if (dsg::mgc::layout(ctx->cl64, l, c64, 128, dsg::kCluster64Cells)) ctx->tail64_top = l;
+  }
+  auto cut = [&](auto &G, int l, int blocks, size_t size, int most_cells, int most_halo) {
+    if (blocks > 0 && (!dsg::mgg::plan(G.g, ctx->lnx[l] - 2, ctx->lny[l] - 2, ctx->lnz[l] - 2, blocks, size, most_cells,
+                                         most_halo) ||
+                       !dsg::mgg::layout(G)))
+      G.g.py = G.g.pz = 0;
+  };
+  for (int l = 2; l <= ctx->ng; l++) {
+    if (l > ctx->tail_top) cut(ctx->gr32[l], l, g32, sizeof(float), dsg::kGrid32Cells, dsg::kGrid32Halo);
+    if (l > ctx->tail64_top) cut(ctx->gr64[l], l, g64, sizeof(double), dsg::kGrid64Cells, dsg::kGrid64Halo);
   }
 }
 
@@ -860,7 +991,11 @@ extern "C" {
 
 const char *dsg_last_error(const dsg_ctx *ctx) { return ctx ? ctx->err.c_str() : g_last_error.c_str(); }
 
-int dsg_create(const dsg_config *cfg, dsg_ctx **out) {
+int dsg_create(const dsg_config *cfg, dsg_ctx **out) { return dsg::create(cfg, true, out); }
+
+}  // extern "C"
+
+int dsg::create(const dsg_config *cfg, bool alone, dsg_ctx **out) {
   if (!cfg || !out) return dsg::set_error(nullptr, DSG_E_ARG, "null argument");
   *out = nullptr;
   if (cfg->nx < 4 || cfg->ny < 4 || cfg->nz < 4)
@@ -909,6 +1044,12 @@ int dsg_create(const dsg_config *cfg, dsg_ctx **out) {
            up(sizeof(unsigned)) + up(dsg::kRedBlocks * 6 * sizeof(double)) + up(16 * sizeof(double));
   const Dims fd{cfg->nx, cfg->ny, cfg->nz};
   total += up(dsg::segment_flags(fd)) + up(dsg::segment_codes(fd));
+  ctx->alone = alone;
+  level_plan(ctx);
+  for (int l = 1; l <= ng; l++) {
+    total += up(dsg::mgg::mail_words<float>(ctx->gr32[l].g) * 8) + up(ctx->gr32[l].g.blocks() * sizeof(unsigned));
+    total += up(dsg::mgg::mail_words<double>(ctx->gr64[l].g) * 8) + up(ctx->gr64[l].g.blocks() * sizeof(unsigned));
+  }
   cudaError_t e = cudaMalloc(&ctx->arena, total);
   if (e != cudaSuccess) {
     int rc = dsg::cuda_fail(ctx, e, "cudaMalloc(arena)");
@@ -952,6 +1093,17 @@ int dsg_create(const dsg_config *cfg, dsg_ctx **out) {
   ctx->seg_flags = (unsigned char *)p;
   p += up(dsg::segment_flags(fd));
   ctx->seg_codes = (unsigned char *)p;
+  p += up(dsg::segment_codes(fd));
+  for (int l = 1; l <= ng; l++) {
+    auto mail = [&](auto &G, size_t words) {
+      G.mail = (unsigned long long *)p;
+      p += up(words * 8);
+      G.epoch = (unsigned *)p;
+      p += up(G.g.blocks() * sizeof(unsigned));
+    };
+    mail(ctx->gr32[l], dsg::mgg::mail_words<float>(ctx->gr32[l].g));
+    mail(ctx->gr64[l], dsg::mgg::mail_words<double>(ctx->gr64[l].g));
+  }
   e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->red_host, 16 * sizeof(double));
   if (e == cudaSuccess) e = cudaMemsetAsync(ctx->arena, 0, total, ctx->own_stream);
@@ -970,11 +1122,12 @@ int dsg_create(const dsg_config *cfg, dsg_ctx **out) {
   ctx->s.cycles = cfg->cycles;
   ctx->s.ng = ng;
   ctx->s.last_epsdiv = -1.0;
-  cluster_plan(ctx);
   nondim(ctx);
   *out = ctx;
   return DSG_OK;
 }
+
+extern "C" {
 
 void dsg_destroy(dsg_ctx *ctx) {
   if (!ctx) return;

@@ -43,6 +43,28 @@ struct Dims {
   __host__ __device__ __forceinline__ size_t sz() const { return (size_t)nx * ny; }
 };
 
+#ifdef __CUDACC__
+// The ghosts whose nearest interior cell is (i,j,k), as bc_scalar sets them: 0
+// beyond x = nx, the cell's value v elsewhere.
+template <class T>
+__device__ __forceinline__ void write_ghosts(T *u, Dims d, int i, int j, int k, T v) {
+  const int i0 = i == 2 ? 1 : i, i1 = i == d.nx - 1 ? d.nx : i;
+  const int j0 = j == 2 ? 1 : j, j1 = j == d.ny - 1 ? d.ny : j;
+  const int k0 = k == 2 ? 1 : k, k1 = k == d.nz - 1 ? d.nz : k;
+  if (i0 == i1 && j0 == j1 && k0 == k1) return;
+  for (int kk = k0; kk <= k1; kk++)
+    for (int jj = j0; jj <= j1; jj++)
+      for (int ii = i0; ii <= i1; ii++)
+        if (ii != i || jj != j || kk != k) u[d.ix(ii, jj, kk)] = ii == d.nx ? T(0) : v;
+}
+#endif
+
+}  // namespace dsg
+
+#include "mggrid.cuh"
+
+namespace dsg {
+
 // Bit-pattern tests of doubles on the integer pipe.  GB300's FP64 comparisons
 // issue on the FP64 pipe (as slow as its FMAs), and the exact fast paths test
 // up to 27 values per cell.  same_bits differs from == only for +0/-0 and
@@ -218,6 +240,15 @@ int cluster32_size();
 int cluster64_size();
 cudaError_t cluster32(const mgc::Args<float> &args, cudaStream_t st);
 cudaError_t cluster64(const mgc::Args<double> &args, bool fma, cudaStream_t st);
+// a smoothing phase of one level in one cooperative launch (mggrid.cuh);
+// grid*_blocks: blocks it may have (0: none); cells
+// and halo cells per thread and colour, at most.  FP64 stops at one cell (42^3
+// cells): at 64^3 the FP64 units take 5.9 us for a pass either way.
+constexpr int kGrid32Cells = 8, kGrid32Halo = 8, kGrid64Cells = 1, kGrid64Halo = 2;
+int grid32_blocks();
+int grid64_blocks();
+cudaError_t grid32(const mgg::Args<float> &args, cudaStream_t st);
+cudaError_t grid64(const mgg::Args<double> &args, bool fma, cudaStream_t st);
 // finest level in colour-split storage ({even, odd} arrays of (nx-2)/2 x (ny-2) x (nz-2))
 // (flags: of the uniform segments, to32_flags)
 cudaError_t relax32_split_n(int n, float *const u[2], float *const rhs[2], const float *cc,
@@ -303,6 +334,10 @@ struct dsg_ctx {
   int tail64_top = 0;         // the same for the FP64 multigrid
   dsg::mgc::Args<float> cl32;    // their slabs and shared-memory layout
   dsg::mgc::Args<double> cl64;
+  bool alone = true;          // not a member of an ensemble, whose members share the GPU
+  // levels whose smoothing phases are one cooperative launch (blocks() = 0: not)
+  dsg::mgg::Args<float> gr32[32];
+  dsg::mgg::Args<double> gr64[32];
   int lnx[32], lny[32], lnz[32];
   double *lv[32][8];          // [level][CC,P,RES,RHS,A,B,C,EI], level 1..ng
   float *lv32[32][6];         // FP32 hierarchy [level][U,RHS,A,B,C,EI] of the mixed mode;
@@ -484,6 +519,8 @@ inline void tail_args(dsg_ctx *ctx, int top, dsg::TailArgs *A) {
 
 }  // namespace mixed
 
+// dsg_create; alone: the context expects the GPU for itself (not an ensemble's member)
+int create(const dsg_config *cfg, bool alone, dsg_ctx **out);
 int set_error(dsg_ctx *ctx, int code, const char *fmt, ...);
 int cuda_fail(dsg_ctx *ctx, cudaError_t e, const char *where);
 // A time step in two halves around its pressure solve (dsg.cu), and the

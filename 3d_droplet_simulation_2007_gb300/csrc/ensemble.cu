@@ -234,7 +234,7 @@ int dsg_ensemble_create(const dsg_config *cfgs, int n, int workers, dsg_ensemble
   dsg_ensemble *e = new dsg_ensemble();
   for (int i = 0; i < n; i++) {
     dsg_ctx *c = nullptr;
-    int rc = dsg_create(&cfgs[i], &c);
+    int rc = dsg::create(&cfgs[i], false, &c);
     if (!rc) rc = dsg_init_drop(c);
     if (rc) {
       std::string msg = std::string("member ") + std::to_string(i) + ": " + dsg_last_error(c);

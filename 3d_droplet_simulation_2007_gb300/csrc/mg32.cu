@@ -101,6 +101,25 @@ struct Cluster32 {
     acc += r7;
     return 0.125f * acc;
   }
+  // u of a coarse node array at fine node (i, j, k)
+  static __device__ __forceinline__ float coarse(const float *uc, Dims dc, int i, int j, int k, int tri) {
+    return tri ? coarse_at<true>(uc, dc, i, j, k) : coarse_at<false>(uc, dc, i, j, k);
+  }
+  // Face coefficients and ei of a node of the finest level from its cc, as
+  // relax32_split_cell forms them.
+  static __device__ __forceinline__ void split_coefs(const mgg::Args<float> &G, Dims d, int i, int j, int k,
+                                                     float (&f)[8]) {
+    const float *cq = G.cc + ix32(d, i, j, k);
+    const int sy = d.nx, sz = d.nx * d.ny;
+    const float c0 = cq[0];
+    f[0] = face_coef(c0, cq[1], G.r1, G.r2);
+    f[1] = (i == 2) ? f[0] : face_coef(cq[-1], c0, G.r1, G.r2);
+    f[2] = face_coef(c0, cq[sy], G.r1, G.r2);
+    f[3] = face_coef(cq[-sy], c0, G.r1, G.r2);
+    f[4] = face_coef(c0, cq[sz], G.r1, G.r2);
+    f[5] = face_coef(cq[-sz], c0, G.r1, G.r2);
+    f[6] = rcp_approx(f[0] + f[1] + f[2] + f[3] + f[4] + f[5]);
+  }
   // Coarse planes c0, c0 + 1 .. of `buf` at fine cell (x, y, k), 0-based.
   static __device__ __forceinline__ float prolong(const float *buf, int nx, int ny, int nz, int c0, int x, int y,
                                                   int k, int tri) {
@@ -120,6 +139,11 @@ struct Cluster32 {
 
 __global__ void __launch_bounds__(mgc::kThreads, 1) k_cluster32(const __grid_constant__ mgc::Args<float> G) {
   mgc::cluster_mg<Cluster32>(G);
+}
+
+template <int NC, int NH, bool SPLIT>
+__global__ void __launch_bounds__(mgg::kThreads, 1) k_grid32(const __grid_constant__ mgg::Args<float> G) {
+  mgg::phase<Cluster32, NC, NH, SPLIT>(G);
 }
 
 __global__ void k_restrict32(float *__restrict__ uc, const float *__restrict__ uf, Dims dc, Dims df) {
@@ -480,6 +504,24 @@ cudaError_t resid_restrict32(float *rhs_c, float *u_c, const float *u, const flo
   const Dims dc{df.nx / 2 + 1, df.ny / 2 + 1, df.nz / 2 + 1};
   DSG_COUNT k_resid_restrict32<<<interior_grid(dc, kBlk), kBlk, 0, st>>>(rhs_c, u_c, u, rhs, a, b, c, df, dc, h2i);
   return cudaGetLastError();
+}
+
+template <bool SPLIT>
+static cudaError_t grid32_s(const mgg::Args<float> &G, cudaStream_t st) {
+  const int halo = (G.g.words() + mgg::kThreads - 1) / mgg::kThreads;
+  if (G.g.cells <= 1 && halo <= 2) return mgg::launch(k_grid32<1, 2, SPLIT>, G, st);
+  if (G.g.cells <= 2 && halo <= 4) return mgg::launch(k_grid32<2, 4, SPLIT>, G, st);
+  if (G.g.cells <= 4 && halo <= 4) return mgg::launch(k_grid32<4, 4, SPLIT>, G, st);
+  return mgg::launch(k_grid32<8, 8, SPLIT>, G, st);
+}
+
+int grid32_blocks() {
+  return mgg::grid_blocks(k_grid32<1, 2, false>, k_grid32<2, 4, false>, k_grid32<4, 4, false>, k_grid32<8, 8, false>,
+                          k_grid32<1, 2, true>, k_grid32<2, 4, true>, k_grid32<4, 4, true>, k_grid32<8, 8, true>);
+}
+
+cudaError_t grid32(const mgg::Args<float> &args, cudaStream_t st) {
+  return args.u ? grid32_s<false>(args, st) : grid32_s<true>(args, st);
 }
 
 int cluster32_size() { return mgc::cluster_size(k_cluster32); }

@@ -172,18 +172,7 @@ __global__ void k_relax_colour(double *__restrict__ u, const double *__restrict_
   const double v = relax_value<R>(uc, xp, xm, yp, ym, zp, zm, a[q], a[q - 1], b[q], b[q - sy], c[q], c[q - sz], ei[q],
                                   rhs[q], h2, omega);
   u[q] = v;
-  if (GHOSTS) {
-    // ghosts whose nearest interior cell this is: 1 = v, nx = 0 along x; the
-    // cell's own value along y and z
-    const int i0 = i == 2 ? 1 : i, i1 = i == d.nx - 1 ? d.nx : i;
-    const int j0 = j == 2 ? 1 : j, j1 = j == d.ny - 1 ? d.ny : j;
-    const int k0 = k == 2 ? 1 : k, k1 = k == d.nz - 1 ? d.nz : k;
-    if (i0 == i1 && j0 == j1 && k0 == k1) return;
-    for (int kk = k0; kk <= k1; kk++)
-      for (int jj = j0; jj <= j1; jj++)
-        for (int ii = i0; ii <= i1; ii++)
-          if (ii != i || jj != j || kk != k) u[d.ix(ii, jj, kk)] = ii == d.nx ? 0.0 : v;
-  }
+  if (GHOSTS) write_ghosts(u, d, i, j, k, v);
 }
 
 // Arithmetic of the cluster kernel on the FP64 levels: the two forms of
@@ -206,6 +195,10 @@ struct Cluster64 {
                                                  double r6, double r7) {
     return 0.125 * (r0 + r1 + r2 + r3 + r4 + r5 + r6 + r7);
   }
+  // u of a coarse node array at fine node (i, j, k)
+  static __device__ __forceinline__ double coarse(const double *uc, Dims dc, int i, int j, int k, int) {
+    return uc[dc.ix((i >> 1) + 1, (j >> 1) + 1, (k >> 1) + 1)];
+  }
   static __device__ __forceinline__ double prolong(const double *buf, int nx, int ny, int, int c0, int x, int y, int k,
                                                    int) {
     return buf[((k >> 1) - c0) * nx * ny + (y >> 1) * nx + (x >> 1)];
@@ -215,6 +208,11 @@ struct Cluster64 {
 template <Round R>
 __global__ void __launch_bounds__(mgc::kThreads, 1) k_cluster64(const __grid_constant__ mgc::Args<double> G) {
   mgc::cluster_mg<Cluster64<R>>(G);
+}
+
+template <Round R>
+__global__ void __launch_bounds__(mgg::kThreads, 1) k_grid64(const __grid_constant__ mgg::Args<double> G) {
+  mgg::phase<Cluster64<R>, kGrid64Cells, kGrid64Halo, false>(G);
 }
 
 // Residual of an interior cell, its neighbours' values from memory.
@@ -710,6 +708,16 @@ cudaError_t cluster64(const mgc::Args<double> &args, bool fma, cudaStream_t st) 
   for (int l = 2; l <= args.top && r == REF2; l++) r = rounding(fma, args.lv[l].h2, args.omega);
   return r == FMA ? mgc::launch(k_cluster64<FMA>, args, st)
                   : (r == REF2 ? mgc::launch(k_cluster64<REF2>, args, st) : mgc::launch(k_cluster64<REF>, args, st));
+}
+
+int grid64_blocks() { return mgg::grid_blocks(k_grid64<REF>, k_grid64<REF2>, k_grid64<FMA>); }
+
+cudaError_t grid64(const mgg::Args<double> &args, bool fma, cudaStream_t st) {
+  switch (rounding(fma, args.h2, args.omega)) {
+    case FMA: return mgg::launch(k_grid64<FMA>, args, st);
+    case REF2: return mgg::launch(k_grid64<REF2>, args, st);
+    default: return mgg::launch(k_grid64<REF>, args, st);
+  }
 }
 
 cudaError_t relax(double *u, double lengthsize, const double *rhs, const double *a, const double *b,
