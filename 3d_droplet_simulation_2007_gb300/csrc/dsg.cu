@@ -376,6 +376,12 @@ int coarse32(dsg_ctx *ctx, bool fmg) {
   return DSG_OK;
 }
 
+// Flags and bulk coefficients of a level with phases of mgbox.cuh.
+void box_coefs(dsg_ctx *ctx, int l, dsg::mgg::Args<float> &G) {
+  G.flags = ctx->node_flags[l];
+  dsg::bulk_coefs(0.5 * (ctx->s.rho1 - ctx->s.rho2), ctx->s.rho2, l == ctx->ng - 1, G.bulk, G.bulk_ei);
+}
+
 // phase64's counterpart on the FP32 levels.
 int phase32(dsg_ctx *ctx, int l, int n, bool down, bool up, bool add) {
   dsg::mgg::Args<float> &G = ctx->gr32[l];
@@ -396,6 +402,7 @@ int phase32(dsg_ctx *ctx, int l, int n, bool down, bool up, bool add) {
     G.b = L[B32];
     G.c = L[C32];
     G.ei = L[EI32];
+    if (G.box) box_coefs(ctx, l, G);
   }
   G.h2 = level_h2(ctx, l);
   G.h2i = 1.0f / level_h2(ctx, l);
@@ -575,6 +582,13 @@ int coef_hierarchy32(dsg_ctx *ctx, cudaStream_t st) {
   for (int g = ng - 2; g >= 1; g--) {
     float **C = ctx->lv32[g], **Fi = ctx->lv32[g + 1];
     DSG_CK(ctx, dsg::acfromac32(C[A32], C[B32], C[C32], C[EI32], Fi[A32], Fi[B32], Fi[C32], ctx->level(g), st));
+  }
+  for (int g = 2; g < ng; g++) {
+    float **L = ctx->lv32[g];
+    auto &G = ctx->gr32[g];
+    if (!G.box) continue;
+    box_coefs(ctx, g, G);
+    DSG_CK(ctx, dsg::node_flags(ctx->node_flags[g], L[A32], L[B32], L[C32], L[EI32], ctx->level(g), G.bulk, G.bulk_ei, st));
   }
   return DSG_OK;
 }
@@ -976,8 +990,12 @@ void level_plan(dsg_ctx *ctx) {
                        !dsg::mgg::layout(G)))
       G.g.py = G.g.pz = 0;
   };
+  const int box = g32 > 0 ? dsg::box32_blocks() : 0;
   for (int l = 2; l <= ctx->ng; l++) {
     if (l > ctx->tail_top) cut(ctx->gr32[l], l, g32, sizeof(float), dsg::kGrid32Cells, dsg::kGrid32Halo);
+    auto &G = ctx->gr32[l];
+    if (l > ctx->tail_top && l < ctx->ng && box > 0 && G.g.blocks() == 0)
+      dsg::mgg::plan_box(G, ctx->lnx[l] - 2, ctx->lny[l] - 2, ctx->lnz[l] - 2, box);
     if (l > ctx->tail64_top) cut(ctx->gr64[l], l, g64, sizeof(double), dsg::kGrid64Cells, dsg::kGrid64Halo);
   }
 }
@@ -1047,6 +1065,7 @@ int dsg::create(const dsg_config *cfg, bool alone, dsg_ctx **out) {
   ctx->alone = alone;
   level_plan(ctx);
   for (int l = 1; l <= ng; l++) {
+    if (ctx->gr32[l].box && l < ng) total += up(dsg::node_flag_bytes(ctx->level(l)));
     total += up(dsg::mgg::mail_words<float>(ctx->gr32[l].g) * 8) + up(ctx->gr32[l].g.blocks() * sizeof(unsigned));
     total += up(dsg::mgg::mail_words<double>(ctx->gr64[l].g) * 8) + up(ctx->gr64[l].g.blocks() * sizeof(unsigned));
   }
@@ -1101,6 +1120,8 @@ int dsg::create(const dsg_config *cfg, bool alone, dsg_ctx **out) {
       G.epoch = (unsigned *)p;
       p += up(G.g.blocks() * sizeof(unsigned));
     };
+    ctx->node_flags[l] = (unsigned char *)p;
+    if (ctx->gr32[l].box && l < ng) p += up(dsg::node_flag_bytes(ctx->level(l)));
     mail(ctx->gr32[l], dsg::mgg::mail_words<float>(ctx->gr32[l].g));
     mail(ctx->gr64[l], dsg::mgg::mail_words<double>(ctx->gr64[l].g));
   }

@@ -62,6 +62,7 @@ __device__ __forceinline__ void write_ghosts(T *u, Dims d, int i, int j, int k, 
 }  // namespace dsg
 
 #include "mggrid.cuh"
+#include "mgbox.cuh"
 
 namespace dsg {
 
@@ -246,6 +247,7 @@ cudaError_t cluster64(const mgc::Args<double> &args, bool fma, cudaStream_t st);
 // cells): at 64^3 the FP64 units take 5.9 us for a pass either way.
 constexpr int kGrid32Cells = 8, kGrid32Halo = 8, kGrid64Cells = 1, kGrid64Halo = 2;
 int grid32_blocks();
+int box32_blocks();  // of mgbox.cuh
 int grid64_blocks();
 cudaError_t grid32(const mgg::Args<float> &args, cudaStream_t st);
 cudaError_t grid64(const mgg::Args<double> &args, bool fma, cudaStream_t st);
@@ -267,6 +269,13 @@ cudaError_t correct64(double *p, float *const e[2], Dims d, int init, cudaStream
 // FP32 volume fraction of all nodes, and the flags of the finest level's
 // uniform segments (codes: scratch), segment_flags / segment_codes bytes
 size_t segment_codes(Dims d);
+size_t node_flag_bytes(Dims d);
+// flags of the uniform cells of a level with node arrays; the coefficient and ei
+// of gas and liquid there (a uniform coefficient is its own mean on every
+// level, ei as acfromac64to32 (from64) or acfromac32 forms it)
+cudaError_t node_flags(unsigned char *flags, const float *a, const float *b, const float *c, const float *ei, Dims d,
+                       const float (&f)[2], const float (&e)[2], cudaStream_t st);
+void bulk_coefs(double r1, double r2, bool from64, float (&f)[2], float (&e)[2]);
 size_t segment_flags(Dims d);
 cudaError_t to32_flags(float *dst, unsigned char *flags, unsigned char *codes, const double *src, Dims d,
                        cudaStream_t st);
@@ -338,6 +347,7 @@ struct dsg_ctx {
   // levels whose smoothing phases are one cooperative launch (blocks() = 0: not)
   dsg::mgg::Args<float> gr32[32];
   dsg::mgg::Args<double> gr64[32];
+  unsigned char *node_flags[32];  // uniform cells of a level below the finest with phases of mgbox.cuh
   int lnx[32], lny[32], lnz[32];
   double *lv[32][8];          // [level][CC,P,RES,RHS,A,B,C,EI], level 1..ng
   float *lv32[32][6];         // FP32 hierarchy [level][U,RHS,A,B,C,EI] of the mixed mode;

@@ -105,6 +105,12 @@ struct Cluster32 {
   static __device__ __forceinline__ float coarse(const float *uc, Dims dc, int i, int j, int k, int tri) {
     return tri ? coarse_at<true>(uc, dc, i, j, k) : coarse_at<false>(uc, dc, i, j, k);
   }
+  // its parts: the combination along y and z at coarse x-index x, and along x
+  static __device__ __forceinline__ float coarse_yz(const float *uc, Dims dc, int x, int j, int k) {
+    const int pj = (j >> 1) + 1, pk = (k >> 1) + 1;
+    return tri_yz(uc, dc, x, pj, tri_nb(j, pj, dc.ny), pk, tri_nb(k, pk, dc.nz));
+  }
+  static __device__ __forceinline__ float coarse_x(float yp, float yn) { return tri_x(yp, yn); }
   // Face coefficients and ei of a node of the finest level from its cc, as
   // relax32_split_cell forms them.
   static __device__ __forceinline__ void split_coefs(const mgg::Args<float> &G, Dims d, int i, int j, int k,
@@ -144,6 +150,29 @@ __global__ void __launch_bounds__(mgc::kThreads, 1) k_cluster32(const __grid_con
 template <int NC, int NH, bool SPLIT>
 __global__ void __launch_bounds__(mgg::kThreads, 1) k_grid32(const __grid_constant__ mgg::Args<float> G) {
   mgg::phase<Cluster32, NC, NH, SPLIT>(G);
+}
+
+__global__ void __launch_bounds__(mgg::kBoxThreads, 1) k_box32(const __grid_constant__ mgg::Args<float> G) {
+  mgg::box_phase<Cluster32>(G);
+}
+
+// Flags of mgbox.cuh on a level with node arrays: whether eight cells of a row,
+// from x = 8 m on, have gas's (1) or liquid's (2) coefficient on every face and
+// its ei.
+__global__ void k_node_flags(unsigned char *__restrict__ flags, const float *__restrict__ a,
+                             const float *__restrict__ b, const float *__restrict__ c, const float *__restrict__ ei,
+                             Dims d, float gas, float e_gas, float liq, float e_liq) {
+  const int n8 = (d.nx - 2) >> 3, m = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y + 2,
+            k = blockIdx.z + 2;
+  if (m >= n8 || j > d.ny - 1) return;
+  const unsigned q = ix32(d, 8 * m + 2, j, k), sy = d.nx, sz = (unsigned)d.nx * d.ny;
+  const bool liquid = a[q] != gas;
+  const float f = liquid ? liq : gas, e = liquid ? e_liq : e_gas;
+  bool same = a[q - 1] == f;
+#pragma unroll
+  for (int t = 0; t < 8; t++)
+    same = same && a[q + t] == f && b[q + t] == f && b[q + t - sy] == f && c[q + t] == f && c[q + t - sz] == f && ei[q + t] == e;
+  flags[(unsigned)m + (unsigned)n8 * ((unsigned)(j - 2) + (unsigned)(d.ny - 2) * (unsigned)(k - 2))] = !same ? 0 : liquid ? 2 : 1;
 }
 
 __global__ void k_restrict32(float *__restrict__ uc, const float *__restrict__ uf, Dims dc, Dims df) {
@@ -509,18 +538,21 @@ cudaError_t resid_restrict32(float *rhs_c, float *u_c, const float *u, const flo
 template <bool SPLIT>
 static cudaError_t grid32_s(const mgg::Args<float> &G, cudaStream_t st) {
   const int halo = (G.g.words() + mgg::kThreads - 1) / mgg::kThreads;
-  if (G.g.cells <= 1 && halo <= 2) return mgg::launch(k_grid32<1, 2, SPLIT>, G, st);
-  if (G.g.cells <= 2 && halo <= 4) return mgg::launch(k_grid32<2, 4, SPLIT>, G, st);
-  if (G.g.cells <= 4 && halo <= 4) return mgg::launch(k_grid32<4, 4, SPLIT>, G, st);
-  return mgg::launch(k_grid32<8, 8, SPLIT>, G, st);
+  if (G.g.cells <= 1 && halo <= 2) return mgg::launch(k_grid32<1, 2, SPLIT>, mgg::kThreads, G, st);
+  if (G.g.cells <= 2 && halo <= 4) return mgg::launch(k_grid32<2, 4, SPLIT>, mgg::kThreads, G, st);
+  if (G.g.cells <= 4 && halo <= 4) return mgg::launch(k_grid32<4, 4, SPLIT>, mgg::kThreads, G, st);
+  return mgg::launch(k_grid32<8, 8, SPLIT>, mgg::kThreads, G, st);
 }
 
 int grid32_blocks() {
-  return mgg::grid_blocks(k_grid32<1, 2, false>, k_grid32<2, 4, false>, k_grid32<4, 4, false>, k_grid32<8, 8, false>,
+  return mgg::grid_blocks(mgg::kThreads, mgg::kMaxShared, k_grid32<1, 2, false>, k_grid32<2, 4, false>, k_grid32<4, 4, false>, k_grid32<8, 8, false>,
                           k_grid32<1, 2, true>, k_grid32<2, 4, true>, k_grid32<4, 4, true>, k_grid32<8, 8, true>);
 }
 
+int box32_blocks() { return mgg::grid_blocks(mgg::kBoxThreads, mgg::kBoxShared, k_box32); }
+
 cudaError_t grid32(const mgg::Args<float> &args, cudaStream_t st) {
+  if (args.box) return mgg::launch(k_box32, mgg::kBoxThreads, args, st);
   return args.u ? grid32_s<false>(args, st) : grid32_s<true>(args, st);
 }
 
@@ -588,6 +620,24 @@ cudaError_t to32_flags(float *dst, unsigned char *flags, unsigned char *codes, c
                        cudaStream_t st) {
   DSG_COUNT k_codes<<<flat_blocks(32 * segment_codes(d)), 256, 0, st>>>(dst, codes, src, d);
   if (split_vec(Split{(d.nx - 2) >> 1, d.ny - 2, d.nz - 2})) DSG_COUNT k_flags<<<flat_blocks(segment_flags(d)), 256, 0, st>>>(flags, codes, d);
+  return cudaGetLastError();
+}
+
+size_t node_flag_bytes(Dims d) { return (size_t)((d.nx - 2) >> 3) * (d.ny - 2) * (d.nz - 2); }
+
+void bulk_coefs(double r1, double r2, bool from64, float (&f)[2], float (&e)[2]) {
+  for (int q = 0; q < 2; q++) {
+    const double x = 1.0 / (r1 * (q + q) + r2);
+    f[q] = (float)x;
+    e[q] = from64 ? (float)(1.0 / (x + x + x + x + x + x)) : 1.f / (f[q] + f[q] + f[q] + f[q] + f[q] + f[q]);
+  }
+}
+
+cudaError_t node_flags(unsigned char *flags, const float *a, const float *b, const float *c, const float *ei, Dims d,
+                       const float (&f)[2], const float (&e)[2], cudaStream_t st) {
+  const dim3 blk(16, 16);
+  DSG_COUNT k_node_flags<<<dim3(((d.nx - 2) / 8 + 15) / 16, (d.ny - 2 + 15) / 16, d.nz - 2), blk, 0, st>>>(
+      flags, a, b, c, ei, d, f[0], e[0], f[1], e[1]);
   return cudaGetLastError();
 }
 

@@ -85,6 +85,16 @@ __device__ __forceinline__ float face_sum(float ae, float xp, float aw, float xm
   t = fmaf(cb, zm, t);
   return fmaf(-h2, rhs, t);
 }
+// Sum over the six faces of coefficient times the difference to the
+// neighbour, and the residual that follows from it.
+__device__ __forceinline__ float face_diff(float uc, float ae, float xp, float aw, float xm, float bn, float yp,
+                                           float bs, float ym, float ct, float zp, float cb, float zm) {
+  float t = fmaf(ae, xp - uc, aw * (xm - uc));
+  t = fmaf(bn, yp - uc, t);
+  t = fmaf(bs, ym - uc, t);
+  t = fmaf(ct, zp - uc, t);
+  return fmaf(cb, zm - uc, t);
+}
 // omega * t + (1 - omega) * u
 __device__ __forceinline__ float over_relax(float omega, float t, float u) {
   return fmaf(1.f - omega, u, omega * t);
@@ -397,9 +407,7 @@ __device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const ui
           ct = face_coef(c0, cq[sz], r1, r2);
           cb = face_coef(cq[-sz], c0, r1, r2);
         }
-        const float lap = ae * (xp - uc) + aw * (xm - uc) + bn * (yp - uc) + bs * (ym - uc) + ct * (zp - uc) +
-                          cb * (zm - uc);
-        acc += split_get(re, ro, sp, i, j, k) - h2i * lap;
+        acc += fmaf(-h2i, face_diff(uc, ae, xp, aw, xm, bn, yp, bs, ym, ct, zp, cb, zm), split_get(re, ro, sp, i, j, k));
       }
   const unsigned qc = ix32(dc, ic, jc, kc);
   rhs_c[qc] = 0.125f * acc;
@@ -479,9 +487,7 @@ __device__ __forceinline__ float relax32_value(float uc, const Nb &n, float ae, 
 }
 __device__ __forceinline__ float resid32_value(float uc, const Nb &n, float ae, float aw, float bn, float bs, float ct,
                                                float cb, float rhs, float h2i) {
-  const float lap = ae * (n.xp - uc) + aw * (n.xm - uc) + bn * (n.yp - uc) + bs * (n.ym - uc) + ct * (n.zp - uc) +
-                    cb * (n.zm - uc);
-  return rhs - h2i * lap;
+  return fmaf(-h2i, face_diff(uc, ae, n.xp, aw, n.xm, bn, n.yp, bs, n.ym, ct, n.zp, cb, n.zm), rhs);
 }
 
 // One red-black update of cell (i,j,k).

@@ -710,13 +710,13 @@ cudaError_t cluster64(const mgc::Args<double> &args, bool fma, cudaStream_t st) 
                   : (r == REF2 ? mgc::launch(k_cluster64<REF2>, args, st) : mgc::launch(k_cluster64<REF>, args, st));
 }
 
-int grid64_blocks() { return mgg::grid_blocks(k_grid64<REF>, k_grid64<REF2>, k_grid64<FMA>); }
+int grid64_blocks() { return mgg::grid_blocks(mgg::kThreads, mgg::kMaxShared, k_grid64<REF>, k_grid64<REF2>, k_grid64<FMA>); }
 
 cudaError_t grid64(const mgg::Args<double> &args, bool fma, cudaStream_t st) {
   switch (rounding(fma, args.h2, args.omega)) {
-    case FMA: return mgg::launch(k_grid64<FMA>, args, st);
-    case REF2: return mgg::launch(k_grid64<REF2>, args, st);
-    default: return mgg::launch(k_grid64<REF>, args, st);
+    case FMA: return mgg::launch(k_grid64<FMA>, mgg::kThreads, args, st);
+    case REF2: return mgg::launch(k_grid64<REF2>, mgg::kThreads, args, st);
+    default: return mgg::launch(k_grid64<REF>, mgg::kThreads, args, st);
   }
 }
 

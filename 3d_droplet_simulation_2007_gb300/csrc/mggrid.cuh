@@ -68,6 +68,9 @@ struct Args {
   int staged;                   // ei and rhs in shared memory
   int o_er, o_res;              // element offsets in shared memory
   size_t shared;
+  int box;                      // a phase of mgbox.cuh
+  const unsigned char *flags;   // per eight cells of a row: uniform (1 gas, 2 liquid)
+  T bulk[2], bulk_ei[2];        // face coefficient and ei of gas and liquid
 };
 
 // The cut of a level over at most `sms` blocks: the boxes with the least work
@@ -419,15 +422,15 @@ __device__ void phase(const Args<typename A::T> &G) {
 // the current device, a few SMs left to other streams; 0: none.  Sets the
 // kernels' shared-memory attribute on that device.
 template <class... K>
-int grid_blocks(K... kernels) {
+int grid_blocks(int threads, size_t shared, K... kernels) {
   int dev = 0, sms = 0, coop = 0;
   bool ok = cudaGetDevice(&dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop;
   auto one = [&](auto k) {
     int n = 0;
-    ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxShared) == cudaSuccess &&
-         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kThreads, kMaxShared) == cudaSuccess && n > 0;
+    ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, shared) == cudaSuccess && n > 0;
   };
   (one(kernels), ...);
   cudaGetLastError();
@@ -435,13 +438,13 @@ int grid_blocks(K... kernels) {
 }
 
 template <class K, class T>
-cudaError_t launch(K kernel, const Args<T> &args, cudaStream_t st) {
+cudaError_t launch(K kernel, int threads, const Args<T> &args, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   cfg.gridDim = dim3((unsigned)args.g.blocks());
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = args.shared;
   cfg.stream = st;
   cfg.attrs = at;
