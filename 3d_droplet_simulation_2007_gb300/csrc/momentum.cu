@@ -76,46 +76,103 @@ __global__ void k_predictor(double *__restrict__ w1, double *__restrict__ w2, do
   w3[q] = w[q] + c[q - sz] * (S13[q + 1] - S13[q] + S23[q + sy] - S23[q] + S33[q] - S33[q - sz]);
 }
 
+// Explicit convection (main.f's convective): per component three differences of
+// products of two-point sums.  The FP64 pipe bounds it, and cell by cell it
+// takes 51 instructions per cell, 30 of them sums that its neighbours along x, y
+// and z form as well: 1360 us at 256^3.  Here a cell forms nine sums once and
+// takes its neighbours': along x by shuffle, along y through shared memory,
+// along z from the plane before: 30 instructions.  A block is kConvRows rows of
+// 32 cells, one warp each, and marches through `planes` planes; two more warps
+// form the sums of the row and the column of cells beyond.  256^3: 963 us,
+// 904 at the pipe's rate; 128^3 173 -> 133, 64^3 24.5 -> 22.0.
+//
 // tauq = 0.25*tauh: the reference's tauh*(0.25*x) equals tauq*x bit for bit
 // (scaling by 0.25 is exact, so both round the same product once), one FP64
-// multiply per component less on GB300's narrow FP64 pipe.
-__global__ void k_convective(double *__restrict__ u, double *__restrict__ v, double *__restrict__ w,
-                             const double *__restrict__ w1, const double *__restrict__ w2,
-                             const double *__restrict__ w3, Dims d, double tauq) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  if (i > d.nx - 1 || j > d.ny - 1) return;
-  const size_t q = d.ix(i, j, k);
+// multiply per component less.
+constexpr int kConvRows = 8, kConvThreads = 32 * (kConvRows + 2);
+
+// p*p - m*m + a*b - c*e + f*g - r*t, rounded as the compiler rounds that expression
+__device__ __forceinline__ double flux_balance(double p, double m, double a, double b, double c, double e, double f,
+                                               double g, double r, double t) {
+  double x = fma(p, p, -(m * m));
+  x = fma(a, b, x);
+  x = fma(-c, e, x);
+  x = fma(f, g, x);
+  return fma(-r, t, x);
+}
+
+__global__ void __launch_bounds__(kConvThreads) k_convective(double *__restrict__ u, double *__restrict__ v,
+                                                             double *__restrict__ w, const double *__restrict__ w1,
+                                                             const double *__restrict__ w2,
+                                                             const double *__restrict__ w3, Dims d, double tauq,
+                                                             int planes) {
+  __shared__ double rows[2][5][kConvRows + 1][32], column[2][5][kConvRows];
+  const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+  const bool beside = wy == kConvRows + 1, below = wy == kConvRows;  // the column's, the row's warp
+  int i = 2 + 32 * (int)blockIdx.x + (beside ? 32 : lane);
+  int j = 2 + kConvRows * (int)blockIdx.y + (beside ? min(lane, kConvRows - 1) : wy);
+  const bool cell = wy < kConvRows && i <= d.nx - 1 && j <= d.ny - 1;
+  i = min(i, d.nx);
+  j = min(j, d.ny);
+  const int k0 = 2 + planes * (int)blockIdx.z, k1 = min(k0 + planes, d.nz);
   const long sy = (long)d.sy(), sz = (long)d.sz();
-#define W1(di, dj, dk) w1[(long)q + (long)(di) + (long)(dj) * sy + (long)(dk) * sz]
-#define W2(di, dj, dk) w2[(long)q + (long)(di) + (long)(dj) * sy + (long)(dk) * sz]
-#define W3(di, dj, dk) w3[(long)q + (long)(di) + (long)(dj) * sy + (long)(dk) * sz]
-  double p, m, x;
-  p = W1(0, 0, 0) + W1(-1, 0, 0);
-  m = W1(1, 0, 0) + W1(0, 0, 0);
-  x = p * p - m * m + (W1(0, -1, 0) + W1(0, 0, 0)) * (W2(0, 0, 0) + W2(-1, 0, 0)) -
-      (W1(0, 1, 0) + W1(0, 0, 0)) * (W2(0, 1, 0) + W2(-1, 1, 0)) +
-      (W1(0, 0, -1) + W1(0, 0, 0)) * (W3(0, 0, 0) + W3(-1, 0, 0)) -
-      (W1(0, 0, 1) + W1(0, 0, 0)) * (W3(0, 0, 1) + W3(-1, 0, 1));
-  u[q] = W1(0, 0, 0) + tauq * x;
-  p = W2(0, 0, 0) + W2(0, -1, 0);
-  m = W2(0, 1, 0) + W2(0, 0, 0);
-  x = p * p - m * m + (W2(-1, 0, 0) + W2(0, 0, 0)) * (W1(0, 0, 0) + W1(0, -1, 0)) -
-      (W2(1, 0, 0) + W2(0, 0, 0)) * (W1(1, 0, 0) + W1(1, -1, 0)) +
-      (W2(0, 0, -1) + W2(0, 0, 0)) * (W3(0, 0, 0) + W3(0, -1, 0)) -
-      (W2(0, 0, 1) + W2(0, 0, 0)) * (W3(0, 0, 1) + W3(0, -1, 1));
-  v[q] = W2(0, 0, 0) + tauq * x;
-  p = W3(0, 0, 0) + W3(0, 0, -1);
-  m = W3(0, 0, 1) + W3(0, 0, 0);
-  x = p * p - m * m + (W3(-1, 0, 0) + W3(0, 0, 0)) * (W1(0, 0, 0) + W1(0, 0, -1)) -
-      (W3(1, 0, 0) + W3(0, 0, 0)) * (W1(1, 0, 0) + W1(1, 0, -1)) +
-      (W3(0, -1, 0) + W3(0, 0, 0)) * (W2(0, 0, 0) + W2(0, 0, -1)) -
-      (W3(0, 1, 0) + W3(0, 0, 0)) * (W2(0, 1, 0) + W2(0, 1, -1));
-  w[q] = W3(0, 0, 0) + tauq * x;
-#undef W1
-#undef W2
-#undef W3
+  long q = (long)d.ix(i, j, k0);
+  // sums with the neighbour below: a1x = w1 here + w1 at x - 1, and so on
+  double c1 = w1[q], c2 = w2[q], c3 = w3[q];
+  double a1z = c1 + w1[q - sz], a2z = c2 + w2[q - sz], a3z = c3 + w3[q - sz], a3x = c3 + w3[q - 1], a3y = c3 + w3[q - sy];
+  for (int k = k0, b = 0; k < k1; k++, b ^= 1, q += sz) {
+    const double n1 = w1[q + sz], n2 = w2[q + sz], n3 = w3[q + sz];
+    const double a1y = c1 + w1[q - sy], a2x = c2 + w2[q - 1];
+    double a1x = 0.0, a2y = 0.0, n1z = 0.0, n2z = 0.0, n3z = 0.0, n3x = 0.0, n3y = 0.0;
+    if (!below) {
+      a1x = c1 + w1[q - 1];
+      n1z = n1 + c1;
+      n3x = n3 + w3[q + sz - 1];
+    }
+    if (!beside) {
+      a2y = c2 + w2[q - sy];
+      n2z = n2 + c2;
+      n3y = n3 + w3[q + sz - sy];
+      double(&r)[5][kConvRows + 1][32] = rows[b];
+      r[0][wy][lane] = a1y;
+      r[1][wy][lane] = a2x;
+      r[2][wy][lane] = a2y;
+      r[3][wy][lane] = a2z;
+      r[4][wy][lane] = a3y;
+    } else if (lane < kConvRows) {
+      double(&r)[5][kConvRows] = column[b];
+      r[0][lane] = a1x;
+      r[1][lane] = a1y;
+      r[2][lane] = a1z;
+      r[3][lane] = a2x;
+      r[4][lane] = a3x;
+    }
+    __syncthreads();
+    if (wy < kConvRows) {
+      n3z = n3 + c3;
+      double x[5] = {a1x, a1y, a1z, a2x, a3x};  // of the cell at x + 1
+#pragma unroll
+      for (int t = 0; t < 5; t++) {
+        x[t] = __shfl_down_sync(0xffffffffu, x[t], 1);
+        if (lane == 31) x[t] = column[b][t][wy];
+      }
+      const double y1y = rows[b][0][wy + 1][lane], y2x = rows[b][1][wy + 1][lane], y2y = rows[b][2][wy + 1][lane],
+                   y2z = rows[b][3][wy + 1][lane], y3y = rows[b][4][wy + 1][lane];
+      if (cell) {
+        u[q] = fma(tauq, flux_balance(a1x, x[0], a1y, a2x, y1y, y2x, a1z, a3x, n1z, n3x), c1);
+        v[q] = fma(tauq, flux_balance(a2y, y2y, a2x, a1y, x[3], x[1], a2z, a3y, n2z, n3y), c2);
+        w[q] = fma(tauq, flux_balance(a3z, n3z, a3x, a1z, x[4], x[2], a3y, a2z, y3y, y2z), c3);
+      }
+    }
+    c1 = n1;
+    c2 = n2;
+    c3 = n3;
+    a1z = n1z;
+    a2z = n2z;
+    a3z = n3z;
+    a3x = n3x;
+    a3y = n3y;
+  }
 }
 
 __global__ void k_copy3_interior(double *__restrict__ u, double *__restrict__ v, double *__restrict__ w,
@@ -376,9 +433,15 @@ cudaError_t predictor(double *w1, double *w2, double *w3, const double *u, const
 
 cudaError_t convective(double *u, double *v, double *w, const double *w1, const double *w2, const double *w3,
                        Dims d, double tauh, int convectype, cudaStream_t st) {
-  if (convectype == 2)
-    DSG_COUNT k_convective<<<interior_grid(d, kBlk), kBlk, 0, st>>>(u, v, w, w1, w2, w3, d, 0.25 * tauh);
-  else
+  if (convectype == 2) {
+    // up to 16 planes per block (the first costs five sums more), fewer where
+    // the GPU would get less than about four blocks per SM
+    const unsigned bx = (d.nx - 2 + 31) / 32, by = (d.ny - 2 + kConvRows - 1) / kConvRows, nz = d.nz - 2;
+    int planes = 16;
+    while (planes > 2 && bx * by * ((nz + planes - 1) / planes) < 608) planes /= 2;
+    DSG_COUNT k_convective<<<dim3(bx, by, (nz + planes - 1) / planes), kConvThreads, 0, st>>>(u, v, w, w1, w2, w3, d,
+                                                                                             0.25 * tauh, planes);
+  } else
     DSG_COUNT k_copy3_interior<<<interior_grid(d, kBlk), kBlk, 0, st>>>(u, v, w, w1, w2, w3, d);
   return cudaGetLastError();
 }
