@@ -605,7 +605,7 @@ struct Planner {
         double **F = c->lv[c->ng];
         float **C = c->lv32[c->ng - 1];
         const Dims dc = c->level(c->ng - 1), df = c->fine();
-        t.add((int)i, dim3(cdiv(dc.nx, 32), cdiv(dc.ny, 4), dc.nz), 1,
+        t.add((int)i, dim3(cdiv(dc.nx, 32), cdiv(dc.ny, 4), cdiv(dc.nz, kAcfPlanes)), 1,
               AAcf64{C[A32], C[B32], C[C32], C[EI32], F[4], F[5], F[6], dc, df});
       }
       emit(out, K_ACF64, t, kDefaultShape, 0, 0, 0, 0, 0, -1);

@@ -7,83 +7,79 @@
 namespace dsg {
 namespace {
 
-// Curvature at interior cells: six face-normal magnitudes with transverse
-// 4-point means (+1e-50 inside the root), kappa = -(d1x-d2x+d1y-d2y+d1z-d2z).
-__global__ void k_curvature(double *__restrict__ kap, const double *__restrict__ f, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  if (i > d.nx - 1 || j > d.ny - 1) return;
-  const size_t q = d.ix(i, j, k);
+// Curvature and face forces at interior cells: six face-normal magnitudes with
+// transverse 4-point means (+1e-50 inside the root), kappa =
+// -(d1x-d2x+d1y-d2y+d1z-d2z); S = sigh * (difference of f) * kappa.  The
+// curvature is used by its own cell only, so it stays in a register.  Bound by
+// memory and, around the interface, the FP64 pipe: 256^3 367 us as two kernels,
+// each warp doing its own interface cells, 124 us now
+// (79 us of memory traffic); 128^3 61 and 26.
+template <int P>
+__global__ void __launch_bounds__(kBandThreads) k_csf(double *__restrict__ s11, double *__restrict__ s22,
+                                                      double *__restrict__ s33, const double *__restrict__ f, Dims d,
+                                                      double sigh) {
   const long sy = (long)d.sy(), sz = (long)d.sz();
+  auto force = [&](size_t q, double kq) {
+    const double fq = f[q], fx = f[q - 1], fy = f[q - sy], fz = f[q - sz];
+    if (same_bits(fx, fq) && same_bits(fy, fq) && same_bits(fz, fq)) {
+      // every difference is +0, so each force is (sigh * +0) * kappa, a zero
+      // whose sign is sign(sigh) xor sign(kappa) (kappa is finite), formed on
+      // the integer pipe
+      const double z = __longlong_as_double((__double_as_longlong(sigh) ^ __double_as_longlong(kq)) &
+                                            (long long)0x8000000000000000ULL);
+      s11[q] = z;
+      s22[q] = z;
+      s33[q] = z;
+      return;
+    }
+    s11[q] = sigh * (fq - fx) * kq;
+    s22[q] = sigh * (fq - fy) * kq;
+    s33[q] = sigh * (fq - fz) * kq;
+  };
 #define F(di, dj, dk) f[(long)q + (long)(di) + (long)(dj) * sy + (long)(dk) * sz]
-  // Uniform 19-point neighbourhood (bulk liquid or gas): every difference is
-  // +0, every d is 0/sqrt(1e-50) = +0 and kappa = -(+0) = -0 exactly.
-  const double f0 = F(0, 0, 0);
-#define EQ(di, dj, dk) same_bits(F(di, dj, dk), f0)
-  if (EQ(1, 0, 0) && EQ(-1, 0, 0) && EQ(0, 1, 0) && EQ(0, -1, 0) && EQ(0, 0, 1) && EQ(0, 0, -1) && EQ(1, 1, 0) &&
-      EQ(1, -1, 0) && EQ(-1, 1, 0) && EQ(-1, -1, 0) && EQ(1, 0, 1) && EQ(1, 0, -1) && EQ(-1, 0, 1) && EQ(-1, 0, -1) &&
-      EQ(0, 1, 1) && EQ(0, 1, -1) && EQ(0, -1, 1) && EQ(0, -1, -1)) {
-#undef EQ
-    kap[q] = -0.0;
-    return;
-  }
-  // d = difference / |normal| as difference * rsqrt(|normal|^2): one FP64
-  // reciprocal square root in place of a square root and a division on
-  // GB300's narrow FP64 pipe (results within a few ulps of the quotient)
-  double t0, t1, t2;
-  t0 = F(1, 0, 0) - F(0, 0, 0);
-  t1 = F(0, 1, 0) - F(0, -1, 0) + F(1, 1, 0) - F(1, -1, 0);
-  t2 = F(0, 0, 1) - F(0, 0, -1) + F(1, 0, 1) - F(1, 0, -1);
-  const double d1x = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 0, 0) - F(-1, 0, 0);
-  t1 = F(0, 1, 0) - F(0, -1, 0) + F(-1, 1, 0) - F(-1, -1, 0);
-  t2 = F(0, 0, 1) - F(0, 0, -1) + F(-1, 0, 1) - F(-1, 0, -1);
-  const double d2x = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 1, 0) - F(0, 0, 0);
-  t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, 1, 0) - F(-1, 1, 0);
-  t2 = F(0, 0, 1) - F(0, 0, -1) + F(0, 1, 1) - F(0, 1, -1);
-  const double d1y = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 0, 0) - F(0, -1, 0);
-  t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, -1, 0) - F(-1, -1, 0);
-  t2 = F(0, 0, 1) - F(0, 0, -1) + F(0, -1, 1) - F(0, -1, -1);
-  const double d2y = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 0, 1) - F(0, 0, 0);
-  t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, 0, 1) - F(-1, 0, 1);
-  t2 = F(0, 1, 0) - F(0, -1, 0) + F(0, 1, 1) - F(0, -1, 1);
-  const double d1z = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 0, 0) - F(0, 0, -1);
-  t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, 0, -1) - F(-1, 0, -1);
-  t2 = F(0, 1, 0) - F(0, -1, 0) + F(0, 1, -1) - F(0, -1, -1);
-  const double d2z = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+  const Flat<P> flat(f, d);
+  bulk_then_cells<P>(d, [&](int i, int j, int k, int p) {
+    // Uniform 19-point neighbourhood (bulk liquid or gas): every difference is
+    // +0, every d is 0/sqrt(1e-50) = +0 and kappa = -(+0) = -0 exactly.
+    if (!flat.uniform(p, false)) return false;
+    const double z = __longlong_as_double((__double_as_longlong(sigh) & (long long)0x8000000000000000ULL) ^
+                                          (long long)0x8000000000000000ULL);  // (sigh * +0) * -0
+    const size_t q = d.ix(i, j, k);
+    s11[q] = s22[q] = s33[q] = z;
+    return true;
+  }, [&](int i, int j, int k) {
+    const size_t q = d.ix(i, j, k);
+    // d = difference / |normal| as difference * rsqrt(|normal|^2): one FP64
+    // reciprocal square root in place of a square root and a division on
+    // GB300's narrow FP64 pipe (results within a few ulps of the quotient)
+    double t0, t1, t2;
+    t0 = F(1, 0, 0) - F(0, 0, 0);
+    t1 = F(0, 1, 0) - F(0, -1, 0) + F(1, 1, 0) - F(1, -1, 0);
+    t2 = F(0, 0, 1) - F(0, 0, -1) + F(1, 0, 1) - F(1, 0, -1);
+    const double d1x = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 0, 0) - F(-1, 0, 0);
+    t1 = F(0, 1, 0) - F(0, -1, 0) + F(-1, 1, 0) - F(-1, -1, 0);
+    t2 = F(0, 0, 1) - F(0, 0, -1) + F(-1, 0, 1) - F(-1, 0, -1);
+    const double d2x = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 1, 0) - F(0, 0, 0);
+    t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, 1, 0) - F(-1, 1, 0);
+    t2 = F(0, 0, 1) - F(0, 0, -1) + F(0, 1, 1) - F(0, 1, -1);
+    const double d1y = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 0, 0) - F(0, -1, 0);
+    t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, -1, 0) - F(-1, -1, 0);
+    t2 = F(0, 0, 1) - F(0, 0, -1) + F(0, -1, 1) - F(0, -1, -1);
+    const double d2y = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 0, 1) - F(0, 0, 0);
+    t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, 0, 1) - F(-1, 0, 1);
+    t2 = F(0, 1, 0) - F(0, -1, 0) + F(0, 1, 1) - F(0, -1, 1);
+    const double d1z = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 0, 0) - F(0, 0, -1);
+    t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, 0, -1) - F(-1, 0, -1);
+    t2 = F(0, 1, 0) - F(0, -1, 0) + F(0, 1, -1) - F(0, -1, -1);
+    const double d2z = t0 * rsqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    force(q, -(d1x - d2x + d1y - d2y + d1z - d2z));
+  });
 #undef F
-  kap[q] = -(d1x - d2x + d1y - d2y + d1z - d2z);
-}
-
-__global__ void k_csf_force(double *__restrict__ s11, double *__restrict__ s22, double *__restrict__ s33,
-                            const double *__restrict__ f, const double *__restrict__ kap, Dims d,
-                            double sigh) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  if (i > d.nx - 1 || j > d.ny - 1) return;
-  const size_t q = d.ix(i, j, k);
-  const double kq = kap[q], fq = f[q];
-  const double fx = f[q - 1], fy = f[q - d.sy()], fz = f[q - d.sz()];
-  if (same_bits(fx, fq) && same_bits(fy, fq) && same_bits(fz, fq)) {
-    // bulk cell: every difference is +0, so each force is (sigh * +0) * kappa,
-    // a zero whose sign is sign(sigh) xor sign(kappa) (kappa is finite),
-    // formed on the integer pipe
-    const double z = __longlong_as_double((__double_as_longlong(sigh) ^ __double_as_longlong(kq)) &
-                                          (long long)0x8000000000000000ULL);
-    s11[q] = z;
-    s22[q] = z;
-    s33[q] = z;
-    return;
-  }
-  s11[q] = sigh * (fq - fx) * kq;
-  s22[q] = sigh * (fq - fy) * kq;
-  s33[q] = sigh * (fq - fz) * kq;
 }
 
 // bc_tensor, its three ordered steps in one launch: every cell two steps write
@@ -149,7 +145,7 @@ cudaError_t bc_tensor(double *const S[6], Dims d, cudaStream_t st, int k0, int k
 // residual array, w33 = fine rhs array; ccf is the routine's local array.
 // scratch = false (inside a whole step, where the pressure phase overwrites
 // all three before reading them): the filtered field goes straight to ccf
-// and S11..S33 are not copied into w11..w33; w11 still holds the curvature.
+// and S11..S33 are not copied into w11..w33.
 cudaError_t csf(const double *ccc, double *w11, double *w22, double *w33, double *ccf, double *const S[6],
                 Dims d, double tau, double sigma, double h, cudaStream_t st, bool scratch) {
   const size_t bytes = d.count() * sizeof(double);
@@ -170,10 +166,7 @@ cudaError_t csf(const double *ccc, double *w11, double *w22, double *w33, double
     return cudaSuccess;
   }
   const double sigh = 0.5 * (tau * tau) * sigma / (h * h * h);
-  DSG_COUNT k_curvature<<<interior_grid(d, kBlk), kBlk, 0, st>>>(w11, ccf, d);
-  e = bc_out(w11, d, st);
-  if (e != cudaSuccess) return e;
-  DSG_COUNT k_csf_force<<<interior_grid(d, kBlk), kBlk, 0, st>>>(S[0], S[1], S[2], ccf, w11, d, sigh);
+  DSG_BAND(k_csf, d, st, S[0], S[1], S[2], ccf, d, sigh);
   if (scratch) {
     if ((e = cudaMemcpyAsync(w11, S[0], bytes, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
     if ((e = cudaMemcpyAsync(w22, S[1], bytes, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;

@@ -171,7 +171,7 @@ __global__ void k_node_flags(unsigned char *__restrict__ flags, const float *__r
   bool same = a[q - 1] == f;
 #pragma unroll
   for (int t = 0; t < 8; t++)
-    same = same && a[q + t] == f && b[q + t] == f && b[q + t - sy] == f && c[q + t] == f && c[q + t - sz] == f && ei[q + t] == e;
+    same &= (a[q + t] == f) & (b[q + t] == f) & (b[q + t - sy] == f) & (c[q + t] == f) & (c[q + t - sz] == f) & (ei[q + t] == e);
   flags[(unsigned)m + (unsigned)n8 * ((unsigned)(j - 2) + (unsigned)(d.ny - 2) * (unsigned)(k - 2))] = !same ? 0 : liquid ? 2 : 1;
 }
 
@@ -590,7 +590,7 @@ cudaError_t acfromac64to32(float *a, float *b, float *c, float *ei, const double
                            const double *c2, Dims dc, cudaStream_t st) {
   const Dims df{2 * dc.nx - 2, 2 * dc.ny - 2, 2 * dc.nz - 2};
   const dim3 grid((unsigned)((dc.nx + kBlk.x - 1) / kBlk.x), (unsigned)((dc.ny + kBlk.y - 1) / kBlk.y),
-                  (unsigned)dc.nz);
+                  (unsigned)((dc.nz + kAcfPlanes - 1) / kAcfPlanes));
   DSG_COUNT k_acfromac64to32<<<grid, kBlk, 0, st>>>(a, b, c, ei, a2, b2, c2, dc, df);
   return cudaGetLastError();
 }

@@ -161,7 +161,7 @@ __device__ __forceinline__ void b_flags(const uint3 B, const uint3 G, unsigned c
     const unsigned row = t / ns, s = t - row * ns, k = row / ny2, j = row - k * ny2;
     const unsigned sy = ns, sz = ns * (unsigned)d.ny, q = s + sy * (j + 1) + sz * (k + 1);
     const unsigned char c = codes[q];
-    flags[t] = codes[q - sy] == c && codes[q + sy] == c && codes[q - sz] == c && codes[q + sz] == c ? c : 0;
+    flags[t] = (codes[q - sy] == c) & (codes[q + sy] == c) & (codes[q - sz] == c) & (codes[q + sz] == c) ? c : 0;
   }
 }
 
@@ -797,26 +797,62 @@ __device__ __forceinline__ void b_correct64(const uint3 B, const uint3 G, double
 }
 
 // Coarse FP32 coefficients (acfromac) straight from the FP64 fine ones.
+// FP64 fine coefficients to an FP32 coarse level, kAcfPlanes planes per block.
+// Where all 24 fine faces of a coarse cell are the same (bulk gas or liquid),
+// their means are that value, exactly, and ei is formed once for a run of such
+// cells: the FP64 pipe, on which it ran into the momentum kernels beside it,
+// has little left to do (256^3: 177 us, 64 now, what
+// its memory traffic takes).
+constexpr int kAcfPlanes = 2;
 __device__ __forceinline__ void b_acfromac64to32(const uint3 B, const uint3 G, float *__restrict__ a, float *__restrict__ b, float *__restrict__ c,
                                  float *__restrict__ ei, const double *__restrict__ a2,
                                  const double *__restrict__ b2, const double *__restrict__ c2, Dims dc, Dims df) {
   const int i = B.x * blockDim.x + threadIdx.x + 1;
   const int j = B.y * blockDim.y + threadIdx.y + 1;
-  const int k = B.z + 1;
   if (i > dc.nx || j > dc.ny) return;
-  const bool ii = i >= 2 && i <= dc.nx - 1, ji = j >= 2 && j <= dc.ny - 1, ki = k >= 2 && k <= dc.nz - 1;
-  const size_t q = dc.ix(i, j, k);
 #define FA(i, j, k) (0.25 * (a2[df.ix(2 * (i) - 1, 2 * (j) - 1, 2 * (k) - 1)] + a2[df.ix(2 * (i) - 1, 2 * (j) - 2, 2 * (k) - 1)] + \
                              a2[df.ix(2 * (i) - 1, 2 * (j) - 1, 2 * (k) - 2)] + a2[df.ix(2 * (i) - 1, 2 * (j) - 2, 2 * (k) - 2)]))
 #define FB(i, j, k) (0.25 * (b2[df.ix(2 * (i) - 1, 2 * (j) - 1, 2 * (k) - 1)] + b2[df.ix(2 * (i) - 2, 2 * (j) - 1, 2 * (k) - 1)] + \
                              b2[df.ix(2 * (i) - 1, 2 * (j) - 1, 2 * (k) - 2)] + b2[df.ix(2 * (i) - 2, 2 * (j) - 1, 2 * (k) - 2)]))
 #define FC(i, j, k) (0.25 * (c2[df.ix(2 * (i) - 1, 2 * (j) - 1, 2 * (k) - 1)] + c2[df.ix(2 * (i) - 2, 2 * (j) - 1, 2 * (k) - 1)] + \
                              c2[df.ix(2 * (i) - 1, 2 * (j) - 2, 2 * (k) - 1)] + c2[df.ix(2 * (i) - 2, 2 * (j) - 2, 2 * (k) - 1)]))
-  double va = 0.0, vb = 0.0, vc = 0.0;
-  if (i <= dc.nx - 1 && ji && ki) { va = FA(i, j, k); a[q] = (float)va; }
-  if (j <= dc.ny - 1 && ii && ki) { vb = FB(i, j, k); b[q] = (float)vb; }
-  if (k <= dc.nz - 1 && ii && ji) { vc = FC(i, j, k); c[q] = (float)vc; }
-  if (ii && ji && ki) ei[q] = (float)(1.0 / (va + FA(i - 1, j, k) + vb + FB(i, j - 1, k) + vc + FC(i, j, k - 1)));
+  // coefficient and ei of the last cell in a uniform neighbourhood
+  double v = 0.0;
+  float vf = 0.f, ef = 0.f;
+  bool some = false;
+  const size_t fy = df.sy(), fz = df.sz();
+  for (int k = kAcfPlanes * (int)B.z + 1; k <= kAcfPlanes * (int)(B.z + 1) && k <= dc.nz; k++) {
+    const bool ii = i >= 2 && i <= dc.nx - 1, ji = j >= 2 && j <= dc.ny - 1, ki = k >= 2 && k <= dc.nz - 1;
+    const size_t q = dc.ix(i, j, k);
+    if (ii && ji && ki) {
+      // its 24 fine faces; node f is the first of the cell's eight
+      const size_t f = df.ix(2 * i - 2, 2 * j - 2, 2 * k - 2);
+      const double x = a2[f];
+      bool same = true;
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        const size_t yz = f + (m & 1 ? fy : 0) + (m & 2 ? fz : 0), xz = f + (m & 1) + (m & 2 ? fz : 0), xy = f + (m & 1) + (m & 2 ? fy : 0);
+        same &= same_bits(a2[yz + 1], x) & same_bits(a2[yz - 1], x) & same_bits(b2[xz + fy], x) & same_bits(b2[xz - fy], x) &
+                same_bits(c2[xy + fz], x) & same_bits(c2[xy - fz], x);
+      }
+      if (same) {
+        if (!some || !same_bits(x, v)) {
+          some = true;
+          v = x;
+          vf = (float)x;
+          ef = (float)(1.0 / (x + x + x + x + x + x));
+        }
+        a[q] = b[q] = c[q] = vf;
+        ei[q] = ef;
+        continue;
+      }
+    }
+    double va = 0.0, vb = 0.0, vc = 0.0;
+    if (i <= dc.nx - 1 && ji && ki) { va = FA(i, j, k); a[q] = (float)va; }
+    if (j <= dc.ny - 1 && ii && ki) { vb = FB(i, j, k); b[q] = (float)vb; }
+    if (k <= dc.nz - 1 && ii && ji) { vc = FC(i, j, k); c[q] = (float)vc; }
+    if (ii && ji && ki) ei[q] = (float)(1.0 / (va + FA(i - 1, j, k) + vb + FB(i, j - 1, k) + vc + FC(i, j, k - 1)));
+  }
 #undef FA
 #undef FB
 #undef FC

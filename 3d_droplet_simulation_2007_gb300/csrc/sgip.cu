@@ -204,114 +204,153 @@ struct Heights {
 
 // Heights of every interior cell.  The first failing cell (a STOP of the
 // reference) is recorded as (code << 48 | linear index) in *err.
-__global__ void k_calch3d(Heights H, const double *__restrict__ cc, Dims d, unsigned long long *err) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  if (i > d.nx - 1 || j > d.ny - 1) return;
-  const size_t q = d.ix(i, j, k);
-  double h[6];
-  const int rc = h3d_cell(cc, q, (long)d.sy(), (long)d.sz(), h);
-  if (rc) {
-    atomicCAS(err, 0ull, ((unsigned long long)rc << 48) | (unsigned long long)q);
-    return;
-  }
+//
+// A cell in a uniform neighbourhood of 0 or 1 has a zero normal, the third case
+// and constant heights; the others, around the interface, are some 300 FP64
+// operations each.  96 x 48 x 96 cells, every cell computed: 343 us; now 54.
+__global__ void __launch_bounds__(kBandThreads) k_calch3d(Heights H, const double *__restrict__ cc, Dims d,
+                                                          unsigned long long *err) {
+  const long sy = (long)d.sy(), sz = (long)d.sz();
+  bulk_then_cells<1>(d, [&](int i, int j, int k, int) {
+    const size_t q = d.ix(i, j, k);
+    const double c0 = cc[q];
+    const bool gas = is_zero_bits(c0);
+    bool uni = gas || is_one_bits(c0);
 #pragma unroll
-  for (int m = 0; m < 6; m++) H.p[m][q] = h[m];
+    for (int dk = -1; dk <= 1; dk++)
+#pragma unroll
+      for (int dj = -1; dj <= 1; dj++)
+#pragma unroll
+        for (int di = -1; di <= 1; di++) uni &= same_bits(cc[(long)q + di + dj * sy + dk * sz], c0);
+    if (!uni) return false;
+    // h1 = h2 = 0 (liquid: 1), h3 = {1, 0} ({0, 1}), of which x, y and z take
+    // h1, h2 and h3, min and max exchanged in gas
+    const double v = gas ? 0.0 : 1.0;
+    H.p[0][q] = H.p[1][q] = H.p[2][q] = H.p[3][q] = v;
+    H.p[4][q] = 1.0;
+    H.p[5][q] = 0.0;
+    return true;
+  }, [&](int i, int j, int k) {
+    const size_t q = d.ix(i, j, k);
+    double h[6];
+    const int rc = h3d_cell(cc, q, sy, sz, h);
+    if (rc) {
+      atomicCAS(err, 0ull, ((unsigned long long)rc << 48) | (unsigned long long)q);
+      return;
+    }
+#pragma unroll
+    for (int m = 0; m < 6; m++) H.p[m][q] = h[m];
+  });
 }
 
 // SGIP's curvature: csf's face-normal formula with the transverse differences
 // summed in SGIP's own order (main.f:2880-2913).
-__global__ void k_sgip_curvature(double *__restrict__ kap, const double *__restrict__ f, Dims d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  if (i > d.nx - 1 || j > d.ny - 1) return;
-  const size_t q = d.ix(i, j, k);
+__global__ void __launch_bounds__(kBandThreads) k_sgip_curvature(double *__restrict__ kap, const double *__restrict__ f, Dims d) {
   const long sy = (long)d.sy(), sz = (long)d.sz();
 #define F(di, dj, dk) f[(long)q + (long)(di) + (long)(dj) * sy + (long)(dk) * sz]
-  // uniform 19-point neighbourhood: every difference +0, kappa = -0 exactly
-  const double f0 = F(0, 0, 0);
+  bulk_then_cells<1>(d, [&](int i, int j, int k, int) {
+    const size_t q = d.ix(i, j, k);
+    // uniform 19-point neighbourhood: every difference +0, kappa = -0 exactly
+    const double f0 = F(0, 0, 0);
 #define EQ(di, dj, dk) same_bits(F(di, dj, dk), f0)
-  if (EQ(1, 0, 0) && EQ(-1, 0, 0) && EQ(0, 1, 0) && EQ(0, -1, 0) && EQ(0, 0, 1) && EQ(0, 0, -1) && EQ(1, 1, 0) &&
-      EQ(1, -1, 0) && EQ(-1, 1, 0) && EQ(-1, -1, 0) && EQ(1, 0, 1) && EQ(1, 0, -1) && EQ(-1, 0, 1) && EQ(-1, 0, -1) &&
-      EQ(0, 1, 1) && EQ(0, 1, -1) && EQ(0, -1, 1) && EQ(0, -1, -1)) {
+    if (!(EQ(1, 0, 0) & EQ(-1, 0, 0) & EQ(0, 1, 0) & EQ(0, -1, 0) & EQ(0, 0, 1) & EQ(0, 0, -1) & EQ(1, 1, 0) &
+          EQ(1, -1, 0) & EQ(-1, 1, 0) & EQ(-1, -1, 0) & EQ(1, 0, 1) & EQ(1, 0, -1) & EQ(-1, 0, 1) &
+          EQ(-1, 0, -1) & EQ(0, 1, 1) & EQ(0, 1, -1) & EQ(0, -1, 1) & EQ(0, -1, -1)))
+      return false;
 #undef EQ
     kap[q] = -0.0;
-    return;
-  }
-  double t0, t1, t2;
-  t0 = F(1, 0, 0) - F(0, 0, 0);
-  t1 = F(0, 1, 0) - F(0, -1, 0) + F(1, 1, 0) - F(1, -1, 0);
-  t2 = F(0, 0, 1) - F(0, 0, -1) + F(1, 0, 1) - F(1, 0, -1);
-  const double nxu = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 0, 0) - F(-1, 0, 0);
-  t1 = F(-1, 1, 0) - F(-1, -1, 0) + F(0, 1, 0) - F(0, -1, 0);
-  t2 = F(-1, 0, 1) - F(-1, 0, -1) + F(0, 0, 1) - F(0, 0, -1);
-  const double nxd = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 1, 0) - F(0, 0, 0);
-  t1 = F(1, 1, 0) - F(-1, 1, 0) + F(1, 0, 0) - F(-1, 0, 0);
-  t2 = F(0, 1, 1) - F(0, 1, -1) + F(0, 0, 1) - F(0, 0, -1);
-  const double nyu = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 0, 0) - F(0, -1, 0);
-  t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, -1, 0) - F(-1, -1, 0);
-  t2 = F(0, 0, 1) - F(0, 0, -1) + F(0, -1, 1) - F(0, -1, -1);
-  const double nyd = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 0, 1) - F(0, 0, 0);
-  t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, 0, 1) - F(-1, 0, 1);
-  t2 = F(0, 1, 0) - F(0, -1, 0) + F(0, 1, 1) - F(0, -1, 1);
-  const double nzu = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  t0 = F(0, 0, 0) - F(0, 0, -1);
-  t1 = F(1, 0, -1) - F(-1, 0, -1) + F(1, 0, 0) - F(-1, 0, 0);
-  t2 = F(0, 1, -1) - F(0, -1, -1) + F(0, 1, 0) - F(0, -1, 0);
-  const double nzd = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
-  const double d1x = (F(1, 0, 0) - F(0, 0, 0)) / nxu;
-  const double d2x = (F(0, 0, 0) - F(-1, 0, 0)) / nxd;
-  const double d1y = (F(0, 1, 0) - F(0, 0, 0)) / nyu;
-  const double d2y = (F(0, 0, 0) - F(0, -1, 0)) / nyd;
-  const double d1z = (F(0, 0, 1) - F(0, 0, 0)) / nzu;
-  const double d2z = (F(0, 0, 0) - F(0, 0, -1)) / nzd;
+    return true;
+  }, [&](int i, int j, int k) {
+    const size_t q = d.ix(i, j, k);
+    double t0, t1, t2;
+    t0 = F(1, 0, 0) - F(0, 0, 0);
+    t1 = F(0, 1, 0) - F(0, -1, 0) + F(1, 1, 0) - F(1, -1, 0);
+    t2 = F(0, 0, 1) - F(0, 0, -1) + F(1, 0, 1) - F(1, 0, -1);
+    const double nxu = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 0, 0) - F(-1, 0, 0);
+    t1 = F(-1, 1, 0) - F(-1, -1, 0) + F(0, 1, 0) - F(0, -1, 0);
+    t2 = F(-1, 0, 1) - F(-1, 0, -1) + F(0, 0, 1) - F(0, 0, -1);
+    const double nxd = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 1, 0) - F(0, 0, 0);
+    t1 = F(1, 1, 0) - F(-1, 1, 0) + F(1, 0, 0) - F(-1, 0, 0);
+    t2 = F(0, 1, 1) - F(0, 1, -1) + F(0, 0, 1) - F(0, 0, -1);
+    const double nyu = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 0, 0) - F(0, -1, 0);
+    t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, -1, 0) - F(-1, -1, 0);
+    t2 = F(0, 0, 1) - F(0, 0, -1) + F(0, -1, 1) - F(0, -1, -1);
+    const double nyd = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 0, 1) - F(0, 0, 0);
+    t1 = F(1, 0, 0) - F(-1, 0, 0) + F(1, 0, 1) - F(-1, 0, 1);
+    t2 = F(0, 1, 0) - F(0, -1, 0) + F(0, 1, 1) - F(0, -1, 1);
+    const double nzu = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    t0 = F(0, 0, 0) - F(0, 0, -1);
+    t1 = F(1, 0, -1) - F(-1, 0, -1) + F(1, 0, 0) - F(-1, 0, 0);
+    t2 = F(0, 1, -1) - F(0, -1, -1) + F(0, 1, 0) - F(0, -1, 0);
+    const double nzd = sqrt(t0 * t0 + 0.0625 * (t1 * t1) + 0.0625 * (t2 * t2) + 1.e-50);
+    const double d1x = (F(1, 0, 0) - F(0, 0, 0)) / nxu;
+    const double d2x = (F(0, 0, 0) - F(-1, 0, 0)) / nxd;
+    const double d1y = (F(0, 1, 0) - F(0, 0, 0)) / nyu;
+    const double d2y = (F(0, 0, 0) - F(0, -1, 0)) / nyd;
+    const double d1z = (F(0, 0, 1) - F(0, 0, 0)) / nzu;
+    const double d2z = (F(0, 0, 0) - F(0, 0, -1)) / nzd;
+    kap[q] = -(d1x - d2x + d1y - d2y + d1z - d2z);
+  });
 #undef F
-  kap[q] = -(d1x - d2x + d1y - d2y + d1z - d2z);
 }
 
 // SGIP's face forces: curvature x filtered-fraction difference x the jump of
 // the mean interface height between the cell and its lower neighbour; on the
 // wall plane j = 2 the contact-angle model (angle from the contact-line
 // speed, sin/cos of degrees as dsind/dcosd).
-__global__ void k_sgip_force(double *__restrict__ s11, double *__restrict__ s22, double *__restrict__ s33,
-                             const double *__restrict__ f, const double *__restrict__ kap, Heights H,
-                             const double *__restrict__ u, const double *__restrict__ w, Dims d, double sigh) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  if (i > d.nx - 1 || j > d.ny - 1) return;
-  const size_t q = d.ix(i, j, k);
+//
+// Where the fraction differences are +0 and the curvatures -0 (away from the
+// interface), each force is a zero with the sign of -sigh.
+__global__ void __launch_bounds__(kBandThreads)
+    k_sgip_force(double *__restrict__ s11, double *__restrict__ s22, double *__restrict__ s33,
+                 const double *__restrict__ f, const double *__restrict__ kap, Heights H,
+                 const double *__restrict__ u, const double *__restrict__ w, Dims d, double sigh) {
   const size_t sy = d.sy(), sz = d.sz();
-  const double Lx = (H.p[1][q] + H.p[0][q]) / 2.0, Lxd = (H.p[1][q - 1] + H.p[0][q - 1]) / 2.0;
-  const double Ly = (H.p[3][q] + H.p[2][q]) / 2.0, Lyd = (H.p[3][q - sy] + H.p[2][q - sy]) / 2.0;
-  const double Lz = (H.p[5][q] + H.p[4][q]) / 2.0, Lzd = (H.p[5][q - sz] + H.p[4][q - sz]) / 2.0;
-  if (j != 2) {
-    s11[q] = sigh * (kap[q] + kap[q - 1]) * (f[q + 1] - f[q - 1]) * fabs(Lx - Lxd) / 2.0;
-    s22[q] = sigh * (kap[q] + kap[q - sy]) * (f[q + sy] - f[q - sy]) * fabs(Ly - Lyd) / 2.0;
-    s33[q] = sigh * (kap[q] + kap[q - sz]) * (f[q + sz] - f[q - sz]) * fabs(Lz - Lzd) / 2.0;
-    return;
-  }
-  const double mx = f[q + 1] - f[q - 1], mz = f[q + sz] - f[q - sz];
-  const double mmx = mx / sqrt(mz * mz + mx * mx + 1.e-50), mmz = mz / sqrt(mz * mz + mx * mx + 1.e-50);
-  double normv = mmx * u[q] + mmz * w[q];
-  normv = -normv;
-  double theta;
-  if (fabs(normv) > (double)0.1f)
-    theta = normv > 0 ? 115.0 : 45.0;
-  else
-    theta = 350.0 * normv + 80.0;
-  const double my = f[q + sy] - f[q - sy];
-  const double rad = theta * (3.14159265358979323846 / 180.0);
-  const double sind = sin(rad), mmy = cos(rad);
-  s11[q] = sigh * (kap[q] + kap[q - 1]) * mx * sind / 2.0;
-  s22[q] = sigh * (kap[q] + kap[q - sy]) * mmy * sqrt(mz * mz + mx * mx + my * my) * -1.0;
-  s33[q] = sigh * (kap[q] + kap[q - sz]) * mz * sind / 2.0;
+  bulk_then_cells<1>(d, [&](int i, int j, int k, int) {
+    const size_t q = d.ix(i, j, k);
+    auto none = [&](size_t low) { return same_bits(kap[low], -0.0); };
+    auto finite = [&](const double *p, size_t low) { return finite_bits(p[q]) & finite_bits(p[q - low]); };
+    const bool zero = (j != 2) & finite_bits(sigh) & none(q) & none(q - 1) & none(q - sy) & none(q - sz) &
+                      same_bits(f[q + 1], f[q - 1]) & same_bits(f[q + sy], f[q - sy]) & same_bits(f[q + sz], f[q - sz]) &
+                      finite(H.p[0], 1) & finite(H.p[1], 1) & finite(H.p[2], sy) & finite(H.p[3], sy) &
+                      finite(H.p[4], sz) & finite(H.p[5], sz) & finite_bits(f[q + 1]) & finite_bits(f[q + sy]) &
+                      finite_bits(f[q + sz]);
+    if (!zero) return false;
+    const double z = __longlong_as_double((__double_as_longlong(sigh) & (long long)0x8000000000000000ULL) ^
+                                          (long long)0x8000000000000000ULL);
+    s11[q] = s22[q] = s33[q] = z;
+    return true;
+  }, [&](int i, int j, int k) {
+    const size_t q = d.ix(i, j, k);
+    const double Lx = (H.p[1][q] + H.p[0][q]) / 2.0, Lxd = (H.p[1][q - 1] + H.p[0][q - 1]) / 2.0;
+    const double Ly = (H.p[3][q] + H.p[2][q]) / 2.0, Lyd = (H.p[3][q - sy] + H.p[2][q - sy]) / 2.0;
+    const double Lz = (H.p[5][q] + H.p[4][q]) / 2.0, Lzd = (H.p[5][q - sz] + H.p[4][q - sz]) / 2.0;
+    if (j != 2) {
+      s11[q] = sigh * (kap[q] + kap[q - 1]) * (f[q + 1] - f[q - 1]) * fabs(Lx - Lxd) / 2.0;
+      s22[q] = sigh * (kap[q] + kap[q - sy]) * (f[q + sy] - f[q - sy]) * fabs(Ly - Lyd) / 2.0;
+      s33[q] = sigh * (kap[q] + kap[q - sz]) * (f[q + sz] - f[q - sz]) * fabs(Lz - Lzd) / 2.0;
+      return;
+    }
+    const double mx = f[q + 1] - f[q - 1], mz = f[q + sz] - f[q - sz];
+    const double mmx = mx / sqrt(mz * mz + mx * mx + 1.e-50), mmz = mz / sqrt(mz * mz + mx * mx + 1.e-50);
+    double normv = mmx * u[q] + mmz * w[q];
+    normv = -normv;
+    double theta;
+    if (fabs(normv) > (double)0.1f)
+      theta = normv > 0 ? 115.0 : 45.0;
+    else
+      theta = 350.0 * normv + 80.0;
+    const double my = f[q + sy] - f[q - sy];
+    const double rad = theta * (3.14159265358979323846 / 180.0);
+    const double sind = sin(rad), mmy = cos(rad);
+    s11[q] = sigh * (kap[q] + kap[q - 1]) * mx * sind / 2.0;
+    s22[q] = sigh * (kap[q] + kap[q - sy]) * mmy * sqrt(mz * mz + mx * mx + my * my) * -1.0;
+    s33[q] = sigh * (kap[q] + kap[q - sz]) * mz * sind / 2.0;
+  });
 }
 
 // SGIP2's face forces (main.f:3124-3140): central differences of the mean
@@ -340,7 +379,7 @@ const dim3 kBlk(32, 4, 1);
 cudaError_t calch3d(double *const H[6], const double *cc, Dims d, unsigned long long *err, cudaStream_t st) {
   Heights h;
   for (int m = 0; m < 6; m++) h.p[m] = H[m];
-  DSG_COUNT k_calch3d<<<interior_grid(d, kBlk), kBlk, 0, st>>>(h, cc, d, err);
+  DSG_COUNT k_calch3d<<<band_grid(d, 1), dim3(32, 8), 0, st>>>(h, cc, d, err);
   return cudaGetLastError();
 }
 
@@ -362,7 +401,7 @@ cudaError_t sgip2(const double *ccc, double *w11, double *w22, double *w33, doub
     return cudaSuccess;
   }
   const double sigh = 0.5 * tau * sigma / (h * h);
-  DSG_COUNT k_sgip_curvature<<<interior_grid(d, kBlk), kBlk, 0, st>>>(w11, ccf, d);
+  DSG_COUNT k_sgip_curvature<<<band_grid(d, 1), dim3(32, 8), 0, st>>>(w11, ccf, d);
   if ((e = bc_out(w11, d, st)) != cudaSuccess) return e;
   Heights hh;
   for (int m = 0; m < 6; m++) hh.p[m] = H[m];
@@ -388,11 +427,11 @@ cudaError_t sgip(const double *ccc, double *w11, double *w22, double *w33, doubl
     return cudaSuccess;
   }
   const double sigh = 0.5 * (tau * tau) * sigma / (h * h * h);
-  DSG_COUNT k_sgip_curvature<<<interior_grid(d, kBlk), kBlk, 0, st>>>(w11, ccf, d);
+  DSG_COUNT k_sgip_curvature<<<band_grid(d, 1), dim3(32, 8), 0, st>>>(w11, ccf, d);
   if ((e = bc_out(w11, d, st)) != cudaSuccess) return e;
   Heights hh;
   for (int m = 0; m < 6; m++) hh.p[m] = H[m];
-  DSG_COUNT k_sgip_force<<<interior_grid(d, kBlk), kBlk, 0, st>>>(S[0], S[1], S[2], ccf, w11, hh, u, w, d, sigh);
+  DSG_COUNT k_sgip_force<<<band_grid(d, 1), dim3(32, 8), 0, st>>>(S[0], S[1], S[2], ccf, w11, hh, u, w, d, sigh);
   for (int m = 0; m < 3; m++)
     if ((e = bc_out(S[m], d, st)) != cudaSuccess) return e;
   if ((e = cudaMemcpyAsync(w11, S[0], bytes, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
