@@ -126,6 +126,25 @@ inline bool fp64_fma(const dsg_ctx *ctx) {
   return ctx->cfg.mode == DSG_MODE_TOL_FP64 && ctx->cfg.fp64_exact == 0;
 }
 
+template <class A>
+bool phases(const dsg_ctx *ctx, const A &level, int l);
+
+// Whether level l's FP64 sweeps share products (sweeps pass by pass in the
+// reference's rounding); they and the flags lie in the level's FP32 arrays,
+// which only the mixed modes use.
+bool products(const dsg_ctx *ctx, int l, dsg::Products *P) {
+  if (ctx->cfg.mode == DSG_MODE_TOL_MIXED || ctx->cfg.mode == DSG_MODE_LEARNED || fp64_fma(ctx)) return false;
+  if (l <= ctx->tail64_top || phases(ctx, ctx->gr64[l], l)) return false;
+  P->v = (double *)ctx->lv32[l][0];
+  P->flags = (unsigned char *)ctx->lv32[l][2];
+  const double r1 = 0.5 * (ctx->s.rho1 - ctx->s.rho2), r2 = ctx->s.rho2;
+  P->k = 1.0 / (r1 * (0.0 + 0.0) + r2);
+  P->k1 = 1.0 / (r1 * (1.0 + 1.0) + r2);
+  P->e = 1.0 / (P->k + P->k + P->k + P->k + P->k + P->k);
+  P->e1 = 1.0 / (P->k1 + P->k1 + P->k1 + P->k1 + P->k1 + P->k1);
+  return true;
+}
+
 // relax_n on level jj; the finest level is timed with an event pair when the
 // live profile is on.
 cudaError_t relax_level(dsg_ctx *ctx, int n, int jj, double ls) {
@@ -144,8 +163,10 @@ cudaError_t relax_level(dsg_ctx *ctx, int n, int jj, double ls) {
     cudaError_t r = cudaEventRecord(ctx->prof_ev[ctx->prof_used], ctx->stream);
     if (r != cudaSuccess) return r;
   }
-  cudaError_t e =
-      dsg::relax_n(n, L[1], ls, L[3], L[4], L[5], L[6], L[7], d, ctx->cfg.omega, ctx->stream, fp64_fma(ctx));
+  dsg::Products P;
+  const bool shared = products(ctx, jj, &P);
+  cudaError_t e = dsg::relax_n(n, L[1], ls, L[3], L[4], L[5], L[6], L[7], d, ctx->cfg.omega, ctx->stream,
+                               fp64_fma(ctx), shared ? &P : nullptr);
   if (timed) {
     cudaError_t r = cudaEventRecord(ctx->prof_ev[ctx->prof_used + 1], ctx->stream);
     if (r != cudaSuccess) return r;
@@ -879,6 +900,11 @@ int mglin(dsg_ctx *ctx, dsg_mg_stats *stats) {
     DSG_CK(ctx, dsg::rstrct(ctx->lv[g][3], ctx->lv[g + 1][3], dc, st));
     DSG_CK(ctx, dsg::acfromac(ctx->lv[g][4], ctx->lv[g][5], ctx->lv[g][6], ctx->lv[g][7], ctx->lv[g + 1][4],
                               ctx->lv[g + 1][5], ctx->lv[g + 1][6], dc, st));
+  }
+  for (int l = 2; l <= ng; l++) {
+    dsg::Products P;
+    double **L = ctx->lv[l];
+    if (products(ctx, l, &P)) DSG_CK(ctx, dsg::bulk_flags(P, L[4], L[5], L[6], L[7], ctx->level(l), st));
   }
   if (ctx->tail64_top >= 1) {
     int rc = coarse64(ctx, true);

@@ -205,9 +205,17 @@ cudaError_t relax(double *u, double lengthsize, const double *rhs, const double 
 // fma = true: the fused multiply-add form of the FP64 sweep and residual
 // (fewer FP64 operations, results within ulps of the reference order);
 // fma = false: the reference's operation order, bit-identical to the oracle.
+// P: the coefficient times u in gas, shared between neighbours (k_relax_colour)
+struct Products {
+  double *v;             // product per node, scratch
+  unsigned char *flags;  // per warp of a colour pass (bulk_flags)
+  double k, e, k1, e1;   // face coefficient and ei of gas, of liquid
+};
 cudaError_t relax_n(int n, double *u, double lengthsize, const double *rhs, const double *a,
                     const double *b, const double *c, const double *ei, Dims d, double omega,
-                    cudaStream_t st, bool fma = false);
+                    cudaStream_t st, bool fma = false, const Products *P = nullptr);
+cudaError_t bulk_flags(const Products &P, const double *a, const double *b, const double *c, const double *ei, Dims d,
+                       cudaStream_t st);
 cudaError_t resid(double lengthsize, double *res, const double *u, const double *rhs, const double *a,
                   const double *b, const double *c, Dims d, cudaStream_t st, bool fma = false);
 // resid (virtual ghosts) and rstrct in one pass, the coarse correction zeroed
