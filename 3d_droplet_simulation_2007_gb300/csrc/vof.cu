@@ -19,84 +19,97 @@ namespace {
 // executes every branch that one of its lanes takes, at 16 cycles of the SM's
 // FP64 pipe per instruction.  The branches below therefore only pick operands;
 // the divisions, square roots and acos/cos that several of them share stand
-// behind the branches and are executed once (same operations per cell;
-// 64^3: 36 -> 30 us).
+// behind the branches and are executed once (same operations per cell).
 
 // AL3D: plane constant alpha of m1 x1 + m2 x2 + m3 x3 = alpha cutting volume cc
-// from the unit cube (m1+m2+m3 = 1, all >= 0).  Scardovelli-Zaleski analytic
-// inversion with five regimes.
-__device__ double al3d(double b1, double b2, double b3, double cc) {
-  double m1 = dmin1(b1, b2), m3 = dmax1(b1, b2), m2 = b3, tmp;
-  if (m2 < m1) {
+// from the unit cube (m1+m2+m3 = 1, 0 <= m1 <= m2 <= m3).  Scardovelli-Zaleski
+// analytic inversion with five regimes; here its parts, as flux_cells deals
+// them out.
+struct Ordered {
+  double m1, m2, m3, m12;
+};
+// Comparisons on the integer pipe, where one of the values is >= 0: then the bit
+// patterns order like the values (an FP64 comparison costs as much as an FMA).
+__device__ __forceinline__ bool less_bits(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+__device__ __forceinline__ double min_bits(double a, double b) { return less_bits(b, a) ? b : a; }
+__device__ __forceinline__ double max_bits(double a, double b) { return less_bits(a, b) ? b : a; }
+// x < 0, x == 0 (either sign), max(0, x), min(0, x); a NaN stays one
+__device__ __forceinline__ bool negative(double x) {
+  return __double_as_longlong(x) < 0 && (__double_as_longlong(x) << 1) != 0;
+}
+__device__ __forceinline__ bool zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool is_nan(double x) {
+  return (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFLL) > 0x7FF0000000000000LL;
+}
+__device__ __forceinline__ double max0(double x) { return positive_bits(x) || is_nan(x) ? x : 0.0; }
+__device__ __forceinline__ double min0(double x) { return negative(x) || is_nan(x) ? x : 0.0; }
+__device__ __forceinline__ Ordered ordered(double b1, double b2, double b3) {
+  double m1 = min_bits(b1, b2), m3 = max_bits(b1, b2), m2 = b3, tmp;
+  if (less_bits(m2, m1)) {
     tmp = m1; m1 = m2; m2 = tmp;
-  } else if (m2 > m3) {
+  } else if (less_bits(m3, m2)) {
     tmp = m3; m3 = m2; m2 = tmp;
   }
-  const double m12 = m1 + m2;
-  const double pr = dmax1(6.0 * m1 * m2 * m3, 1.0e-50);
-  const double V1 = m1 * m1 * m1 / pr;
-  const double V2 = V1 + 0.5 * (m2 - m1) / m3;
-  const bool five = m3 < m12;  // regimes 3 and 5 up to m3, else 3 and 4 up to m12
-  const double mm = five ? m3 : m12;
-  double num = 0.5 * mm, den = m3;
+  return {m1, m2, m3, m1 + m2};
+}
+__device__ __forceinline__ double al3d_pr(const Ordered &o) { return max_bits(6.0 * o.m1 * o.m2 * o.m3, 1.0e-50); }
+// V1 = m1^3 / pr; V2 = V1 + 0.5 (m2 - m1) / m3; V3:
+__device__ __forceinline__ double al3d_v3(const Ordered &o) {
+  const double m1 = o.m1, m2 = o.m2, m3 = o.m3, m12 = o.m12;
+  const bool five = less_bits(m3, m12);  // regimes 3 and 5 up to m3, else 3 and 4 up to m12
+  double num = 0.5 * m12, den = m3;
   if (five) {
     num = m3 * m3 * (3.0 * m12 - m3) + m1 * m1 * (m1 - 3.0 * m3) + m2 * m2 * (m2 - 3.0 * m3);
-    den = pr;
+    den = al3d_pr(o);
   }
-  const double V3 = num / den;
-  const double ch = dmin1(cc, 1.0 - cc);
-  double res;
-  if (ch < V1) {
-    res = pow(pr * ch, 1.0 / 3.0);
-  } else if (ch < V2) {
-    res = 0.5 * (m1 + sqrt(m1 * m1 + 8.0 * m2 * m3 * (ch - V1)));
-  } else if (ch >= V3 && mm == m12) {
-    res = m3 * ch + 0.5 * mm;
-  } else {
-    double p = 2.0 * m1 * m2, q = 1.5 * m1 * m2 * (m12 - 2.0 * m3 * ch), add = m12;
-    if (!(ch < V3)) {
-      p = m1 * (m2 + m3) + m2 * m3 - 0.25;
-      q = 1.5 * m1 * m2 * m3 * (0.5 - ch);
-      add = 0.5;
-    }
-    const double p12 = sqrt(p);
-    double cst = q / (p * p12);
-    if (cst > 1.0) cst = 1.0;
-    if (cst < -1.0) cst = -1.0;
-    const double cs = cos(acos(cst) / 3.0);
-    res = p12 * (sqrt(3.0 * (1.0 - cs * cs)) - cs) + add;
+  return num / den;
+}
+__device__ __forceinline__ double al3d_cubic(const Ordered &o, double ch, bool below_v3) {
+  const double m1 = o.m1, m2 = o.m2, m3 = o.m3, m12 = o.m12;
+  double p = 2.0 * m1 * m2, q = 1.5 * m1 * m2 * (m12 - 2.0 * m3 * ch), add = m12;
+  if (!below_v3) {
+    p = m1 * (m2 + m3) + m2 * m3 - 0.25;
+    q = 1.5 * m1 * m2 * m3 * (0.5 - ch);
+    add = 0.5;
   }
-  if (cc > 0.5) res = 1.0 - res;
-  return res;
+  const double p12 = sqrt(p);
+  double cst = q / (p * p12);
+  if (cst > 1.0) cst = 1.0;
+  if (cst < -1.0) cst = -1.0;
+  const double cs = cos(acos(cst) / 3.0);
+  return p12 * (sqrt(3.0 * (1.0 - cs * cs)) - cs) + add;
 }
 
 // FL3D: volume of the part of [r0, r0+dr0] x [0,1]^2 below the plane.
 __device__ double fl3d(double m1, double m2, double m3, double alpha, double r0, double dr0) {
   double al = alpha - m1 * r0;
-  al = al + dmax1(0.0, -m1 * dr0) + dmax1(0.0, -m2) + dmax1(0.0, -m3);
+  al = al + max0(-m1 * dr0) + max0(-m2) + max0(-m3);
   double tmp = fabs(m1) * dr0 + fabs(m2) + fabs(m3);
   const double n1 = fabs(m1) / tmp, n2 = fabs(m2) / tmp, n3 = fabs(m3) / tmp;
-  al = dmax1(0.0, dmin1(1.0, al / tmp));
-  const double al0 = dmin1(al, 1.0 - al);
-  double b1 = dmin1(n1 * dr0, n2), b3 = dmax1(n1 * dr0, n2), b2 = n3;
-  if (b2 < b1) {
+  al = al / tmp;
+  al = is_nan(al) ? al : max0(min_bits(1.0, al));
+  const double al0 = min_bits(al, 1.0 - al);
+  double b1 = min_bits(n1 * dr0, n2), b3 = max_bits(n1 * dr0, n2), b2 = n3;
+  if (less_bits(b2, b1)) {
     tmp = b1; b1 = b2; b2 = tmp;
-  } else if (b2 > b3) {
+  } else if (less_bits(b3, b2)) {
     tmp = b3; b3 = b2; b2 = tmp;
   }
   const double b12 = b1 + b2;
-  const double bm = dmin1(b12, b3);
-  const double pr = dmax1(6.0 * b1 * b2 * b3, 1.0e-50);
+  const double bm = min_bits(b12, b3);
+  const double pr = max_bits(6.0 * b1 * b2 * b3, 1.0e-50);
   double num, den = pr;
-  const bool two = !(al0 < b1) && al0 < b2;  // the regime with a second term, b1^3 / pr
-  if (al0 < b1) {
+  const bool two = !less_bits(al0, b1) && less_bits(al0, b2);  // the regime with a second term, b1^3 / pr
+  if (less_bits(al0, b1)) {
     num = al0 * al0 * al0;
-  } else if (al0 < b2) {
+  } else if (less_bits(al0, b2)) {
     num = 0.5 * al0 * (al0 - b1);
     den = b2 * b3;
-  } else if (al0 < bm) {
+  } else if (less_bits(al0, bm)) {
     num = al0 * al0 * (3.0 * b12 - al0) + b1 * b1 * (b1 - 3.0 * al0) + b2 * b2 * (b2 - 3.0 * al0);
-  } else if (bm == b12) {
+  } else if (same_bits(bm, b12)) {
     num = al0 - 0.5 * bm;
     den = b3;
   } else {
@@ -105,84 +118,114 @@ __device__ double fl3d(double m1, double m2, double m3, double alpha, double r0,
   }
   tmp = num / den;
   if (two) tmp = tmp + b1 * b1 * b1 / pr;
-  return al <= 0.5 ? tmp * dr0 : (1.0 - tmp) * dr0;
+  return (less_bits(0.5, al) ? 1.0 - tmp : tmp) * dr0;
 }
 
-// Fluxes of one interface cell q (0 < c < 1): Youngs normal from the 27-point
-// stencil, AL3D plane constant, Lagrangian stretch along D and the FL3D cut
-// volumes (swp, main.f:896-995).
+// Youngs normal from the 27-point stencil, component A (swp, main.f:896-925).
+template <int A>
+__device__ __forceinline__ double youngs(size_t q, const double *__restrict__ cc, long sy, long sz) {
+  const long sa = A == 1 ? 1 : (A == 2 ? sy : sz), sb = A == 1 ? sy : 1, sc = A == 3 ? sy : sz;
+  // the sums' order of the reference: the corners' two other axes, ...
+#define C(a, b, c) cc[(long)q + (long)(a) * sa + (long)(b) * sb + (long)(c) * sc]
+  double mm[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int s = 2 * h - 1;
+    mm[h] = C(s, -1, -1) + C(s, -1, 1) + C(s, 1, -1) + C(s, 1, 1) +
+            2.0 * (C(s, -1, 0) + C(s, 1, 0) + C(s, 0, -1) + C(s, 0, 1)) + 4.0 * C(s, 0, 0);
+  }
+#undef C
+  return mm[0] - mm[1];
+}
+
+// Fluxes of interface cells (0 < c < 1): Youngs normal, AL3D plane constant,
+// Lagrangian stretch along D and the FL3D cut volumes (swp, main.f:896-995).
+//
+// A warp scheduler starts one FP64 instruction every 64 cycles, and a cell is
+// some 900 of them in a row: 30 us, whatever the grid.  So a block's four warps
+// (one per scheduler) take the same 32 cells and deal out what is independent:
+// the components of the normal and their divisions, AL3D's three volumes and
+// its regimes, FL3D's calls.  64^3: 30 -> 16.5 us per sweep,
+// 128^3 32 -> 20; at 256^3, with many cells per scheduler, 39 and 41.
 template <int D>
-__device__ void iface_flux(size_t q, const double *__restrict__ us, const double *__restrict__ cc,
-                           double *__restrict__ vof1, double *__restrict__ vof2, double *__restrict__ vof3, Dims d,
-                           double tauh) {
+__device__ __forceinline__ void flux_cells(size_t q, bool in, const double *__restrict__ us,
+                                           const double *__restrict__ cc, double *__restrict__ vof1,
+                                           double *__restrict__ vof2, double *__restrict__ vof3, Dims d, double tauh) {
+  __shared__ double part[9][32];  // normal, its quotients, AL3D's parts
+  const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
   const long sy = (long)d.sy(), sz = (long)d.sz();
   const long sd = D == 1 ? 1 : (D == 2 ? sy : sz);
-  const double a1 = us[q] * tauh;
-  const double a2 = us[q + sd] * tauh;
-  const double c0 = cc[q];
-  double f1 = 0.0, f2 = 0.0, f3 = 0.0;
-#define C(di, dj, dk) cc[(long)q + (long)(di) + (long)(dj) * sy + (long)(dk) * sz]
-  double mm1, mm2, mx, my, mz;
-  mm1 = C(-1, -1, -1) + C(-1, -1, 1) + C(-1, 1, -1) + C(-1, 1, 1) +
-        2.0 * (C(-1, -1, 0) + C(-1, 1, 0) + C(-1, 0, -1) + C(-1, 0, 1)) + 4.0 * C(-1, 0, 0);
-  mm2 = C(1, -1, -1) + C(1, -1, 1) + C(1, 1, -1) + C(1, 1, 1) +
-        2.0 * (C(1, -1, 0) + C(1, 1, 0) + C(1, 0, -1) + C(1, 0, 1)) + 4.0 * C(1, 0, 0);
-  mx = mm1 - mm2;
-  mm1 = C(-1, -1, -1) + C(-1, -1, 1) + C(1, -1, -1) + C(1, -1, 1) +
-        2.0 * (C(-1, -1, 0) + C(1, -1, 0) + C(0, -1, -1) + C(0, -1, 1)) + 4.0 * C(0, -1, 0);
-  mm2 = C(-1, 1, -1) + C(-1, 1, 1) + C(1, 1, -1) + C(1, 1, 1) +
-        2.0 * (C(-1, 1, 0) + C(1, 1, 0) + C(0, 1, -1) + C(0, 1, 1)) + 4.0 * C(0, 1, 0);
-  my = mm1 - mm2;
-  mm1 = C(-1, -1, -1) + C(-1, 1, -1) + C(1, -1, -1) + C(1, 1, -1) +
-        2.0 * (C(-1, 0, -1) + C(1, 0, -1) + C(0, -1, -1) + C(0, 1, -1)) + 4.0 * C(0, 0, -1);
-  mm2 = C(-1, -1, 1) + C(-1, 1, 1) + C(1, -1, 1) + C(1, 1, 1) +
-        2.0 * (C(-1, 0, 1) + C(1, 0, 1) + C(0, -1, 1) + C(0, 1, 1)) + 4.0 * C(0, 0, 1);
-  mz = mm1 - mm2;
-#undef C
-  if (mx == 0.0 && my == 0.0 && mz == 0.0) {
+  const double a1 = us[q] * tauh, a2 = us[q + sd] * tauh, c0 = cc[q];
+  if (role == 0) part[0][lane] = youngs<1>(q, cc, sy, sz);
+  if (role == 1) part[1][lane] = youngs<2>(q, cc, sy, sz);
+  if (role == 2) part[2][lane] = youngs<3>(q, cc, sy, sz);
+  __syncthreads();
+  double mx = part[0][lane], my = part[1][lane], mz = part[2][lane];
+  const bool flat = zero(mx) && zero(my) && zero(mz), store = in && !flat;
+  const bool nx = negative(mx), ny = negative(my), nz = negative(mz);
+  if (nx) mx = -mx;
+  if (ny) my = -my;
+  if (nz) mz = -mz;
+  if (role < 3) {
+    const double mm2 = mx + my + mz + (double)1.e-30f;  // default-REAL literal of main.f:927
+    part[3 + role][lane] = (role == 0 ? mx : role == 1 ? my : mz) / mm2;
+  } else if (in && flat) {
     // Deviation from swp: a symmetric neighbourhood gives an all-zero Youngs
     // normal, for which FL3D divides 0/0.  Such a cell is advected as a
     // uniformly filled one (donor-cell fluxes scaled by c).
     vof1[q] = c0 * dmax1(-a1, 0.0);
     vof2[q] = c0 * (1.0 - dmax1(a1, 0.0) + dmin1(a2, 0.0));
     vof3[q] = c0 * dmax1(a2, 0.0);
-    return;
   }
-  double invx = 1.0, invy = 1.0, invz = 1.0;
-  if (mx < 0.0) { mx = -mx; invx = -1.0; }
-  if (my < 0.0) { my = -my; invy = -1.0; }
-  if (mz < 0.0) { mz = -mz; invz = -1.0; }
-  mm2 = mx + my + mz + (double)1.e-30f;  // default-REAL literal of main.f:927
-  mx = mx / mm2;
-  my = my / mm2;
-  mz = mz / mm2;
-  double alpha = al3d(mx, my, mz, c0);
-  mx = invx * mx;
-  my = invy * my;
-  mz = invz * mz;
-  alpha = alpha + dmin1(0.0, mx) + dmin1(0.0, my) + dmin1(0.0, mz);
-  mm1 = dmax1(a1, 0.0);
-  mm2 = 1.0 - mm1 + dmin1(0.0, a2);
+  __syncthreads();
+  mx = part[3][lane];
+  my = part[4][lane];
+  mz = part[5][lane];
+  const Ordered o = ordered(mx, my, mz);
+  const double ch = min_bits(c0, 1.0 - c0);
+  if (nx) mx = -mx;
+  if (ny) my = -my;
+  if (nz) mz = -mz;
   // The sweep direction's normal component goes first in FL3D.
   double n1, n2, n3;
   if (D == 1) { n1 = mx; n2 = my; n3 = mz; }
   else if (D == 2) { n1 = my; n2 = mz; n3 = mx; }
   else { n1 = mz; n2 = mx; n3 = my; }
-  n1 = n1 / (1.0 - a1 + a2);
-  alpha = alpha + n1 * a1;
-  // The outflow at either end: in most cells there is one at most, so lanes
-  // with an outflow to the left and lanes with one to the right share a call.
-  const bool left = a1 < 0.0, right = a2 > 0.0;
-  if (left || right) {
-    const double f = fl3d(n1, n2, n3, alpha, left ? a1 : 1.0, left ? -a1 : a2);
-    if (left) f1 = f;
-    else f3 = f;
+  if (role == 0) part[6][lane] = o.m1 * o.m1 * o.m1 / al3d_pr(o);
+  if (role == 1) part[7][lane] = 0.5 * (o.m2 - o.m1) / o.m3;
+  if (role == 2) part[8][lane] = al3d_v3(o);
+  if (role == 3) part[0][lane] = n1 / (1.0 - a1 + a2);
+  __syncthreads();
+  const double V1 = part[6][lane], V2 = V1 + part[7][lane], V3 = part[8][lane];
+  n1 = part[0][lane];
+  const bool one = less_bits(ch, V1), two = !one && less_bits(ch, V2), third = less_bits(ch, V3);
+  const bool four = !one && !two && !third && !less_bits(o.m3, o.m12);
+  if (role == 0 && one) part[1][lane] = pow(al3d_pr(o) * ch, 1.0 / 3.0);
+  if (role == 1 && two) part[1][lane] = 0.5 * (o.m1 + sqrt(o.m1 * o.m1 + 8.0 * o.m2 * o.m3 * (ch - V1)));
+  if (role == 1 && four) part[1][lane] = o.m3 * ch + 0.5 * o.m12;
+  if (role == 2 && !(one || two || four)) part[1][lane] = al3d_cubic(o, ch, third);
+  __syncthreads();
+  if (role < 3) {
+    double alpha = part[1][lane];
+    if (less_bits(0.5, c0)) alpha = 1.0 - alpha;
+    alpha = alpha + min0(mx) + min0(my) + min0(mz);
+    alpha = alpha + n1 * a1;
+    // The outflow at either end: in most cells there is one at most, so lanes
+    // with an outflow to the left and lanes with one to the right share a call.
+    const bool left = negative(a1), right = positive_bits(a2);
+    if (role == 0 && store) {
+      const double mm1 = max0(a1);
+      vof2[q] = fl3d(n1, n2, n3, alpha, mm1, 1.0 - mm1 + min0(a2));
+    }
+    if (role == 1 && store) {
+      double f = 0.0;
+      if (left || right) f = fl3d(n1, n2, n3, alpha, left ? a1 : 1.0, left ? -a1 : a2);
+      vof1[q] = left ? f : 0.0;
+      if (!(left && right)) vof3[q] = left ? 0.0 : f;
+    }
+    if (role == 2 && store && left && right) vof3[q] = fl3d(n1, n2, n3, alpha, 1.0, a2);
   }
-  if (left && right) f3 = fl3d(n1, n2, n3, alpha, 1.0, a2);
-  f2 = fl3d(n1, n2, n3, alpha, mm1, mm2);
-  vof1[q] = f1;
-  vof2[q] = f2;
-  vof3[q] = f3;
+  __syncthreads();
 }
 
 // Bits of the cells with c != +0, one word per 32 cells along x: word w of row
@@ -243,15 +286,15 @@ __global__ void k_swp_scan(const double *__restrict__ us, const double *__restri
   }
 }
 
-// Pass 2: the listed interface cells, one per thread.
+// Pass 2: the listed interface cells, 32 per block at a time.
 template <int D>
 __global__ void k_swp_flux_iface(const unsigned *__restrict__ list, const unsigned *__restrict__ count,
                                  const double *__restrict__ us, const double *__restrict__ cc,
                                  double *__restrict__ vof1, double *__restrict__ vof2, double *__restrict__ vof3,
                                  Dims d, double tauh) {
-  const unsigned n = *count;
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-    iface_flux<D>(list[t], us, cc, vof1, vof2, vof3, d, tauh);
+  const unsigned n = *count, lane = threadIdx.x & 31;
+  for (unsigned t = 32 * blockIdx.x; t < n; t += 32 * gridDim.x)
+    flux_cells<D>(list[min(t + lane, n - 1)], t + lane < n, us, cc, vof1, vof2, vof3, d, tauh);
 }
 
 // Pass 3: c = vof3(-1) + vof2 + vof1(+1) along D clipped to [0,1], a missing
@@ -386,7 +429,7 @@ void sweep(const double *us, double *cc, double *v1, double *v2, double *v3, Dim
   // One warp per block: a cell is some thousand FP64 operations in sequence,
   // and warps on one SM share its FP64 pipe, so a short list goes to as many
   // SMs as it has warps (64^3 droplet: 36 us, 40 us with four warps per block).
-  DSG_COUNT k_swp_flux_iface<D><<<4 * kRedBlocks, 32, 0, st>>>(list, count, us, cc, v1, v2, v3, d, tauh);
+  DSG_COUNT k_swp_flux_iface<D><<<kRedBlocks, 128, 0, st>>>(list, count, us, cc, v1, v2, v3, d, tauh);
   const size_t words = (size_t)wpr * (d.ny - 2) * (d.nz - 2);
   // Words per warp: on small grids few, because a warp goes through its busy
   // words one after the other (64^3: 4 us with 4, 12 us with 32); on large ones
