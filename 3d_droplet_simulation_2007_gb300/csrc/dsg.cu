@@ -129,13 +129,13 @@ inline bool fp64_fma(const dsg_ctx *ctx) {
 template <class A>
 bool phases(const dsg_ctx *ctx, const A &level, int l);
 
-// Whether level l's FP64 sweeps share products (sweeps pass by pass in the
-// reference's rounding); they and the flags lie in the level's FP32 arrays,
-// which only the mixed modes use.
+// Whether level l's FP64 sweeps run pass by pass and so have short forms for
+// cells in one fluid; the products that they share in the reference's rounding
+// and the flags lie in the level's FP32 arrays, which only the mixed modes use.
 bool products(const dsg_ctx *ctx, int l, dsg::Products *P) {
-  if (ctx->cfg.mode == DSG_MODE_TOL_MIXED || ctx->cfg.mode == DSG_MODE_LEARNED || fp64_fma(ctx)) return false;
+  if (ctx->cfg.mode == DSG_MODE_TOL_MIXED || ctx->cfg.mode == DSG_MODE_LEARNED) return false;
   if (l <= ctx->tail64_top || phases(ctx, ctx->gr64[l], l)) return false;
-  P->v = (double *)ctx->lv32[l][0];
+  P->v = fp64_fma(ctx) ? nullptr : (double *)ctx->lv32[l][0];
   P->flags = (unsigned char *)ctx->lv32[l][2];
   const double r1 = 0.5 * (ctx->s.rho1 - ctx->s.rho2), r2 = ctx->s.rho2;
   P->k = 1.0 / (r1 * (0.0 + 0.0) + r2);

@@ -207,9 +207,11 @@ cudaError_t relax(double *u, double lengthsize, const double *rhs, const double 
 // fma = false: the reference's operation order, bit-identical to the oracle.
 // P: the coefficient times u in gas, shared between neighbours (k_relax_colour)
 struct Products {
-  double *v;             // product per node, scratch
+  double *v;             // product per node, scratch (null: the fused form)
   unsigned char *flags;  // per warp of a colour pass (bulk_flags)
   double k, e, k1, e1;   // face coefficient and ei of gas, of liquid
+  // fused form: u = keep * u + w * sum + z * rhs (relax_n sets them)
+  double keep, w, z, w1, z1;
 };
 cudaError_t relax_n(int n, double *u, double lengthsize, const double *rhs, const double *a,
                     const double *b, const double *c, const double *ei, Dims d, double omega,
