@@ -129,12 +129,19 @@ inline bool fp64_fma(const dsg_ctx *ctx) {
 template <class A>
 bool phases(const dsg_ctx *ctx, const A &level, int l);
 
+constexpr long long kShortFormCells = 80000;  // a cooperative phase: 256 cells per colour on each SM
+
 // Whether level l's FP64 sweeps run pass by pass and so have short forms for
 // cells in one fluid; the products that they share in the reference's rounding
 // and the flags lie in the level's FP32 arrays, which only the mixed modes use.
 bool products(const dsg_ctx *ctx, int l, dsg::Products *P) {
   if (ctx->cfg.mode == DSG_MODE_TOL_MIXED || ctx->cfg.mode == DSG_MODE_LEARNED) return false;
   if (l <= ctx->tail64_top || phases(ctx, ctx->gr64[l], l)) return false;
+  // The fused form rounds differently, so a level has it or not whether the
+  // context runs alone or in an ensemble: those that no cluster and no
+  // cooperative phase can hold.
+  const Dims d = ctx->level(l);
+  if (fp64_fma(ctx) && (long long)(d.nx - 2) * (d.ny - 2) * (d.nz - 2) <= kShortFormCells) return false;
   P->v = fp64_fma(ctx) ? nullptr : (double *)ctx->lv32[l][0];
   P->flags = (unsigned char *)ctx->lv32[l][2];
   const double r1 = 0.5 * (ctx->s.rho1 - ctx->s.rho2), r2 = ctx->s.rho2;

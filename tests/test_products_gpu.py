@@ -33,3 +33,19 @@ def test_mglin_matches_oracle(gpu_lib, shape, npre, rho2):
     ora.mglin()
     gpu.mglin()
     assert np.array_equal(gpu.field("p"), ora.field("p"))
+
+
+def test_fused_form_is_the_same_in_an_ensemble(gpu_lib):
+    """Members keep levels in clusters and passes that a context of its own runs
+    as cooperative phases; the short fused form applies to neither."""
+    dsg = gpu_lib
+    inputs = [dsg.config.droplet(n, mode=1, tol=1e-8, impact_speed=2.0) for n in (32, 40, 48, 64)]
+    alone = []
+    for inp in inputs:
+        with dsg.Solver(inp) as s:
+            s.step(1)
+            alone.append(s.field("p"))
+    with dsg.Ensemble(inputs, workers=2) as e:
+        e.step(1)
+        for i, p in enumerate(alone):
+            assert np.array_equal(e.member(i).field("p"), p), i
