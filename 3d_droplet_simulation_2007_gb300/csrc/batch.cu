@@ -162,12 +162,16 @@ __global__ void kb_relax32(BATCH_PARAMS(ARelax), int colour) {
 
 __global__ void kb_resid_restrict32_split(BATCH_PARAMS(ARRSplit)) {
   FOR_MEMBER_BLOCKS(ARRSplit) {
-    if (split_vec(a.sp))
-      b_resid_restrict32_split<true>(B, G, a.rhs_c, a.u_c, a.ue, a.uo, a.re, a.ro, a.cc, a.flags, a.df, a.sp, a.dc,
-                                     a.h2i, a.r1, a.r2);
+    const int form = split_form(a.sp);
+    if (form == 2)
+      b_resid_restrict32_split<2>(B, G, a.rhs_c, a.u_c, a.ue, a.uo, a.re, a.ro, a.cc, a.flags, a.df, a.sp, a.dc, a.h2i,
+                                  a.r1, a.r2);
+    else if (form == 1)
+      b_resid_restrict32_split<1>(B, G, a.rhs_c, a.u_c, a.ue, a.uo, a.re, a.ro, a.cc, a.flags, a.df, a.sp, a.dc, a.h2i,
+                                  a.r1, a.r2);
     else
-      b_resid_restrict32_split<false>(B, G, a.rhs_c, a.u_c, a.ue, a.uo, a.re, a.ro, a.cc, a.flags, a.df, a.sp, a.dc,
-                                      a.h2i, a.r1, a.r2);
+      b_resid_restrict32_split<0>(B, G, a.rhs_c, a.u_c, a.ue, a.uo, a.re, a.ro, a.cc, a.flags, a.df, a.sp, a.dc, a.h2i,
+                                  a.r1, a.r2);
   });
 }
 
@@ -359,7 +363,11 @@ dim3 grid_of(int k, const Dims &d, dim3 blk) {
     }
     case K_PRO_SPLIT: {
       const int hx = (d.nx - 2) >> 1;
-      return dim3(cdiv(hx, blk.x), cdiv(d.ny - 2, blk.y), d.nz - 2);
+      return dim3(cdiv(hx, blk.x), cdiv((d.ny - 2) / 2, blk.y), (d.nz - 2) / 2);
+    }
+    case K_RR_SPLIT: {  // d: the coarse level
+      const Split sp{d.nx - 2, 2 * (d.ny - 2), 2 * (d.nz - 2)};
+      return dim3(cdiv(split_pairs(sp) ? sp.hx / 2 : sp.hx, blk.x), cdiv(d.ny - 2, blk.y), d.nz - 2);
     }
     default:  // interior grid of d
       return dim3(cdiv(d.nx - 2, blk.x), cdiv(d.ny - 2, blk.y), d.nz - 2);

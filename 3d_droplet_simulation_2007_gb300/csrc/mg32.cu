@@ -30,13 +30,13 @@ __global__ void k_relax32_split(float *__restrict__ self, const float *__restric
   b_relax32_split<VEC>(blockIdx, gridDim, self, other, rhs_self, cc, flags, d, sp, c, h2, omega, r1, r2);
 }
 
-template <bool VEC>
+template <int V>
 __global__ void k_resid_restrict32_split(float *__restrict__ rhs_c, float *__restrict__ u_c, const float *__restrict__ ue,
                                          const float *__restrict__ uo, const float *__restrict__ re,
                                          const float *__restrict__ ro, const float *__restrict__ cc,
                                          const unsigned char *__restrict__ flags, Dims df, Split sp, Dims dc, float h2i,
                                          float r1, float r2) {
-  b_resid_restrict32_split<VEC>(blockIdx, gridDim, rhs_c, u_c, ue, uo, re, ro, cc, flags, df, sp, dc, h2i, r1, r2);
+  b_resid_restrict32_split<V>(blockIdx, gridDim, rhs_c, u_c, ue, uo, re, ro, cc, flags, df, sp, dc, h2i, r1, r2);
 }
 
 template <bool TRI>
@@ -494,20 +494,24 @@ cudaError_t resid_restrict32_split(float *rhs_c, float *u_c, float *const u[2], 
                                    cudaStream_t st) {
   const Dims dc{df.nx / 2 + 1, df.ny / 2 + 1, df.nz / 2 + 1};
   const Split sp{(df.nx - 2) >> 1, df.ny - 2, df.nz - 2};
-  if (split_vec(sp))
-    DSG_COUNT k_resid_restrict32_split<true><<<interior_grid(dc, kBlk), kBlk, 0, st>>>(
-        rhs_c, u_c, u[0], u[1], rhs[0], rhs[1], cc, flags, df, sp, dc, h2i, r1, r2);
-  else
-    DSG_COUNT k_resid_restrict32_split<false><<<interior_grid(dc, kBlk), kBlk, 0, st>>>(
-        rhs_c, u_c, u[0], u[1], rhs[0], rhs[1], cc, flags, df, sp, dc, h2i, r1, r2);
+  const unsigned x = split_pairs(sp) ? sp.hx / 2 : sp.hx, bx = split_pairs(sp) && x < 128 ? x : kBlk.x;  // whole rows of pairs
+  const dim3 blk(bx, 128 / bx), grid((x + bx - 1) / bx, (dc.ny - 2 + blk.y - 1) / blk.y, dc.nz - 2);
+  auto go = [&](auto kernel) {
+    DSG_COUNT kernel<<<grid, blk, 0, st>>>(rhs_c, u_c, u[0], u[1], rhs[0], rhs[1], cc, flags, df, sp, dc, h2i, r1, r2);
+  };
+  switch (split_form(sp)) {
+    case 2: go(k_resid_restrict32_split<2>); break;
+    case 1: go(k_resid_restrict32_split<1>); break;
+    default: go(k_resid_restrict32_split<0>);
+  }
   return cudaGetLastError();
 }
 
 cudaError_t prolong32_split(float *const u[2], const float *uc, Dims df, int add, int tri, cudaStream_t st) {
   const Dims dc{df.nx / 2 + 1, df.ny / 2 + 1, df.nz / 2 + 1};
   const Split sp{(df.nx - 2) >> 1, df.ny - 2, df.nz - 2};
-  const dim3 grid((unsigned)((sp.hx + kBlk.x - 1) / kBlk.x), (unsigned)((df.ny - 2 + kBlk.y - 1) / kBlk.y),
-                  (unsigned)(df.nz - 2));
+  const dim3 grid((unsigned)((sp.hx + kBlk.x - 1) / kBlk.x), (unsigned)((dc.ny - 2 + kBlk.y - 1) / kBlk.y),
+                  (unsigned)(dc.nz - 2));
   if (tri)
     DSG_COUNT k_prolong32_split<true><<<grid, kBlk, 0, st>>>(u[0], u[1], uc, df, sp, dc, add);
   else

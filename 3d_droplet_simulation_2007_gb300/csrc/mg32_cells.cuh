@@ -356,30 +356,14 @@ __device__ __forceinline__ void b_relax32_split(const uint3 B, const uint3 G, fl
                   upd(u.z, xp.z, xm.z, yp.z, ym.z, zp.z, zm.z, f4.z), upd(u.w, xp.w, xm.w, yp.w, ym.w, zp.w, zm.w, f4.w));
 }
 
-// Finest-level residual (cc-derived operator, virtual ghosts) restricted to the
-// coarse rhs: mean of the 8 fine residuals of each coarse cell.
-template <bool VEC>
-__device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const uint3 G, float *__restrict__ rhs_c, float *__restrict__ u_c, const float *__restrict__ ue,
-                                         const float *__restrict__ uo, const float *__restrict__ re,
-                                         const float *__restrict__ ro, const float *__restrict__ cc,
-                                         const unsigned char *__restrict__ flags, Dims df, Split sp, Dims dc, float h2i,
-                                         float r1, float r2) {
-  const int ic = B.x * blockDim.x + threadIdx.x + 2;
-  const int jc = B.y * blockDim.y + threadIdx.y + 2;
-  const int kc = B.z + 2;
-  if (ic > dc.nx - 1 || jc > dc.ny - 1) return;
-  // the warp's 32 coarse cells lie in one segment of each of the four rows
-  unsigned f00 = 0;
-  bool uniform = false;
-  if (VEC) {
-    const int seg = (ic - 2) >> 5;
-    f00 = seg_flag(flags, df, 2 * jc - 2, 2 * kc - 2)[seg];
-    const unsigned f10 = seg_flag(flags, df, 2 * jc - 1, 2 * kc - 2)[seg],
-                   f01 = seg_flag(flags, df, 2 * jc - 2, 2 * kc - 1)[seg],
-                   f11 = seg_flag(flags, df, 2 * jc - 1, 2 * kc - 1)[seg];
-    uniform = f00 && f00 == f10 && f00 == f01 && f00 == f11;
-  }
-  const float cu = f00 == 2 ? 1.f : 0.f, ku = face_coef(cu, cu, r1, r2);
+// Mean of the 8 fine residuals of coarse cell (ic, jc, kc), from cc or, where
+// its rows lie in one fluid (flag 1 or 2), with that one's coefficient.
+__device__ __forceinline__ void resid_restrict32_split_cell(float *__restrict__ rhs_c, float *__restrict__ u_c,
+                                                            const float *__restrict__ ue, const float *__restrict__ uo,
+                                                            const float *__restrict__ re, const float *__restrict__ ro,
+                                                            const float *__restrict__ cc, unsigned flag, Dims df, Split sp,
+                                                            Dims dc, float h2i, float r1, float r2, int ic, int jc, int kc) {
+  const float cu = flag == 2 ? 1.f : 0.f, ku = face_coef(cu, cu, r1, r2);
   float acc = 0.f;
 #pragma unroll
   for (int dk = 0; dk < 2; dk++)
@@ -396,7 +380,7 @@ __device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const ui
         const float zp = (k + 1 == df.nz) ? uc : split_get(ue, uo, sp, i, j, k + 1);
         const float zm = (k == 2) ? uc : split_get(ue, uo, sp, i, j, k - 1);
         float ae = ku, aw = ku, bn = ku, bs = ku, ct = ku, cb = ku;
-        if (!uniform) {
+        if (!flag) {
           const float *cq = cc + ix32(df, i, j, k);
           const int sy = df.nx, sz = df.nx * df.ny;
           const float c0 = cq[0];
@@ -414,34 +398,142 @@ __device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const ui
   u_c[qc] = 0.f;
 }
 
+// Finest-level residual (cc-derived operator, virtual ghosts) restricted to the
+// coarse rhs: mean of the 8 fine residuals of each coarse cell.  A thread
+// has two coarse cells, and where its rows lie in one fluid it loads the 24 rows
+// of u and 8 of the right-hand side that their 16 residuals need as pairs, 40
+// loads in place of 128 (256^3: 65 -> 34 us, 160^3 15.5 -> 13); grids below
+// kPairCells have too few threads that way (128^3: 8.7 us, 10.1 so).
+constexpr int kPairCells = 1500000;  // per colour
+__host__ __device__ __forceinline__ bool split_pairs(Split sp) {
+  return split_vec(sp) && (long long)sp.hx * sp.ny2 * sp.nz2 >= kPairCells;
+}
+// V: split_form, 0: no uniform segments, 1: one coarse cell per thread, 2: two.
+__host__ __device__ __forceinline__ int split_form(Split sp) { return !split_vec(sp) ? 0 : split_pairs(sp) ? 2 : 1; }
+template <int V>
+__device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const uint3 G, float *__restrict__ rhs_c, float *__restrict__ u_c, const float *__restrict__ ue,
+                                         const float *__restrict__ uo, const float *__restrict__ re,
+                                         const float *__restrict__ ro, const float *__restrict__ cc,
+                                         const unsigned char *__restrict__ flags, Dims df, Split sp, Dims dc, float h2i,
+                                         float r1, float r2) {
+  const int jc = B.y * blockDim.y + threadIdx.y + 2;
+  const int kc = B.z + 2;
+  // the warp's coarse cells lie in one segment of each of the four rows
+  const int m = (V == 2 ? 2 : 1) * (int)(B.x * blockDim.x + threadIdx.x);
+  if (m >= sp.hx || jc > dc.ny - 1) return;
+  const int seg = m >> 5, j0 = 2 * jc - 2, k0 = 2 * kc - 2;
+  unsigned f00 = 0;
+  if (V) {
+    f00 = seg_flag(flags, df, j0, k0)[seg];
+    const unsigned f10 = seg_flag(flags, df, j0 + 1, k0)[seg], f01 = seg_flag(flags, df, j0, k0 + 1)[seg],
+                   f11 = seg_flag(flags, df, j0 + 1, k0 + 1)[seg];
+    if (f00 != f10 || f00 != f01 || f00 != f11) f00 = 0;
+  }
+  if (V < 2 || !f00) {
+    for (int t = 0; t < (V == 2 ? 2 : 1); t++)
+      resid_restrict32_split_cell(rhs_c, u_c, ue, uo, re, ro, cc, V == 2 ? 0 : f00, df, sp, dc, h2i, r1, r2, m + t + 2, jc, kc);
+    return;
+  }
+  const unsigned row = sp.hx, plane = sp.hx * sp.ny2;
+  const unsigned q0 = (unsigned)m + row * (unsigned)(j0 - 2) + plane * (unsigned)(k0 - 2);
+  auto vec = [](const float *x) { return *reinterpret_cast<const float2 *>(x); };
+  // u of the four rows and of those beside them, even and odd cells
+  float2 ev[4][4], od[4][4];
+#pragma unroll
+  for (int z = 0; z < 4; z++)
+#pragma unroll
+    for (int y = 0; y < 4; y++) {
+      ev[z][y] = od[z][y] = make_float2(0.f, 0.f);
+      if (((y == 0 || y == 3) && (z == 0 || z == 3)) || (y == 0 && j0 == 2) || (y == 3 && j0 + 2 == df.ny) ||
+          (z == 0 && k0 == 2) || (z == 3 && k0 + 2 == df.nz))
+        continue;
+      const unsigned q = q0 + row * (unsigned)(y - 1) + plane * (unsigned)(z - 1);
+      ev[z][y] = vec(ue + q);
+      od[z][y] = vec(uo + q);
+    }
+  const float cu = f00 == 2 ? 1.f : 0.f, ku = face_coef(cu, cu, r1, r2);
+  float acc0 = 0.f, acc1 = 0.f;
+#pragma unroll
+  for (int dk = 0; dk < 2; dk++)
+#pragma unroll
+    for (int dj = 0; dj < 2; dj++) {
+      const int z = dk + 1, y = dj + 1;
+      const bool odd = (dj + dk) & 1;  // colour of i = 2 + 2m, as j0 + k0 is even
+      const unsigned q = q0 + row * (unsigned)dj + plane * (unsigned)dk;
+      // of a row: cells 2 + 2m, 4 + 2m (first) and 3 + 2m, 5 + 2m; in the rows beside it the colours change places
+      auto first = [&](int z, int y) { return ((y + z) & 1) ? od[z][y] : ev[z][y]; };
+      auto second = [&](int z, int y) { return ((y + z) & 1) ? ev[z][y] : od[z][y]; };
+      const float2 a = first(z, y), b = second(z, y);
+      const float before = m == 0 ? a.x : (odd ? ue : uo)[q - 1], after = m + 2 == sp.hx ? 0.f : (odd ? uo : ue)[q + 2];
+#pragma unroll
+      for (int s = 0; s < 2; s++) {
+        auto of = [&](int z, int y) { return s ? second(z, y) : first(z, y); };
+        const float2 u = s ? b : a, f = vec(((s != 0) != odd ? ro : re) + q);
+        const float2 xp = s ? make_float2(a.y, after) : b, xm = s ? a : make_float2(before, b.x);
+        const float2 yp = dj == 1 && j0 + 2 == df.ny ? u : of(z, y + 1), ym = dj == 0 && j0 == 2 ? u : of(z, y - 1);
+        const float2 zp = dk == 1 && k0 + 2 == df.nz ? u : of(z + 1, y), zm = dk == 0 && k0 == 2 ? u : of(z - 1, y);
+        acc0 += fmaf(-h2i, face_diff(u.x, ku, xp.x, ku, xm.x, ku, yp.x, ku, ym.x, ku, zp.x, ku, zm.x), f.x);
+        acc1 += fmaf(-h2i, face_diff(u.y, ku, xp.y, ku, xm.y, ku, yp.y, ku, ym.y, ku, zp.y, ku, zm.y), f.y);
+      }
+    }
+  const unsigned qc = ix32(dc, m + 2, jc, kc);
+  rhs_c[qc] = 0.125f * acc0;
+  rhs_c[qc + 1] = 0.125f * acc1;
+  u_c[qc] = u_c[qc + 1] = 0.f;
+}
+
 // Fine (split) u = or += the interpolated coarse correction.
-// One thread per colour-split index (m, j, k): its even and odd cells are
-// i = 2+2m and 3+2m in some order, both children of coarse cell m+2 along x,
-// so both arrays are updated with coalesced accesses.
+// One thread per coarse cell (m + 2, jc, kc): in each of its four fine rows the
+// even and odd cell of split index m are its children, so both arrays are
+// updated with coalesced accesses.  The eight children interpolate from 27
+// coarse values, which a thread per row and split index would load as 48
+// (160^3: 13.5 -> 10.1 us, 128^3 7.6 -> 6.7; at
+// 256^3 memory takes 41 either way).
 template <bool TRI>
 __device__ __forceinline__ void b_prolong32_split(const uint3 B, const uint3 G, float *__restrict__ ue, float *__restrict__ uo, const float *__restrict__ uc,
                                   Dims df, Split sp, Dims dc, int add) {
   const int m = B.x * blockDim.x + threadIdx.x;
-  const int j = B.y * blockDim.y + threadIdx.y + 2;
-  const int k = B.z + 2;
-  if (m >= sp.hx || j > df.ny - 1) return;
-  const int pi = m + 2, pj = (j >> 1) + 1, pk = (k >> 1) + 1;
-  float v0, v1;  // cells i = 2+2m and i = 3+2m
+  const int jc = B.y * blockDim.y + threadIdx.y + 2;
+  const int kc = B.z + 2;
+  if (m >= sp.hx || jc > dc.ny - 1) return;
+  const int pi = m + 2;
+  float v[3][3][3];  // coarse values at x, y, z -1 .. +1, Neumann ghosts resolved
   if (TRI) {
-    const int nj = tri_nb(j, pj, dc.ny), nk = tri_nb(k, pk, dc.nz);
-    const float yc = tri_yz(uc, dc, pi, pj, nj, pk, nk);
-    const float yl = pi == 2 ? yc : tri_yz(uc, dc, pi - 1, pj, nj, pk, nk);
-    const float yr = pi + 1 == dc.nx ? 0.f : tri_yz(uc, dc, pi + 1, pj, nj, pk, nk);
-    v0 = tri_x(yc, yl);
-    v1 = tri_x(yc, yr);
+    const int jn[3] = {jc == 2 ? jc : jc - 1, jc, jc + 1 == dc.ny ? jc : jc + 1};
+    const int kn[3] = {kc == 2 ? kc : kc - 1, kc, kc + 1 == dc.nz ? kc : kc + 1};
+#pragma unroll
+    for (int z = 0; z < 3; z++)
+#pragma unroll
+      for (int y = 0; y < 3; y++) {
+        const float *p = uc + ix32(dc, pi, jn[y], kn[z]);
+        v[1][y][z] = p[0];
+        v[0][y][z] = p[-1];  // beyond the faces: not used
+        v[2][y][z] = p[1];
+      }
   } else {
-    v0 = v1 = uc[ix32(dc, pi, pj, pk)];
+    v[1][1][1] = uc[ix32(dc, pi, jc, kc)];
   }
-  const bool odd_first = (j + k) & 1;  // cell 2+2m has odd i+j+k
-  const float ve = odd_first ? v1 : v0, vo = odd_first ? v0 : v1;
-  const unsigned q = at32(sp, m, j, k);
-  ue[q] = add ? ue[q] + ve : ve;
-  uo[q] = add ? uo[q] + vo : vo;
+#pragma unroll
+  for (int dk = 0; dk < 2; dk++)
+#pragma unroll
+    for (int dj = 0; dj < 2; dj++) {
+      float v0, v1;  // cells i = 2+2m and i = 3+2m
+      if (TRI) {
+        auto yz = [&](int x) {
+          return tri_yz_value(v[x][1][1], v[x][2 * dj][1], v[x][1][2 * dk], v[x][2 * dj][2 * dk]);
+        };
+        const float yc = yz(1), yl = pi == 2 ? yc : yz(0), yr = pi + 1 == dc.nx ? 0.f : yz(2);
+        v0 = tri_x(yc, yl);
+        v1 = tri_x(yc, yr);
+      } else {
+        v0 = v1 = v[1][1][1];
+      }
+      const bool odd_first = (dj + dk) & 1;  // cell 2+2m of row (2 jc - 2 + dj, 2 kc - 2 + dk) has odd i+j+k
+      const float ve = odd_first ? v1 : v0, vo = odd_first ? v0 : v1;
+      const unsigned q = at32(sp, m, 2 * jc - 2 + dj, 2 * kc - 2 + dk);
+      ue[q] = add ? ue[q] + ve : ve;
+      uo[q] = add ? uo[q] + vo : vo;
+    }
 }
 
 // 8-cell mean of the split fine rhs into the coarse interior (rstrct).
