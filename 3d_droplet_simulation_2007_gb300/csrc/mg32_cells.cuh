@@ -301,12 +301,20 @@ __device__ __forceinline__ float lap32_split_cell(const float *__restrict__ self
 // One colour pass on the finest level.  Rows of a multiple of four split
 // indices: a thread updates four neighbours; a warp whose cells all lie in
 // uniform segments reads and writes them as 16-byte vectors, any other warp one
-// by one (256^3: 28.6 us per pass, 45.4 with two cells per thread, uniform or
+// by one (256^3: 28.4 us per pass, 45.4 with two cells per thread, uniform or
 // not: that form issues 110 instructions per cell; 160^3: 7.6 against 12.9).
 // Other rows, and grids of fewer than kVecCells cells per colour, which have
 // too few threads that way (64^3: 3.3 us with two cells per thread, 3.7 with
 // four): split indices m and m + blockDim.x.  split_cells: the split indices
 // a block covers along a row.  VEC = split_vec(sp).
+//
+// The passes go through the planes back and forth (prolongation up, colour 0
+// down, colour 1 up, restriction down), so that each begins with what the one
+// before left in L2, and the right-hand side, which comes only every second
+// pass, is loaded as streaming data that need not stay there: at 256^3, where u
+// (67 MB) fits L2 and u and the right-hand side do not, a pass takes 28.4 us in
+// one direction, 25.0 back and forth, 22.0 with both (the prolongation 42, 38,
+// 33); at 160^3, which fits, it makes no difference.
 __host__ __device__ __forceinline__ int split_cells(Split sp, int blk_x) { return (split_vec(sp) ? 4 : 2) * blk_x; }
 
 template <bool VEC>
@@ -315,7 +323,7 @@ __device__ __forceinline__ void b_relax32_split(const uint3 B, const uint3 G, fl
                                 const unsigned char *__restrict__ flags, Dims d, Split sp, int c, float h2, float omega,
                                 float r1, float r2) {
   const int j = B.y * blockDim.y + threadIdx.y + 2;
-  const int k = B.z + 2;
+  const int k = (int)(c == 0 ? G.z - 1 - B.z : B.z) + 2;
   if (!VEC) {
     const int m = B.x * 2 * blockDim.x + threadIdx.x, m2 = m + (int)blockDim.x;
     if (j > d.ny - 1) return;
@@ -338,7 +346,7 @@ __device__ __forceinline__ void b_relax32_split(const uint3 B, const uint3 G, fl
   const unsigned q = (unsigned)m + row * (unsigned)(j - 2) + plane * (unsigned)(k - 2);
   auto vec = [](const float *x) { return *reinterpret_cast<const float4 *>(x); };
   const float *o = other + q;
-  const float4 u = vec(self + q), x = vec(o), f4 = vec(rhs_self + q);
+  const float4 u = vec(self + q), x = vec(o), f4 = __ldcs(reinterpret_cast<const float4 *>(rhs_self + q));
   const float4 ym = (j == 2) ? u : vec(o - row), yp = (j == d.ny - 1) ? u : vec(o + row);
   const float4 zm = (k == 2) ? u : vec(o - plane), zp = (k == d.nz - 1) ? u : vec(o + plane);
   // along x: the cell before (p = 0) or after (p = 1) the vector x as well
@@ -417,7 +425,7 @@ __device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const ui
                                          const unsigned char *__restrict__ flags, Dims df, Split sp, Dims dc, float h2i,
                                          float r1, float r2) {
   const int jc = B.y * blockDim.y + threadIdx.y + 2;
-  const int kc = B.z + 2;
+  const int kc = (int)(G.z - 1 - B.z) + 2;
   // the warp's coarse cells lie in one segment of each of the four rows
   const int m = (V == 2 ? 2 : 1) * (int)(B.x * blockDim.x + threadIdx.x);
   if (m >= sp.hx || jc > dc.ny - 1) return;
@@ -468,7 +476,7 @@ __device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const ui
 #pragma unroll
       for (int s = 0; s < 2; s++) {
         auto of = [&](int z, int y) { return s ? second(z, y) : first(z, y); };
-        const float2 u = s ? b : a, f = vec(((s != 0) != odd ? ro : re) + q);
+        const float2 u = s ? b : a, f = __ldcs(reinterpret_cast<const float2 *>(((s != 0) != odd ? ro : re) + q));
         const float2 xp = s ? make_float2(a.y, after) : b, xm = s ? a : make_float2(before, b.x);
         const float2 yp = dj == 1 && j0 + 2 == df.ny ? u : of(z, y + 1), ym = dj == 0 && j0 == 2 ? u : of(z, y - 1);
         const float2 zp = dk == 1 && k0 + 2 == df.nz ? u : of(z + 1, y), zm = dk == 0 && k0 == 2 ? u : of(z - 1, y);
@@ -488,7 +496,7 @@ __device__ __forceinline__ void b_resid_restrict32_split(const uint3 B, const ui
 // updated with coalesced accesses.  The eight children interpolate from 27
 // coarse values, which a thread per row and split index would load as 48
 // (160^3: 13.5 -> 10.1 us, 128^3 7.6 -> 6.7; at
-// 256^3 memory takes 41 either way).
+// 256^3 memory bounds both).
 template <bool TRI>
 __device__ __forceinline__ void b_prolong32_split(const uint3 B, const uint3 G, float *__restrict__ ue, float *__restrict__ uo, const float *__restrict__ uc,
                                   Dims df, Split sp, Dims dc, int add) {
