@@ -369,8 +369,9 @@ cudaError_t relax32_level(dsg_ctx *ctx, int n, int l) {
     ctx->prof_used += 2;
     ctx->prof_relax_calls += n;
     // colour-split sweep: per colour pass the other colour (half), own colour
-    // read+write (half each), own rhs (half) and cc (full): 6 FP32 words per cell
-    ctx->prof_relax_bytes += (double)n * 6.0 * sizeof(float) * (double)d.count();
+    // read+write (half each) and own rhs (half): 4 FP32 words per cell; cc, which
+    // only cells near the interface read, is not counted
+    ctx->prof_relax_bytes += (double)n * 4.0 * sizeof(float) * (double)d.count();
     ctx->prof_relax_bits = 32;
   }
   return e;
@@ -582,7 +583,7 @@ int graph_run(dsg_ctx *ctx, GraphRec &g) {
       DSG_CK(ctx, cudaEventElapsedTime(&x, g.ev[2 * q], g.ev[2 * q + 1]));
       ctx->prof_graph_relax_ms += x;
       ctx->prof_relax_calls += g.ev_n[q];
-      ctx->prof_relax_bytes += (double)g.ev_n[q] * 6.0 * sizeof(float) * (double)ctx->fine().count();
+      ctx->prof_relax_bytes += (double)g.ev_n[q] * 4.0 * sizeof(float) * (double)ctx->fine().count();
       ctx->prof_relax_bits = 32;
     }
   }

@@ -334,7 +334,7 @@ def relax_roofline(prof, step_ms, n):
     kname = "k_relax32_split" if split else "k_relax_colour"
     return {"bound": "hbm",
             "kernel": ("%s: finest-level relax, colour-split FP32 red-black sweep, 2 launches per relax "
-                       "(other colour, own colour r+w, own rhs, cc: 24 B/cell)" % kname if split
+                       "(other colour, own colour r+w, own rhs: 16 B/cell; u stays in L2 between passes)" % kname if split
                        else "%s: finest-level relax, 2 red-black FP64 colour passes (u r+w, a, b, c, rhs: "
                             "48 B/cell)" % kname),
             "achieved": achieved, "peak": peak, "unit": "GB/s",
