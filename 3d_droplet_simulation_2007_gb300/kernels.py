@@ -6,11 +6,14 @@ point of include/dsg.h with the reference subroutine's argument list.  torch
 supplies device memory and the current stream only; the kernels are
 ``libdsg.so``'s.
 """
+import functools
+
 import numpy as np
 
 from . import _lib
 
 
+@functools.lru_cache(maxsize=None)
 def _torch():
     import torch
     return torch
@@ -27,20 +30,35 @@ def to_host(t, shape):
     return t.detach().cpu().numpy().reshape(shape, order="F")
 
 
+@functools.lru_cache(maxsize=None)
+def _binding():
+    """The library, torch's float64 and a function for the current stream's
+    handle on the current device: on small grids a call is bound by the host,
+    so that what does not change between calls is looked up once (a two-grid
+    cycle of 30 calls at 32^3: 137 us, 216 with the lookups in every call)."""
+    torch = _torch()
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or device is None:
+        return _lib.load(), torch.float64, lambda: torch.cuda.current_stream().cuda_stream
+    torch.cuda.init()
+    return _lib.load(), torch.float64, lambda: raw(device())
+
+
 def _stream():
-    return _torch().cuda.current_stream().cuda_stream
+    return _binding()[2]()
 
 
 def _p(t):
     if t is None:
         return None
-    assert t.is_cuda and t.dtype == _torch().float64 and t.is_contiguous()
+    assert t.is_cuda and t.dtype is _binding()[1] and t.is_contiguous()
     return t.data_ptr()
 
 
 def _call(name, *args):
-    lib = _lib.load()
-    _lib.check(getattr(lib, name)(*args))
+    rc = getattr(_binding()[0], name)(*args)
+    if rc != _lib.DSG_OK:
+        _lib.check(rc)
 
 
 def relax(u, lengthsize, rhs, a, b, c, ei, shape, omega):
