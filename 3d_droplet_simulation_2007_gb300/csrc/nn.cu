@@ -408,16 +408,31 @@ __global__ void k_pack_tc(const float *__restrict__ Wt, bf16 *__restrict__ dst, 
 // CTX x CTY x BZ voxels; warp w owns (tap, ci block) pairs w, w+8, ...; for each
 // pair it accumulates a 16 (ci) x COUT tile over the brick with A = X^T and
 // B = G loaded by ldmatrix.trans, then adds it to dW with atomics.
+//
+// The deep layers have few bricks (8^3 voxels: two) and many pairs, so a brick's
+// pairs are dealt out over up to `parts` CTAs, as many as give the GPU about two
+// each.  A voxel's 16-byte chunks are permuted by its index, which puts the eight
+// rows of an ldmatrix into eight different bank groups (in order, 64 channels
+// put them into one).  64 -> 64 channels at 8^3: 310 us without the two, 17
+// with; 32 -> 64 at 16^3 149 and 18; 16 -> 16 at 64^3 45 and 38.
 constexpr int BZ = 4;
+
+// Chunk c of voxel v, of CHUNKS chunks.
+template <int CHUNKS>
+__device__ __forceinline__ int chunk_at(int v, int c) {
+  return v * CHUNKS + (c ^ ((v / (8 / CHUNKS)) & (CHUNKS - 1)));
+}
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(256) k_conv3_wgrad(const bf16 *__restrict__ X, const bf16 *__restrict__ G,
-                                                     float *__restrict__ dW, int W, int H, int D) {
+                                                     float *__restrict__ dW, int W, int H, int D, int parts) {
+  static_assert(CIN >= 16 && CIN <= 64 && COUT >= 16 && COUT <= 64, "two to eight chunks per voxel");
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int HX = CTX + 2, HY = CTY + 2, HZ = BZ + 2;
   bf16 *xt = reinterpret_cast<bf16 *>(smem);               // [HZ][HY][HX][CIN]
   bf16 *gt = xt + (size_t)HZ * HY * HX * CIN;               // [BZ][CTY][CTX][COUT]
-  const int x0 = blockIdx.x * CTX, y0 = blockIdx.y * CTY, z0 = blockIdx.z * BZ;
+  const int part = (int)blockIdx.x % parts;
+  const int x0 = (int)blockIdx.x / parts * CTX, y0 = blockIdx.y * CTY, z0 = blockIdx.z * BZ;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   {
     constexpr int VPV = CIN / 8;
@@ -429,7 +444,7 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad(const bf16 *__restrict__ X,
       uint4 val = make_uint4(0u, 0u, 0u, 0u);
       if (gx >= 0 && gx < W && gy >= 0 && gy < H && gz >= 0 && gz < D)
         val = reinterpret_cast<const uint4 *>(X + (((size_t)gz * H + gy) * W + gx) * CIN)[c8];
-      reinterpret_cast<uint4 *>(xt + (size_t)v * CIN)[c8] = val;
+      reinterpret_cast<uint4 *>(xt)[chunk_at<VPV>(v, c8)] = val;
     }
     constexpr int GPV = COUT / 8;
     const int ngv = BZ * CTY * CTX * GPV;
@@ -439,7 +454,7 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad(const bf16 *__restrict__ X,
       const int gx = x0 + bx, gy = y0 + by, gz = z0 + bz;
       uint4 val = make_uint4(0u, 0u, 0u, 0u);
       if (gx < W && gy < H && gz < D) val = reinterpret_cast<const uint4 *>(G + (((size_t)gz * H + gy) * W + gx) * COUT)[c8];
-      reinterpret_cast<uint4 *>(gt + (size_t)v * COUT)[c8] = val;
+      reinterpret_cast<uint4 *>(gt)[chunk_at<GPV>(v, c8)] = val;
     }
   }
   __syncthreads();
@@ -451,7 +466,7 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad(const bf16 *__restrict__ X,
   // B = G (16 voxels x 8 co): stored rows are voxels with co contiguous; the
   // col-major B fragment is ldmatrix.trans of blocks (v 0-7) and (v 8-15).
   const int lrow = lane & 7, lmat = lane >> 3;
-  for (int pr = warp; pr < npairs; pr += 8) {
+  for (int pr = warp + 8 * part; pr < npairs; pr += 8 * parts) {
     const int tap = pr / KB, kb = pr % KB;
     const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
     float acc[COUT / 8][4];
@@ -461,16 +476,16 @@ __global__ void __launch_bounds__(256) k_conv3_wgrad(const bf16 *__restrict__ X,
       for (int by = 0; by < CTY; by++) {
         // the 16 voxels of this k-step: x = 0..15 of row (by, bz)
         const int av = lrow + ((lmat >> 1) << 3);        // voxel index for this lane's A row address
-        const int ach = kb * 16 + ((lmat & 1) << 3);     // ci offset
+        const int ach = kb * 2 + (lmat & 1);              // ci chunk
         const int hv = ((bz + dz) * HY + (by + dy)) * HX + (av + dx);
         unsigned a0, a1, a2, a3;
-        ldmatrix_x4_trans(a0, a1, a2, a3, smem_u32(xt + (size_t)hv * CIN + ach));
+        ldmatrix_x4_trans(a0, a1, a2, a3, smem_u32(xt + 8 * chunk_at<CIN / 8>(hv, ach)));
         const int gvrow = (bz * CTY + by) * CTX;
 #pragma unroll
         for (int n = 0; n < COUT / 8; n++) {
           const int bvox = (lane & 15);
           unsigned b0, b1;
-          ldmatrix_x2_trans(b0, b1, smem_u32(gt + (size_t)(gvrow + bvox) * COUT + n * 8));
+          ldmatrix_x2_trans(b0, b1, smem_u32(gt + 8 * chunk_at<COUT / 8>(gvrow + bvox, n)));
           mma_bf16(acc[n], a0, a1, a2, a3, b0, b1);
         }
       }
@@ -1005,8 +1020,11 @@ cudaError_t wgrad_launch(const bf16 *X, const bf16 *G, float *dW, int W, int H, 
   static const cudaError_t attr =
       cudaFuncSetAttribute(k_conv3_wgrad<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (attr != cudaSuccess) return attr;
-  const dim3 grid((unsigned)((W + CTX - 1) / CTX), (unsigned)((H + CTY - 1) / CTY), (unsigned)((D + BZ - 1) / BZ));
-  DSG_COUNT k_conv3_wgrad<CIN, COUT><<<grid, 256, smem, st>>>(X, G, dW, W, H, D);
+  dim3 grid((unsigned)((W + CTX - 1) / CTX), (unsigned)((H + CTY - 1) / CTY), (unsigned)((D + BZ - 1) / BZ));
+  const unsigned bricks = grid.x * grid.y * grid.z, most = (27 * CIN / 16 + 7) / 8;
+  const unsigned parts = bricks >= 152 ? 1 : (304 / bricks < most ? 304 / bricks : most);
+  grid.x *= parts;
+  DSG_COUNT k_conv3_wgrad<CIN, COUT><<<grid, 256, smem, st>>>(X, G, dW, W, H, D, (int)parts);
   return cudaGetLastError();
 }
 
