@@ -674,8 +674,10 @@ __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, 
   for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvox; v += (size_t)gridDim.x * blockDim.x) {
     const float d = y[v * 8] - t[v];
     s += (double)d * d;
+    // (one by one 22 us at 64^3, 10.7 so)
+    reinterpret_cast<float4 *>(dy)[4 * v] = make_float4(2.f * d / (float)nvox, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int c = 0; c < 16; c++) dy[v * 16 + c] = c == 0 ? 2.f * d / (float)nvox : 0.f;
+    for (int c = 1; c < 4; c++) reinterpret_cast<float4 *>(dy)[4 * v + c] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   sh[threadIdx.x] = s;
   __syncthreads();
@@ -1233,9 +1235,15 @@ int loss_grad(dsg_net *n, cudaStream_t st) {
 
 // x (FP32 host, 3 channels per voxel) -> n->x0 (bf16, 16 channels)
 __global__ void k_input_from_f32(bf16 *__restrict__ x0, const float *__restrict__ x, size_t nvox) {
-  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvox; v += (size_t)gridDim.x * blockDim.x)
+  // a voxel's 16 channels as two 16-byte stores (one by one 27 us at 64^3, 4.6 so)
+  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvox; v += (size_t)gridDim.x * blockDim.x) {
+    uint4 o[2];
+    bf16 *const e = reinterpret_cast<bf16 *>(o);
 #pragma unroll
-    for (int c = 0; c < 16; c++) x0[v * 16 + c] = __float2bfloat16(c < kIn ? x[v * kIn + c] : 0.f);
+    for (int c = 0; c < 16; c++) e[c] = __float2bfloat16(c < kIn ? x[v * kIn + c] : 0.f);
+    reinterpret_cast<uint4 *>(x0)[2 * v] = o[0];
+    reinterpret_cast<uint4 *>(x0)[2 * v + 1] = o[1];
+  }
 }
 
 __global__ void k_output_ch0(float *__restrict__ y, const float *__restrict__ yout, size_t nvox) {
