@@ -124,7 +124,6 @@ void bct(double *const S[6], Dims d, cudaStream_t st, int k0, int k1) {
                                                                                     d, kx0, kx1, k0, k1);
 }
 
-const dim3 kBlk(32, 4, 1);
 
 }  // namespace
 
