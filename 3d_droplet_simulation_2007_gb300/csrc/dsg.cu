@@ -126,8 +126,19 @@ inline bool fp64_fma(const dsg_ctx *ctx) {
   return ctx->cfg.mode == DSG_MODE_TOL_FP64 && ctx->cfg.fp64_exact == 0;
 }
 
+// Whether level l has cooperative phases (the live profile times the finest
+// level's sweeps as launches of their own).
 template <class A>
-bool phases(const dsg_ctx *ctx, const A &level, int l);
+bool has_phases(const dsg_ctx *ctx, const A &level, int l) {
+  return level.g.blocks() > 0 && !(ctx->prof && l == ctx->ng);
+}
+// Whether n sweeps of level l are one.  Without sweeps there is no exchange to
+// order a block's reads of its neighbours' cells before their owners write them
+// (mggrid.cuh), and the transfers run as launches of their own.
+template <class A>
+bool phases(const dsg_ctx *ctx, const A &level, int l, int n) {
+  return n > 0 && has_phases(ctx, level, l);
+}
 
 constexpr long long kShortFormCells = 80000;  // a cooperative phase: 256 cells per colour on each SM
 
@@ -136,7 +147,7 @@ constexpr long long kShortFormCells = 80000;  // a cooperative phase: 256 cells 
 // and the flags lie in the level's FP32 arrays, which only the mixed modes use.
 bool products(const dsg_ctx *ctx, int l, dsg::Products *P) {
   if (ctx->cfg.mode == DSG_MODE_TOL_MIXED || ctx->cfg.mode == DSG_MODE_LEARNED) return false;
-  if (l <= ctx->tail64_top || phases(ctx, ctx->gr64[l], l)) return false;
+  if (l <= ctx->tail64_top || has_phases(ctx, ctx->gr64[l], l)) return false;
   // The fused form rounds differently, so a level has it or not whether the
   // context runs alone or in an ensemble: those that no cluster and no
   // cooperative phase can hold.
@@ -216,7 +227,7 @@ int coarse64(dsg_ctx *ctx, bool fmg) {
   return DSG_OK;
 }
 
-// A smoothing phase of level l in one cooperative launch: n sweeps; down: the
+// A smoothing phase of level l in one cooperative launch: n >= 1 sweeps; down: the
 // residual restricted into level l - 1 at the end; up: level l - 1's correction
 // added (add) or set at the start.
 int phase64(dsg_ctx *ctx, int l, int n, bool down, bool up, bool add) {
@@ -232,21 +243,14 @@ int phase64(dsg_ctx *ctx, int l, int n, bool down, bool up, bool add) {
   G.h2 = h1 * h1;
   G.h2i = 1.0 / (h1 * h1);
   G.omega = ctx->cfg.omega;
-  G.n = n > 0 ? n : 0;
+  G.n = n;
   G.rhs_c = down ? ctx->lv[l - 1][3] : nullptr;
   G.u_c = down ? ctx->lv[l - 1][1] : nullptr;
   G.prolong = up ? ctx->lv[l - 1][1] : nullptr;
   G.add = add ? 1 : 0;
-  G.ghosts = l == ctx->ng && n > 0;
+  G.ghosts = l == ctx->ng;
   DSG_CK(ctx, dsg::grid64(G, fp64_fma(ctx), ctx->stream));
   return DSG_OK;
-}
-
-// Whether level l's phases are cooperative launches (the live profile times
-// the finest level's sweeps as launches of their own).
-template <class A>
-bool phases(const dsg_ctx *ctx, const A &level, int l) {
-  return level.g.blocks() > 0 && !(ctx->prof && l == ctx->ng);
 }
 
 // One V-cycle from level j down to 1 and back (main.f:3705-3759); init: level
@@ -258,9 +262,9 @@ int vcycle(dsg_ctx *ctx, int j, bool init) {
   for (int jj = j; jj >= 2 && jj > jt; jj--) {
     double **L = ctx->lv[jj];
     const Dims d = ctx->level(jj);
-    if (init && jj == j && (jj == ctx->ng || !phases(ctx, ctx->gr64[jj], jj)))
-      DSG_CK(ctx, dsg::interp(L[1], ctx->lv[jj - 1][1], d, st));
-    if (phases(ctx, ctx->gr64[jj], jj)) {
+    const bool phase = phases(ctx, ctx->gr64[jj], jj, ctx->s.npre);
+    if (init && jj == j && (jj == ctx->ng || !phase)) DSG_CK(ctx, dsg::interp(L[1], ctx->lv[jj - 1][1], d, st));
+    if (phase) {
       int rc = phase64(ctx, jj, ctx->s.npre, true, init && jj == j && jj < ctx->ng, false);
       if (rc) return rc;
       continue;
@@ -278,7 +282,8 @@ int vcycle(dsg_ctx *ctx, int j, bool init) {
   for (int jj = jt >= 1 ? jt + 1 : 2; jj <= j; jj++) {
     double **L = ctx->lv[jj];
     const Dims d = ctx->level(jj);
-    if (jj < ctx->ng && phases(ctx, ctx->gr64[jj], jj)) {
+    const bool phase = phases(ctx, ctx->gr64[jj], jj, ctx->s.npost);
+    if (jj < ctx->ng && phase) {
       int rc = phase64(ctx, jj, ctx->s.npost, false, true, true);
       if (rc) return rc;
       continue;
@@ -286,7 +291,7 @@ int vcycle(dsg_ctx *ctx, int j, bool init) {
     // the finest level's residual array keeps addint's values: its ghosts
     // are read in the next step's momentum phase
     DSG_CK(ctx, dsg::addint(L[1], ctx->lv[jj - 1][1], jj == ctx->ng ? L[2] : nullptr, d, st));
-    if (phases(ctx, ctx->gr64[jj], jj)) {
+    if (phase) {
       int rc = phase64(ctx, jj, ctx->s.npost, false, false, false);
       if (rc) return rc;
       continue;
@@ -436,7 +441,7 @@ int phase32(dsg_ctx *ctx, int l, int n, bool down, bool up, bool add) {
   G.h2 = level_h2(ctx, l);
   G.h2i = 1.0f / level_h2(ctx, l);
   G.omega = omega32(ctx);
-  G.n = n > 0 ? n : 0;
+  G.n = n;
   G.rhs_c = down ? ctx->lv32[l - 1][RHS32] : nullptr;
   G.u_c = down ? ctx->lv32[l - 1][U32] : nullptr;
   G.prolong = up ? ctx->lv32[l - 1][U32] : nullptr;
@@ -458,7 +463,7 @@ int vcycle32(dsg_ctx *ctx, int j, bool init) {
     float **L = ctx->lv32[jj];
     float **Lc = ctx->lv32[jj - 1];
     const bool set = init && jj == j;
-    if (phases(ctx, ctx->gr32[jj], jj)) {
+    if (phases(ctx, ctx->gr32[jj], jj, pre32(ctx, jj))) {
       int rc = phase32(ctx, jj, pre32(ctx, jj), true, set, false);
       if (rc) return rc;
       continue;
@@ -484,7 +489,7 @@ int vcycle32(dsg_ctx *ctx, int j, bool init) {
     DSG_CK(ctx, relax32_level(ctx, ctx->s.ntop, 1));
   }
   for (int jj = jt >= 1 ? jt + 1 : 2; jj <= j; jj++) {
-    if (phases(ctx, ctx->gr32[jj], jj)) {
+    if (phases(ctx, ctx->gr32[jj], jj, post32(ctx, jj))) {
       int rc = phase32(ctx, jj, post32(ctx, jj), false, true, true);
       if (rc) return rc;
       continue;
