@@ -301,6 +301,70 @@ int vcycle(dsg_ctx *ctx, int j, bool init) {
   return DSG_OK;
 }
 
+// One V-cycle of levels j .. 1 pass by pass with the sweeps of the last cluster
+// launch, every array written as main.f:3703-3759 does.
+int plain_vcycle(dsg_ctx *ctx, int j) {
+  const double ls = ctx->s.lengthsize, om = ctx->cfg.omega;
+  const bool fma = fp64_fma(ctx);
+  const dsg::mgc::Args<double> &G = ctx->cl64;
+  cudaStream_t st = ctx->stream;
+  auto sweeps = [&](int n, int l) {
+    double **L = ctx->lv[l];
+    return dsg::relax_n(n, L[1], ls, L[3], L[4], L[5], L[6], L[7], ctx->level(l), om, st, fma);
+  };
+  for (int l = j; l >= 2; l--) {
+    double **L = ctx->lv[l], **C = ctx->lv[l - 1];
+    const Dims dc = ctx->level(l - 1);
+    DSG_CK(ctx, sweeps(G.lv[l].npre, l));
+    DSG_CK(ctx, dsg::resid(ls, L[2], L[1], L[3], L[4], L[5], L[6], ctx->level(l), st, fma));
+    DSG_CK(ctx, dsg::rstrct(C[3], L[2], dc, st));
+    DSG_CK(ctx, dsg::fill_zero(C[1], dc.count(), st));
+  }
+  DSG_CK(ctx, sweeps(G.ntop, 1));
+  for (int l = 2; l <= j; l++) {
+    double **L = ctx->lv[l];
+    DSG_CK(ctx, dsg::addint(L[1], ctx->lv[l - 1][1], L[2], ctx->level(l), st));
+    DSG_CK(ctx, sweeps(G.lv[l].npost, l));
+  }
+  return DSG_OK;
+}
+
+// p, res and rhs of the levels below the finest as the reference's schedule
+// leaves them, for callers of dsg_level_ptr.  A solve leaves less behind: what a
+// cluster launch forms stays in its shared memory, and the other levels below
+// the finest have neither ghosts nor the residual array's last values.  The last
+// cluster launch, a function of arrays that are still there, is repeated pass
+// by pass.
+int complete_levels(dsg_ctx *ctx) {
+  const dsg::mgc::Args<double> &G = ctx->cl64;
+  const int top = ctx->tail64_top;
+  cudaStream_t st = ctx->stream;
+  ctx->levels_pending = false;
+  for (int l = top > 0 ? top : 1; l < ctx->ng; l++) DSG_CK(ctx, dsg::bc_scalar(ctx->lv[l][3], ctx->level(l), st));
+  if (top > 0 && G.fmg) {
+    double **L = ctx->lv[1];
+    DSG_CK(ctx, dsg::fill_zero(L[1], ctx->level(1).count(), st));
+    DSG_CK(ctx, dsg::relax_n(G.ntop, L[1], ctx->s.lengthscale, L[3], L[4], L[5], L[6], L[7], ctx->level(1),
+                             ctx->cfg.omega, st, fp64_fma(ctx)));
+    for (int l = 2; l <= top; l++) {
+      DSG_CK(ctx, dsg::interp(ctx->lv[l][1], ctx->lv[l - 1][1], ctx->level(l), st));
+      for (int c = 0; c < G.lv[l].cycles; c++) {
+        int rc = plain_vcycle(ctx, l);
+        if (rc) return rc;
+      }
+    }
+  } else if (top > 0) {
+    DSG_CK(ctx, dsg::fill_zero(ctx->lv[top][1], ctx->level(top).count(), st));
+    int rc = plain_vcycle(ctx, top);
+    if (rc) return rc;
+  }
+  for (int l = top + 1; l < ctx->ng; l++) {
+    DSG_CK(ctx, dsg::bc_scalar(ctx->lv[l][1], ctx->level(l), st));
+    if (l >= 2 && ctx->levels_cycled) DSG_CK(ctx, dsg::interp(ctx->lv[l][2], ctx->lv[l - 1][1], ctx->level(l), st));
+  }
+  return DSG_OK;
+}
+
 int relres_host(dsg_ctx *ctx, double *out) {
   double **L = ctx->lv[ctx->ng];
   DSG_CK(ctx, dsg::relres_sums(ctx->red_out, ctx->red_partials, ctx->s.lengthsize, L[1], L[3], L[4], L[5],
@@ -908,6 +972,7 @@ int mglin(dsg_ctx *ctx, dsg_mg_stats *stats) {
     if (rc) return rc;
     return dsg::mixed_finish(ctx, &s, stats);
   }
+  ctx->levels_pending = false;
   for (int g = ng - 1; g >= 1; g--) {
     const Dims dc = ctx->level(g);
     DSG_CK(ctx, dsg::rstrct(ctx->lv[g][3], ctx->lv[g + 1][3], dc, st));
@@ -973,6 +1038,12 @@ int mglin(dsg_ctx *ctx, dsg_mg_stats *stats) {
   }
   s.fine_sweeps = fine_sweeps;
   if (stats) *stats = s;
+  ctx->levels_pending = true;
+  ctx->levels_cycled = ctx->cfg.cycles > 0 || s.vcycles > 0;
+  if (ctx->levels_wanted) {
+    int rc = complete_levels(ctx);
+    if (rc) return rc;
+  }
   if (ctx->cfg.mode == DSG_MODE_TOL_FP64 && !s.converged)
     return dsg::set_error(ctx, DSG_E_NOT_CONVERGED, "multigrid reached %d V-cycles at relres %.3e > tol %.3e",
                           s.vcycles, s.relres, ctx->cfg.tol);
@@ -1261,6 +1332,14 @@ int dsg_download(dsg_ctx *ctx, int field, double *host) {
 int dsg_level_ptr(dsg_ctx *ctx, int field, int level, double **dev, int *nx, int *ny, int *nz) {
   if (!ctx || field < 0 || field > 7 || level < 1 || level > ctx->ng || !dev)
     return dsg::set_error(ctx, DSG_E_ARG, "bad level field");
+  if (level < ctx->ng && field >= DSG_F_P && field <= DSG_F_RHS) {
+    ctx->levels_wanted = true;
+    if (ctx->levels_pending) {
+      int rc = complete_levels(ctx);
+      if (rc) return rc;
+      DSG_CK(ctx, cudaStreamSynchronize(ctx->stream));
+    }
+  }
   *dev = ctx->lv[level][field];
   if (nx) *nx = ctx->lnx[level];
   if (ny) *ny = ctx->lny[level];

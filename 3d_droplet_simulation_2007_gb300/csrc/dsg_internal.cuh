@@ -440,6 +440,10 @@ struct dsg_ctx {
   unsigned char *node_flags[32];  // uniform cells of a level below the finest with phases of mgbox.cuh
   int lnx[32], lny[32], lnz[32];
   double *lv[32][8];          // [level][CC,P,RES,RHS,A,B,C,EI], level 1..ng
+  // P, RES and RHS of the FP64 levels below the finest: a caller holds pointers
+  // to them, so that every solve completes them; the last solve has not; it ran
+  // a V-cycle from the finest level
+  bool levels_wanted = false, levels_pending = false, levels_cycled = false;
   float *lv32[32][6];         // FP32 hierarchy [level][U,RHS,A,B,C,EI] of the mixed mode;
                               // on the finest level U and RHS are colour-split (even half, odd
                               // half) and A holds cc in FP32

@@ -162,7 +162,12 @@ int64_t dsg_device_bytes(const dsg_ctx *ctx);
 /* Copy a fine field (nx*ny*nz doubles, column-major) host <-> device. */
 int dsg_upload(dsg_ctx *ctx, int field, const double *host);
 int dsg_download(dsg_ctx *ctx, int field, double *host);
-/* Device pointer of a level array (field DSG_F_CC..DSG_F_EI, level 1..ng). */
+/* Device pointer of a level array (field DSG_F_CC..DSG_F_EI, level 1..ng).
+ * A solve of the FP64 modes keeps much of P, RES and RHS below the finest level
+ * on the chip; the first call for one of them completes the arrays of the last
+ * solve (and waits for that), and from then on every solve of the context
+ * completes them itself, as mglin's schedule leaves them.  That costs one
+ * V-cycle of the coarse levels in a launch per pass. */
 int dsg_level_ptr(dsg_ctx *ctx, int field, int level, double **dev_ptr, int *nx, int *ny, int *nz);
 int dsg_field_ptr(dsg_ctx *ctx, int field, double **dev_ptr);
 int dsg_get_scalars(const dsg_ctx *ctx, dsg_scalars *out);
