@@ -1434,7 +1434,14 @@ void sweep_order(int tswap, int order[3]) {
 
 extern "C" {
 
-int dsg_vofmethod(dsg_ctx *ctx) {
+int dsg_vofmethod(dsg_ctx *ctx) { return dsg::vof_phase(ctx, true); }
+
+}  // extern "C"
+
+// VOFmethod; whole: with the flux arrays (EI, RES and RHS, the scratch that the
+// reference passes) as its last sweep leaves them, which a whole step overwrites
+// before reading.
+int dsg::vof_phase(dsg_ctx *ctx, bool whole) {
   if (!ctx) return DSG_E_ARG;
   dsg_scalars &s = ctx->s;
   const Dims d = ctx->fine();
@@ -1448,7 +1455,7 @@ int dsg_vofmethod(dsg_ctx *ctx) {
     int rc = sync_point(ctx, SP_SWEEP1 + q);
     if (rc) return rc;
     DSG_CK(ctx, dsg::swp(vel[order[q]], cc, s1, s2, s3, order[q], d, s.tauh, reinterpret_cast<unsigned *>(ctx->ccf),
-                         ctx->iface_count, ctx->stream));
+                         ctx->iface_count, ctx->stream, whole));
   }
   DSG_CK(ctx, dsg::bc_c(cc, d, ctx->stream));
   // turbulent diffusion of the volume fraction (main.f:820)
@@ -1458,6 +1465,8 @@ int dsg_vofmethod(dsg_ctx *ctx) {
                            ctx->stream));
   return DSG_OK;
 }
+
+extern "C" {
 
 // kepsmodel (main.f:39-40): the new values go through the pressure and
 // residual arrays, the scratch the reference passes.
@@ -1699,7 +1708,7 @@ int step_phases(dsg_ctx *ctx, int t, dsg_mg_stats *stats) {
 int dsg::step_pre_solve(dsg_ctx *ctx, int t) {
   (void)t;
   DSG_CK(ctx, phase_mark(ctx, 0));
-  int rc = dsg_vofmethod(ctx);
+  int rc = dsg::vof_phase(ctx, false);
   if (rc) return rc;
   if (ctx->cfg.hswitch == 1) {
     rc = dsg_calch3d(ctx);

@@ -250,9 +250,10 @@ cudaError_t fill_zero(double *f, size_t n, cudaStream_t st);
 // vof.cu
 cudaError_t bc_c(double *cc, Dims d, cudaStream_t st);
 // list/count: scratch of the interface-cell list and the cells' bits (a fine
-// field) and the list's length, zero before the call and after it
+// field) and the list's length, zero before the call and after it; whole: all of
+// the flux arrays are written, as swp does, and not only where c is not zero
 cudaError_t swp(const double *us, double *cc, double *vof1, double *vof2, double *vof3, int dir, Dims d,
-                double tauh, unsigned *list, unsigned *count, cudaStream_t st);
+                double tauh, unsigned *list, unsigned *count, cudaStream_t st, bool whole);
 cudaError_t calcrho(double *rhon, double *mun, const double *cc, Dims d, double rho1, double rho2,
                     double mu1, double mu2, cudaStream_t st);
 // csf.cu (S = {S11,S22,S33,S12,S13,S23})
@@ -409,7 +410,9 @@ void net_begin_solve(dsg_net *n);
 
 struct dsg_ctx;
 namespace dsg {
-// dsg.cu: the surface-tension phase (dsg_csf with scratch = true)
+// dsg.cu: the VOF phase (dsg_vofmethod with whole = true) and the
+// surface-tension phase (dsg_csf with scratch = true)
+int vof_phase(dsg_ctx *ctx, bool whole);
 int csf_phase(dsg_ctx *ctx, bool scratch);
 }  // namespace dsg
 

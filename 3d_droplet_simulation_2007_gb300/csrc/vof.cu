@@ -346,6 +346,22 @@ __global__ void k_swp_update(double *__restrict__ cc, const double *__restrict__
   }
 }
 
+// The parts of the flux arrays that a sweep neither writes nor reads, for callers
+// that see the arrays: all of the interior (the sweep then writes the cells that
+// are not empty) and the faces of bc_flux, main.f:4496-4539.
+template <int D>
+__global__ void k_zero_fluxes(double *__restrict__ vof1, double *__restrict__ vof2, double *__restrict__ vof3, Dims d) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
+  const int k = blockIdx.z + 2;
+  if (i > d.nx - 1 || j > d.ny - 1) return;
+  const size_t q = d.ix(i, j, k), sd = D == 1 ? 1 : (D == 2 ? d.sy() : d.sz());
+  const int m = D == 1 ? i : (D == 2 ? j : k), n = D == 1 ? d.nx : (D == 2 ? d.ny : d.nz);
+  vof1[q] = vof2[q] = vof3[q] = 0.0;
+  if (m == 2) vof3[q - sd] = 0.0;
+  if (m == n - 1) vof1[q + sd] = 0.0;
+}
+
 // bc_c (main.f:4340-4395 without the dead filter block).  Its three ordered
 // steps -- x: plane 2 = plane 1, plane nx = plane nx-1; y: ghosts of i in
 // 2..nx-1 (the lower one clipped); z: likewise over all j -- in one launch: a
@@ -421,7 +437,8 @@ const dim3 kBlk(32, 4, 1);
 
 template <int D>
 void sweep(const double *us, double *cc, double *v1, double *v2, double *v3, Dims d, double tauh, unsigned *list,
-           unsigned *count, cudaStream_t st) {
+           unsigned *count, cudaStream_t st, bool whole) {
+  if (whole) DSG_COUNT k_zero_fluxes<D><<<interior_grid(d, kBlk), kBlk, 0, st>>>(v1, v2, v3, d);
   unsigned *bits = list + (size_t)(d.nx - 2) * (d.ny - 2) * (d.nz - 2);
   const int wpr = words_per_row(d), rows = 4 * kScanRows;
   DSG_COUNT k_swp_scan<D><<<dim3((unsigned)wpr, (unsigned)((d.ny - 2 + rows - 1) / rows), (unsigned)(d.nz - 2)), kBlk,
@@ -448,10 +465,10 @@ cudaError_t bc_c(double *cc, Dims d, cudaStream_t st) {
 }
 
 cudaError_t swp(const double *us, double *cc, double *vof1, double *vof2, double *vof3, int dir, Dims d,
-                double tauh, unsigned *list, unsigned *count, cudaStream_t st) {
-  if (dir == 1) sweep<1>(us, cc, vof1, vof2, vof3, d, tauh, list, count, st);
-  else if (dir == 2) sweep<2>(us, cc, vof1, vof2, vof3, d, tauh, list, count, st);
-  else sweep<3>(us, cc, vof1, vof2, vof3, d, tauh, list, count, st);
+                double tauh, unsigned *list, unsigned *count, cudaStream_t st, bool whole) {
+  if (dir == 1) sweep<1>(us, cc, vof1, vof2, vof3, d, tauh, list, count, st, whole);
+  else if (dir == 2) sweep<2>(us, cc, vof1, vof2, vof3, d, tauh, list, count, st, whole);
+  else sweep<3>(us, cc, vof1, vof2, vof3, d, tauh, list, count, st, whole);
   return bc_c(cc, d, st);
 }
 
