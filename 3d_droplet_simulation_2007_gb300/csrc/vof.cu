@@ -237,7 +237,8 @@ constexpr int kScanRows = 4;  // rows a warp scans, all loaded before the first 
 // Sweep, pass 1: the bits, the fluxes of full cells (the reference's c == 1
 // branch; zero for values that are neither positive nor +0) and the list of
 // interface cells (one atomic per warp), so that the PLIC geometry runs on
-// full warps instead of one busy lane per warp.
+// full warps instead of one busy lane per warp.  Also bc_flux's zeros beyond the
+// upper face along D: vof1 is EI, whose ghosts nothing else in a step writes.
 template <int D>
 __global__ void k_swp_scan(const double *__restrict__ us, const double *__restrict__ cc, double *__restrict__ vof1,
                            double *__restrict__ vof2, double *__restrict__ vof3, Dims d, double tauh,
@@ -258,6 +259,9 @@ __global__ void k_swp_scan(const double *__restrict__ us, const double *__restri
     some |= any;
     if (lane == 0 && j0 + r <= d.ny - 1)
       bits[((size_t)(k - 2) * (d.ny - 2) + (j0 + r - 2)) * words_per_row(d) + blockIdx.x] = any;
+    if (i <= d.nx - 1 && j0 + r <= d.ny - 1 &&
+        (D == 1 ? i == d.nx - 1 : (D == 2 ? j0 + r == d.ny - 1 : k == d.nz - 1)))
+      vof1[d.ix(i, j0 + r, k) + (D == 1 ? 1 : (D == 2 ? d.sy() : d.sz()))] = 0.0;
   }
   if (!some) return;
   unsigned base = 0;
@@ -348,7 +352,7 @@ __global__ void k_swp_update(double *__restrict__ cc, const double *__restrict__
 
 // The parts of the flux arrays that a sweep neither writes nor reads, for callers
 // that see the arrays: all of the interior (the sweep then writes the cells that
-// are not empty) and the faces of bc_flux, main.f:4496-4539.
+// are not empty) and bc_flux's zeros beyond the lower face (main.f:4496-4539).
 template <int D>
 __global__ void k_zero_fluxes(double *__restrict__ vof1, double *__restrict__ vof2, double *__restrict__ vof3, Dims d) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
@@ -356,10 +360,8 @@ __global__ void k_zero_fluxes(double *__restrict__ vof1, double *__restrict__ vo
   const int k = blockIdx.z + 2;
   if (i > d.nx - 1 || j > d.ny - 1) return;
   const size_t q = d.ix(i, j, k), sd = D == 1 ? 1 : (D == 2 ? d.sy() : d.sz());
-  const int m = D == 1 ? i : (D == 2 ? j : k), n = D == 1 ? d.nx : (D == 2 ? d.ny : d.nz);
   vof1[q] = vof2[q] = vof3[q] = 0.0;
-  if (m == 2) vof3[q - sd] = 0.0;
-  if (m == n - 1) vof1[q + sd] = 0.0;
+  if ((D == 1 ? i : (D == 2 ? j : k)) == 2) vof3[q - sd] = 0.0;
 }
 
 // bc_c (main.f:4340-4395 without the dead filter block).  Its three ordered
