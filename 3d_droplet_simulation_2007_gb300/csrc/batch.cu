@@ -900,17 +900,20 @@ int time_probe(BatchSolve *b, int reps, float *ms) {
 // ---- entry points used by ensemble.cu ------------------------------------------
 
 // Whether ctx can take part in a batched solve: the mixed mode with the FP32
-// full-multigrid start, no network, CUDA graphs on, the coarse tail on and an
-// even interior x extent.
+// full-multigrid start, no network, CUDA graphs on, an even interior x extent,
+// and the coarse tail on with a coarsest level that one block can be expected
+// to run: tail_nodes nodes, or 18^3.  (What a context of its own runs in a
+// cluster does not matter here: a batch has its own tail.)
 int batch_eligible(const dsg_ctx *c, char *why, size_t nwhy) {
   const char *r = nullptr;
+  const long long nodes = (long long)c->lnx[1] * c->lny[1] * c->lnz[1],
+                  tail = c->cfg.tail_nodes == 0 ? kSmallLevelNodes : c->cfg.tail_nodes;
   if (c->cfg.mode != DSG_MODE_TOL_MIXED) r = "pressure mode is not DSG_MODE_TOL_MIXED";
   else if (c->net) r = "a network is attached";
   else if (c->cfg.warm_start != 0) r = "the initial guess is not the FP32 full multigrid";
   else if (!c->cfg.use_graphs) r = "CUDA graphs are off";
-  else if (c->tail_top < 1) r = "the coarse tail is off";
+  else if (c->ng < 2 || nodes > tail) r = "the coarse tail is off";
   else if ((c->nx - 2) & 1) r = "odd interior x extent";
-  else if (c->ng < 2) r = "a single multigrid level";
   if (r && why) snprintf(why, nwhy, "%s", r);
   return r ? DSG_E_ARG : DSG_OK;
 }

@@ -362,7 +362,8 @@ int dsg_ensemble_plan(const double *cost, int n, int workers, int *assign);
  * member after its solve; the groups of different workers overlap on the
  * GPU.  Every member's results are bit for bit those of its own dsg_step.
  * Needs every member in DSG_MODE_TOL_MIXED with the FP32 full-multigrid
- * start, CUDA graphs and the coarse tail on, no network attached (DSG_E_ARG
+ * start, CUDA graphs and the coarse tail on (a coarsest level of at most
+ * tail_nodes nodes, or 18^3 for 0), no network attached (DSG_E_ARG
  * otherwise), and at most 128 members per group.  groups = 0 returns to
  * per-member solves.  mglin
  * main.f:3645-3763 per member.  dsg_ensemble_batched: the group count. */
