@@ -420,13 +420,14 @@ constexpr int BZ = 4;
 // Chunk c of voxel v, of CHUNKS chunks.
 template <int CHUNKS>
 __device__ __forceinline__ int chunk_at(int v, int c) {
+  // the exclusive or stays within the voxel for a power of two alone
+  static_assert(CHUNKS == 2 || CHUNKS == 4 || CHUNKS == 8, "16, 32 or 64 channels");
   return v * CHUNKS + (c ^ ((v / (8 / CHUNKS)) & (CHUNKS - 1)));
 }
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(256) k_conv3_wgrad(const bf16 *__restrict__ X, const bf16 *__restrict__ G,
                                                      float *__restrict__ dW, int W, int H, int D, int parts) {
-  static_assert(CIN >= 16 && CIN <= 64 && COUT >= 16 && COUT <= 64, "two to eight chunks per voxel");
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int HX = CTX + 2, HY = CTY + 2, HZ = BZ + 2;
   bf16 *xt = reinterpret_cast<bf16 *>(smem);               // [HZ][HY][HX][CIN]
