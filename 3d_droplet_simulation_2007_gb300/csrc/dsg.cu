@@ -437,10 +437,7 @@ cudaError_t relax32_level(dsg_ctx *ctx, int n, int l) {
     if (r != cudaSuccess) return r;
     ctx->prof_used += 2;
     ctx->prof_relax_calls += n;
-    // colour-split sweep: per colour pass the other colour (half), own colour
-    // read+write (half each) and own rhs (half): 4 FP32 words per cell; cc, which
-    // only cells near the interface read, is not counted
-    ctx->prof_relax_bytes += (double)n * 4.0 * sizeof(float) * (double)d.count();
+    ctx->prof_relax_bytes += n * dsg::relax32_split_bytes(d);
     ctx->prof_relax_bits = 32;
   }
   return e;
@@ -652,7 +649,7 @@ int graph_run(dsg_ctx *ctx, GraphRec &g) {
       DSG_CK(ctx, cudaEventElapsedTime(&x, g.ev[2 * q], g.ev[2 * q + 1]));
       ctx->prof_graph_relax_ms += x;
       ctx->prof_relax_calls += g.ev_n[q];
-      ctx->prof_relax_bytes += (double)g.ev_n[q] * 4.0 * sizeof(float) * (double)ctx->fine().count();
+      ctx->prof_relax_bytes += g.ev_n[q] * dsg::relax32_split_bytes(ctx->fine());
       ctx->prof_relax_bits = 32;
     }
   }

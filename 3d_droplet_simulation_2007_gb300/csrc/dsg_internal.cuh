@@ -347,6 +347,7 @@ cudaError_t grid64(const mgg::Args<double> &args, bool fma, cudaStream_t st);
 cudaError_t relax32_split_n(int n, float *const u[2], float *const rhs[2], const float *cc,
                             const unsigned char *flags, Dims d, float h2, float omega, float r1, float r2,
                             cudaStream_t st);
+double relax32_split_bytes(Dims d);  // algorithmic bytes of one of its sweeps
 cudaError_t resid_restrict32_split(float *rhs_c, float *u_c, float *const u[2], float *const rhs[2], const float *cc,
                                    const unsigned char *flags, Dims df, float h2i, float r1, float r2,
                                    cudaStream_t st);

@@ -489,6 +489,14 @@ cudaError_t relax32_split_n(int n, float *const u[2], float *const rhs[2], const
   return cudaGetLastError();
 }
 
+// Per colour pass the other colour (half), own colour read and written (half
+// each) and own right-hand side (half): four words per cell, and where no
+// segment is known to be uniform cc in both passes: two more.
+double relax32_split_bytes(Dims d) {
+  const bool vec = split_vec(Split{(d.nx - 2) >> 1, d.ny - 2, d.nz - 2});
+  return (vec ? 4.0 : 6.0) * sizeof(float) * (double)d.count();
+}
+
 cudaError_t resid_restrict32_split(float *rhs_c, float *u_c, float *const u[2], float *const rhs[2], const float *cc,
                                    const unsigned char *flags, Dims df, float h2i, float r1, float r2,
                                    cudaStream_t st) {

@@ -220,7 +220,9 @@ typedef struct dsg_profile {
   int64_t launches;    /* library kernel launches since dsg_profile_enable */
   int64_t relax_calls; /* finest-level relax calls timed with CUDA events */
   double relax_ms;     /* summed event time of those calls */
-  double relax_bytes;  /* their algorithmic bytes: 6 words (u r+w, a, b, c, rhs) per cell */
+  double relax_bytes;  /* their algorithmic bytes.  FP64: 6 words per cell (u r+w, a, b, c, rhs), an upper
+                          bound where warps lie in one fluid and read no coefficients.  FP32: 4 words (u r+w,
+                          the other colour, rhs) on grids whose uniform segments need no cc, else 6 */
   int relax_bits;      /* word size of the timed relax: 64 (FP64 modes) or 32 (mixed modes) */
   /* CUDA-event time of the phases of dsg_step: 0 VOF advection, 1 CFL check,
    * 2 CSF force, 3 momentum up to the divergence, 4 pressure solve,
