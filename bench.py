@@ -321,27 +321,30 @@ def run_reference(args):
 
 
 def relax_roofline(prof, step_ms, n):
-    """Roofline entry of the finest-level relax from the live CUDA-event
-    profile: algorithmic bytes per call / mean call time against the measured
-    HBM copy bandwidth."""
+    """Roofline entry of the finest-level relax from the live CUDA-event profile.
+    FP32 sweep: u stays in L2 between the passes, so its algorithmic bytes per
+    call time are a rate through L2 (l2_gbs); what is compared with the measured
+    HBM copy bandwidth is the committed DRAM traffic of a call.  FP64 sweep, at
+    the FP64 pipe's rate: algorithmic bytes, an upper bound of what it moves."""
     peak, peak_kind = measured_peaks()
-    achieved = None
-    if prof["relax_calls"]:
-        per_call_ms = prof["relax_ms"] / prof["relax_calls"]
-        per_call_bytes = prof["relax_bytes"] / prof["relax_calls"]
-        achieved = per_call_bytes / (per_call_ms / 1e3) / 1e9
     split = prof.get("relax_bits") == 32
     kname = "k_relax32_split" if split else "k_relax_colour"
-    return {"bound": "hbm",
-            "kernel": ("%s: finest-level relax, colour-split FP32 red-black sweep, 2 launches per relax "
-                       "(other colour, own colour r+w, own rhs: 16 B/cell; u stays in L2 between passes)" % kname if split
-                       else "%s: finest-level relax, 2 red-black FP64 colour passes (u r+w, a, b, c, rhs: "
-                            "48 B/cell)" % kname),
+    traffic = committed_traffic(kname, n)
+    calls = prof["relax_calls"]
+    call_s = prof["relax_ms"] / calls / 1e3 if calls else None
+    call_bytes = prof["relax_bytes"] / calls if calls else None
+    words = call_bytes / (n + 2) ** 3 if calls else 0
+    hbm_bytes = traffic if split else call_bytes
+    achieved = hbm_bytes / call_s / 1e9 if calls and hbm_bytes else None
+    return {"bound": "l2" if split else "fp64",
+            "kernel": ("%s: finest-level relax, colour-split FP32 red-black sweep, 2 launches per relax (%.0f B/cell "
+                       "through L2; achieved and frac: DRAM traffic)" % (kname, words) if split
+                       else "%s: finest-level relax, 2 red-black FP64 colour passes (u r+w, a, b, c, rhs: at most "
+                            "48 B/cell, warps in one fluid read no coefficients)" % kname),
             "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": (achieved / peak) if achieved else None, "traffic": committed_traffic(kname, n),
-            "peak_kind": peak_kind,
-            "bytes_per_launch": (prof["relax_bytes"] / prof["relax_calls"]) if prof["relax_calls"] else None,
-            "relax_calls": prof["relax_calls"],
+            "frac": (achieved / peak) if achieved else None, "traffic": traffic,
+            "l2_gbs": (call_bytes / call_s / 1e9) if split and calls else None,
+            "peak_kind": peak_kind, "bytes_per_launch": call_bytes, "relax_calls": calls,
             "share_of_step": (prof["relax_ms"] / step_ms) if step_ms else None}
 
 
