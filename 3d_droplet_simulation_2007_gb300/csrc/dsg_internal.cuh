@@ -547,7 +547,8 @@ inline int pre32(const dsg_ctx *ctx) { return ctx->cfg.mg32_npre > 0 ? ctx->cfg.
 inline int post32(const dsg_ctx *ctx) { return ctx->cfg.mg32_npost > 0 ? ctx->cfg.mg32_npost : ctx->s.npost; }
 
 // Levels of at most this many nodes may have their own sweep counts
-// (mg32_small_npre/npost): the levels the coarse tail runs by default.
+// (mg32_small_npre/npost); a member's coarsest level has at most as many to be
+// batched (tail_nodes = 0).
 constexpr long long kSmallLevelNodes = 18LL * 18 * 18;
 
 inline bool small_level(const dsg_ctx *ctx, int l) {
@@ -556,8 +557,7 @@ inline bool small_level(const dsg_ctx *ctx, int l) {
 
 // Sweeps on level l: the finest level, the one below it and the small levels
 // may have their own counts (a sweep on the finest level costs 8x and on the
-// next 2-3x one of the smaller levels, which are bound by launch latency or,
-// inside the coarse tail, by one SM's issue rate).
+// next 2-3x one of the smaller levels, which are bound by latency).
 inline int pre32(const dsg_ctx *ctx, int l) {
   if (l == ctx->ng && ctx->cfg.mg32_fine_npre > 0) return ctx->cfg.mg32_fine_npre;
   if (l == ctx->ng - 1 && ctx->cfg.mg32_mid_npre > 0) return ctx->cfg.mg32_mid_npre;

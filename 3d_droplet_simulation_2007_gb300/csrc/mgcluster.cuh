@@ -404,10 +404,9 @@ __device__ __noinline__ void smooth(int level, int rank, int n, typename A::T h2
         for (int b = 0; b < B; b++) {
           const T(&k)[6] = cf[col][q0 + b];
           const T(&x)[9] = v[b];
-          // a warp without a cell would take the FP64 pipe from the others
-          // an FP64 instruction holds its quarter of the SM for 16 cycles, also
-          // for a warp without a cell: skipping those took a pass at 4^3 from
-          // 1.5 to 0.8 us, at 16^3 from 2.3 to 1.4
+          // an FP64 instruction holds its warp scheduler's FP64 pipe for 64
+          // cycles, also for a warp without a cell: skipping those took a pass
+          // at 4^3 from 1.5 to 0.8 us, at 16^3 from 2.3 to 1.4
           if (sizeof(T) == 8 && first + (q0 + b) * kThreads >= total) continue;
           v[b][0] = A::relax(x[0], x[1], x[2], x[3], x[4], x[5], x[6], k[0], k[1], k[2], k[3], k[4], k[5], x[7], x[8],
                              h2, omega);

@@ -445,9 +445,8 @@ void sweep(const double *us, double *cc, double *v1, double *v2, double *v3, Dim
   const int wpr = words_per_row(d), rows = 4 * kScanRows;
   DSG_COUNT k_swp_scan<D><<<dim3((unsigned)wpr, (unsigned)((d.ny - 2 + rows - 1) / rows), (unsigned)(d.nz - 2)), kBlk,
                             0, st>>>(us, cc, v1, v2, v3, d, tauh, bits, list, count);
-  // One warp per block: a cell is some thousand FP64 operations in sequence,
-  // and warps on one SM share its FP64 pipe, so a short list goes to as many
-  // SMs as it has warps (64^3 droplet: 36 us, 40 us with four warps per block).
+  // 32 cells and four warps per block: a short list goes to as many SMs as it
+  // has sets of 32 cells; a block beyond its end has nothing to do.
   DSG_COUNT k_swp_flux_iface<D><<<kRedBlocks, 128, 0, st>>>(list, count, us, cc, v1, v2, v3, d, tauh);
   const size_t words = (size_t)wpr * (d.ny - 2) * (d.nz - 2);
   // Words per warp: on small grids few, because a warp goes through its busy

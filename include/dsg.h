@@ -149,7 +149,10 @@ typedef struct dsg_ctx dsg_ctx;
 
 /* ---- lifecycle ---------------------------------------------------------- */
 /* readinput + memoryaloc + nondim (main.f:185-446).  Allocates the device
- * arena; requires min(nx,ny,nz) = 2^ng+2 (memoryaloc main.f:295-298). */
+ * arena; requires min(nx,ny,nz) = 2^ng+2 (memoryaloc main.f:295-298).
+ * Contexts that step at the same time, each on its own stream and host thread,
+ * take turns on the GPU where a multigrid level runs in one cooperative launch
+ * over all of it; an ensemble's members have no such launches. */
 int dsg_create(const dsg_config *cfg, dsg_ctx **out);
 void dsg_destroy(dsg_ctx *ctx);
 const char *dsg_last_error(const dsg_ctx *ctx); /* ctx may be NULL: last error of this host thread */
@@ -392,7 +395,7 @@ int64_t dsg_ensemble_batch_tail_nodes(const dsg_ensemble *e);
  * memory when they solve (a host that owns its device arrays under an
  * allocator that forbids cudaMalloc after set-up, or a solve inside a region
  * where an allocation would synchronize the device): the fixed-cycle FMG of
- * mglin (main.f:3645-3763, same kernels and result as dsg_mglin in
+ * mglin (main.f:3645-3763, one launch per pass, same result as dsg_mglin in
  * DSG_MODE_REF_EXACT) on caller-owned device arrays p (in/out: overwritten,
  * ghosts included), rhs, a, b, c, ei of size nx*ny*nz.  Coarse levels and the
  * finest residual live in one static device array sized for grids up to
