@@ -549,11 +549,12 @@ cudaError_t resid_restrict32(float *rhs_c, float *u_c, const float *u, const flo
 
 template <bool SPLIT>
 static cudaError_t grid32_s(const mgg::Args<float> &G, cudaStream_t st) {
-  const int halo = (G.g.words() + mgg::kThreads - 1) / mgg::kThreads;
-  if (G.g.cells <= 1 && halo <= 2) return mgg::launch(k_grid32<1, 2, SPLIT>, mgg::kThreads, G, st);
-  if (G.g.cells <= 2 && halo <= 4) return mgg::launch(k_grid32<2, 4, SPLIT>, mgg::kThreads, G, st);
-  if (G.g.cells <= 4 && halo <= 4) return mgg::launch(k_grid32<4, 4, SPLIT>, mgg::kThreads, G, st);
-  return mgg::launch(k_grid32<8, 8, SPLIT>, mgg::kThreads, G, st);
+  switch (mgg::form(G.g)) {
+    case 1: return mgg::launch(k_grid32<1, 2, SPLIT>, mgg::kThreads, G, st);
+    case 2: return mgg::launch(k_grid32<2, 4, SPLIT>, mgg::kThreads, G, st);
+    case 4: return mgg::launch(k_grid32<4, 4, SPLIT>, mgg::kThreads, G, st);
+    default: return mgg::launch(k_grid32<8, 8, SPLIT>, mgg::kThreads, G, st);
+  }
 }
 
 int grid32_blocks() {

@@ -53,6 +53,7 @@ struct Boxes {
   __host__ __device__ int y0(int b) const { return unit * (int)((long long)b * (ny / unit) / py); }
   __host__ __device__ int z0(int b) const { return unit * (int)((long long)b * (nz / unit) / pz); }
   __host__ __device__ int words() const { return 2 * hx * (ry + np); }  // values a block sends per pass, at most
+  int halo() const { return (words() + kThreads - 1) / kThreads; }  // halo cells a thread owns, at most
   __host__ __device__ int half() const { return (np + 2) * (ry + 2) * hx; }
   __host__ __device__ int blocks() const { return py * pz; }
 };
@@ -73,7 +74,7 @@ struct Args {
   int ghosts;                   // write u's ghosts as bc_scalar does
   unsigned long long *mail;     // 2 buffers per block
   unsigned *epoch;              // passes so far, per block
-  int staged;                   // ei and rhs in shared memory
+  int staged;                   // ei and rhs in shared memory (form)
   int o_er, o_res;              // element offsets in shared memory
   size_t shared;
   int box;                      // a phase of mgbox.cuh
@@ -103,7 +104,7 @@ inline bool plan(Boxes &g, int nx, int ny, int nz, int sms, size_t size, int max
       t.np = (uz + pz - 1) / pz * g.unit;
       const long long own = (long long)t.hx * t.ry * t.np, halo = t.words();
       t.cells = (int)((own + kThreads - 1) / kThreads);
-      if (t.cells > max_cells || (halo + kThreads - 1) / kThreads > max_halo) continue;
+      if (t.cells > max_cells || t.halo() > max_halo) continue;
       if (2 * (long long)t.half() * (long long)size + 64 > 0xFFFF) continue;
       const long long cost = own + 2 * halo;
       if (best < 0 || cost < best) {
@@ -114,12 +115,24 @@ inline bool plan(Boxes &g, int nx, int ny, int nz, int sms, size_t size, int max
   return best >= 0;
 }
 
+// The kernel's form for a cut: cells per thread and colour that it has room for
+// (1, 2, 4 or 8), with two, four, four and eight halo cells per thread.  Up to
+// four a thread keeps its cells' ei and right-hand side in registers, in the
+// last form they are staged in shared memory: long rows can need that form for
+// their halo alone.
+inline int form(const Boxes &g) {
+  const int h = g.halo();
+  if (g.cells <= 1 && h <= 2) return 1;
+  if (h > 4) return 8;
+  return g.cells <= 2 ? 2 : g.cells <= 4 ? 4 : 8;
+}
+
 template <class T>
 bool layout(Args<T> &G) {
   const Boxes &g = G.g;
   size_t n = 64 / sizeof(T) + 2 * (size_t)g.half();
   n = (n + 3) & ~(size_t)3;
-  G.staged = g.cells > 4;
+  G.staged = form(g) > 4;
   G.o_er = (int)n;
   if (G.staged) n += 4 * (size_t)g.hx * g.ry * g.np;
   G.o_res = (int)n;
