@@ -62,9 +62,8 @@ __global__ void k_bc_copy(double *__restrict__ s, Dims d) {
   }
   auto put = [&](int i, int j, int k, double x) {
     const size_t n = d.ix(i, j, k);
-    const double old = s[n];
-    if (i == 2) s[n - 1] = old;
-    if (i == d.nx - 1) s[n + 1] = old;
+    if (i == 2) s[n - 1] = s[n];
+    if (i == d.nx - 1) s[n + 1] = s[n];
     s[n] = x;
   };
   if (face == 1) {  // p -> i, q -> k
